@@ -83,7 +83,7 @@ void finishLevel(HostLevel& L) {
                 for (int i = 0; i < L.NX; i++) {
                     const int64_t n = L.node(i, j, int(k));
                     double diag[3] = {0, 0, 0};
-                    bool active = false;
+                    bool active = false, own = false;
                     uint32_t w0 = 0;
                     bool uniform = true;
                     for (int v = 0; v < 8; v++) {
@@ -95,6 +95,7 @@ void finishLevel(HostLevel& L) {
                         uniform = uniform && w == w0;
                         if (!w) continue;
                         active = true;
+                        own = own || (w & OWN_BIT);
                         const int a = cornerIndex(1 - di, 1 - dj, 1 - dk);
                         for (int d = 0; d < 3; d++) diag[d] += entry(L, w, 3 * a + d, 3 * a + d);
                     }
@@ -102,6 +103,7 @@ void finishLevel(HostLevel& L) {
                     if (active) {
                         m |= NM_ACTIVE;
                         if (uniform && w0 && !(w0 & OWN_BIT)) m |= NM_UNIFORM;
+                        if (!own) m |= NM_PLAIN;
                     }
                     for (int d = 0; d < 3; d++) {
                         double dg = diag[d];

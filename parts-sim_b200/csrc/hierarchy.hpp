@@ -19,6 +19,7 @@ constexpr uint32_t OWN_BIT = 0x80000000u;
 constexpr uint8_t NM_FIXED0 = 1, NM_FIXED1 = 2, NM_FIXED2 = 4;  // DOF d held, inactive or zero diagonal
 constexpr uint8_t NM_ACTIVE = 8;    // the node is a corner of some element
 constexpr uint8_t NM_UNIFORM = 16;  // its 8 voxels are the same s * Kb: the 27-point stencil applies
+constexpr uint8_t NM_PLAIN = 32;    // active, and none of its voxels has an own matrix
 
 // An allocator whose new elements are left uninitialised: for large host arrays that parallel
 // loops fill completely right after allocation (no serial zero fill first)

@@ -19,7 +19,7 @@ namespace psfea {
 namespace dev {
 
 constexpr uint32_t OWN_BIT = 0x80000000u;
-constexpr uint8_t NM_ACTIVE = 8, NM_UNIFORM = 16;
+constexpr uint8_t NM_ACTIVE = 8, NM_UNIFORM = 16, NM_PLAIN = 32;
 
 struct LevelView {
     int nx, ny, nz, NX, NY, NZ;  // voxel and node counts per axis
@@ -41,12 +41,6 @@ struct Coefs {
     alignas(16) T Kb[576];  // row-major 24x24 (16-byte aligned: read as pairs by the paired FMAs)
     T S[243];               // [m][3 d + c], m = (ox+1) + 3 (oy+1) + 9 (oz+1)
 };
-// the 32-bit coefficients also as duplicated pairs (s, s), the operand of a paired FMA that
-// advances two nodes at once
-struct Coefs32 : Coefs<float> {
-    float2 S2[243];
-};
-
 // corner index of the unit offset (x, y, z)
 __host__ __device__ constexpr int cornerOf(int x, int y, int z) { return (y ? (x ? 2 : 3) : (x ? 1 : 0)) + 4 * z; }
 
@@ -337,84 +331,28 @@ __device__ bool gridReduce(double (&v)[K], unsigned maxMask, double* partials, u
 namespace psfea {
 namespace dev {
 
-// ---------------------------------------------------------------- tiled operator
-//
-// One CTA per 32 x 8 x 4 node tile (only tiles with an active node are launched). One thread stages
-// what the tile needs with tensor-memory-access (TMA) copies on two shared-memory barriers: the x
-// values with a one-node halo and the voxel words around the tile first, the tile's r and d (the
-// smoother and residual epilogues) second. Each thread then computes its column of four nodes with
-// the 153-FMA assembled stencil from shared memory (uniform nodes) and runs their epilogues in
-// shared memory. Boundary nodes (active, not uniform): 32-bit tiles compact them in a fixed order
-// and give one thread each the per-voxel gather, packed into as few warps as possible; 64-bit tiles
-// leave them to the boundary-node kernel that follows, which overwrites their output slots (the
-// FP64 gather is heavy enough to want a launch of its own at full occupancy). One thread writes
-// the tile back with TMA stores. Inactive nodes are written 0; inactive tiles are never touched
-// (their outputs are 0 already).
-//
-// TMA boxes start on 16-byte boundaries: node rows are pitched (PX, a multiple of 4) and the halo
-// box starts 4 nodes (12 values) left of the tile instead of 1, the voxel box 4 words left of it;
-// boxes reaching outside the grid read zeros.
+// ---------------------------------------------------------------- shared by the operator kernels
 
-constexpr int TX = 32, TY = 8, TZ = 4, TILE_THREADS = TX * TY, TILE_NODES = TX * TY * TZ;
-constexpr int HY = TY + 2, HZ = TZ + 2;          // x halo rows and planes
-constexpr int XLEFT = 4;                         // halo box starts XLEFT nodes left of the tile
-// halo box row: nodes i0-4 .. i0+33 (111 values) padded to 116, so that the plane stride of the
-// shared-memory halo (10 rows, 1160 words) is not a multiple of the 32 banks: the four planes of a
-// column then sit in different banks when the lanes of a warp take the nodes of a few columns
-constexpr int PROW = 116;
-constexpr int VX = TX + 1, VY = TY + 1, VZ = TZ + 1;  // voxel words needed per axis
-constexpr int WROW = 36;                         // voxel box row: words i0-4 .. i0+31 (144 bytes)
-constexpr int TROW = 3 * TX;                     // tile box row (r, d, 1/diag, y): 96 values
-static_assert(3 * (TX + 1 + XLEFT) <= PROW, "halo row");
-static_assert(VX + XLEFT - 1 <= WROW, "voxel row");
-
+// epilogues of the operator passes over a large level's nodes
 enum { TOP_APPLY = 0, TOP_CHEB = 1, TOP_RESID = 2, TOP_DOT = 3 };
 
-// tensor maps of one tiled launch: x (halo box), the voxel words, r, d, 1/diag and y (tile boxes)
-struct TileMaps {
-    CUtensorMap x, w, r, d, inv, y;
-};
-
-template <class T>
-struct TileIO {
+struct MarchIO {
     float c1, c2;      // CHEB: d = c1 d + c2 D^-1 (r - K x)
     int raw;           // APPLY: keep held DOFs
-    int partial;       // DOT: leave the step to the boundary-node kernel (st->pqPart holds the tiles' share)
+    int partial;       // DOT: leave the step to the list kernel (st->pqPart holds the marched share)
+    unsigned outBit;   // the mask bit of the nodes to compute
 };
 
 __host__ __device__ constexpr uint32_t packTile(int tx, int ty, int tz) { return uint32_t(tx) | (uint32_t(ty) << 11) | (uint32_t(tz) << 22); }
 
-// shared-memory layout of a tile CTA, every TMA destination on a 128-byte boundary: x halo, voxel
-// words, the output tile (r for the smoother and residual epilogues, overwritten by y in place;
-// a separate y tile otherwise), d (smoother, updated in place), 1/diag (smoother), the node masks
-// and boundary list (32-bit) and two staging barriers (x and words; the epilogue operands)
 __host__ __device__ constexpr size_t align128(size_t b) { return (b + 127) & ~size_t(127); }
-__host__ __device__ constexpr bool tileHasR(int mode) { return mode == TOP_CHEB || mode == TOP_RESID; }
-__host__ __device__ constexpr bool tileHasD(int mode) { return mode == TOP_CHEB; }
-template <class T> __host__ __device__ constexpr size_t tileBytesX() { return sizeof(T) * PROW * HY * HZ; }
-__host__ __device__ constexpr size_t tileBytesW() { return sizeof(uint32_t) * WROW * VY * VZ; }
-template <class T> __host__ __device__ constexpr size_t tileBytesT() { return sizeof(T) * TROW * TY * TZ; }
-template <class T> __host__ __device__ constexpr size_t tileOffW() { return align128(tileBytesX<T>()); }
-template <class T> __host__ __device__ constexpr size_t tileOffY() { return tileOffW<T>() + align128(tileBytesW()); }
-template <class T, int MODE> __host__ __device__ constexpr size_t tileOffD() {
-    return tileOffY<T>() + align128(tileHasR(MODE) ? tileBytesT<float>() : tileBytesT<T>());
-}
-// INNER: the tile computes its boundary nodes itself (a compacted list in shared memory); else the
-// boundary-node kernel does
-template <class T, int MODE> __host__ __device__ constexpr size_t tileOffI() { return tileOffD<T, MODE>() + (tileHasD(MODE) ? align128(tileBytesT<float>()) : 0); }
-template <class T, int MODE> __host__ __device__ constexpr size_t tileOffM() { return tileOffI<T, MODE>() + (tileHasD(MODE) ? align128(tileBytesT<float>()) : 0); }
-template <class T, int MODE, bool INNER> __host__ __device__ constexpr size_t tileOffB() { return tileOffM<T, MODE>() + (INNER ? align128(TILE_NODES) : 0); }
-template <class T, int MODE, bool INNER> __host__ __device__ constexpr size_t tileOffBar() {
-    return tileOffB<T, MODE, INNER>() + (INNER ? align128(2 * TILE_NODES + 4 * 16) : 0);  // list, warp counts, chunk counter
-}
-template <class T, int MODE, bool INNER> __host__ __device__ constexpr size_t tileSmemBytes() { return tileOffBar<T, MODE, INNER>() + 16; }
-// bytes each staging barrier expects
-template <class T> __host__ __device__ constexpr unsigned tileStage0Bytes() { return unsigned(tileBytesX<T>() + tileBytesW()); }
-template <int MODE> __host__ __device__ constexpr unsigned tileStage1Bytes() {
-    return unsigned((tileHasR(MODE) ? tileBytesT<float>() : 0) + (tileHasD(MODE) ? 2 * tileBytesT<float>() : 0));
-}
 
-// ---- TMA and shared-memory barrier primitives (PTX, sm_90 and later; every copy lands in the issuing CTA's own shared memory)
+// Bound on the polls of a shared-memory barrier. A wait that never completes (it cannot in a correct
+// launch) is given up: the CTA records ST_ERR_STAGING in st->err and ends the solve.
+constexpr unsigned TILE_WAIT_POLLS = 1u << 22;
+constexpr int ST_ERR_STAGING = 1, ST_ERR_ALIGN = 2;
+
+// ---- shared-memory barrier primitives (PTX, sm_90 and later)
 __device__ __forceinline__ unsigned smemAddr(const void* p) { return unsigned(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbarInit(uint64_t* bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smemAddr(bar)), "r"(count) : "memory");
@@ -440,203 +378,8 @@ __device__ __forceinline__ bool mbarWaitParity(uint64_t* bar, unsigned parity, u
     return false;
 }
 __device__ __forceinline__ bool mbarWait(uint64_t* bar, unsigned limit) { return mbarWaitParity(bar, 0, limit); }
-// 3-D tiled load of a box at element coordinates (c0, c1, c2) into shared memory, completing on bar
-__device__ __forceinline__ void tmaLoad3d(void* dst, const void* map, int c0, int c1, int c2, uint64_t* bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];\n" ::"r"(smemAddr(dst)),
-        "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(smemAddr(bar))
-        : "memory");
-}
-// 3-D tiled store of a shared-memory box to (c0, c1, c2), c0..c2 >= 0; elements outside the tensor are skipped
-__device__ __forceinline__ void tmaStore3d(const void* map, const void* src, int c0, int c1, int c2) {
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];\n" ::"l"(map), "r"(smemAddr(src)), "r"(c0),
-                 "r"(c1), "r"(c2)
-                 : "memory");
-}
-__device__ __forceinline__ void tmaStoreCommitWait() {
-    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
-    asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
-}
 // makes this thread's shared-memory writes visible to later TMA (async proxy) reads
 __device__ __forceinline__ void fenceAsyncShared() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-
-// shared-memory offsets of x value (node tx + ox, ty + oy, tz + oz of the tile, component 0) and of
-// the voxel word at tile voxel (vx, vy, vz) (voxel i0 - 1 + vx, ...)
-__device__ __forceinline__ int xOff(int cx, int cy, int cz) { return ((cz + 1) * HY + (cy + 1)) * PROW + 3 * (cx + XLEFT); }
-__device__ __forceinline__ int vOff(int vx, int vy, int vz) { return (vz * VY + vy) * WROW + vx + XLEFT - 1; }
-
-template <class T, bool OWN16, bool DIFF>
-struct TileOp {
-    // adds voxel V's rows at a tile node to acc (V = di + 2 dj + 4 dk: the voxel at offset
-    // (di - 1, dj - 1, dk - 1) from the node); A and B: rows oy = dj - 1 and dj (x offsets -1..1) of
-    // the node's neighbourhood in planes oz = dk - 1 and dk (values already relative to the node's
-    // own value when DIFF). V is a compile-time constant, so every Kb coefficient is a constant-bank
-    // operand.
-    template <int V>
-    static __device__ __forceinline__ void voxel(const LevelView& L, const Coefs<T>& C, const uint32_t* vs, int cx, int cy, int cz,
-                                                 const T (&A)[2][3][3], const T (&B)[2][3][3], T acc[3]) {
-        constexpr int di = V & 1, dj = (V >> 1) & 1, dk = V >> 2;
-        constexpr int a = cornerOf(1 - di, 1 - dj, 1 - dk);
-        const uint32_t w = vs[vOff(cx + di, cy + dj, cz + dk)];
-        if (w == 0) return;
-        T xe[24];
-#pragma unroll
-        for (int b = 0; b < 8; b++) {
-            const int bx = (b == 1 || b == 2 || b == 5 || b == 6), by = (b == 2 || b == 3 || b == 6 || b == 7), bz = b >> 2;
-#pragma unroll
-            for (int c = 0; c < 3; c++) xe[3 * b + c] = bz ? B[by][di + bx][c] : A[by][di + bx][c];
-        }
-        if (!(w & OWN_BIT)) {
-            T t[3];
-            kbRows<T>(C.Kb, a, xe, t);
-            const T s = T(__uint_as_float(w));
-            acc[0] += s * t[0];
-            acc[1] += s * t[1];
-            acc[2] += s * t[2];
-        } else if (OWN16) {
-            T t[3];
-            own16Rows<T>(L.own16 + (long long)(w & ~OWN_BIT) * 576 + 72 * a, xe, t);
-            acc[0] += T(L.hs) * t[0];
-            acc[1] += T(L.hs) * t[1];
-            acc[2] += T(L.hs) * t[2];
-        } else {
-            const float4* K4 = reinterpret_cast<const float4*>(L.own + (long long)(w & ~OWN_BIT) * 576 + 72 * a);
-#pragma unroll
-            for (int d = 0; d < 3; d++)
-#pragma unroll
-                for (int q = 0; q < 6; q++) {
-                    const float4 kv = __ldg(K4 + d * 6 + q);
-                    acc[d] += T(kv.x) * xe[4 * q] + T(kv.y) * xe[4 * q + 1] + T(kv.z) * xe[4 * q + 2] + T(kv.w) * xe[4 * q + 3];
-                }
-        }
-    }
-    // rows oy and oy + 1 (x offsets -1..1) of plane oz around tile node (cx, cy, cz), less own (DIFF)
-    static __device__ __forceinline__ void rowPair(const T* xs, int cx, int cy, int cz, int oy, int oz, const T own[3], T (&R)[2][3][3]) {
-#pragma unroll
-        for (int yy = 0; yy < 2; yy++)
-#pragma unroll
-            for (int e = 0; e < 3; e++) {
-                const T* xp = xs + xOff(cx + e - 1, cy + oy + yy, cz + oz);
-                R[yy][e][0] = xp[0] - own[0];
-                R[yy][e][1] = xp[1] - own[1];
-                R[yy][e][2] = xp[2] - own[2];
-            }
-    }
-    // K x at tile node (cx, cy, cz) by the per-voxel gather over its 8 voxels, two at a time: each
-    // pair of voxels sharing (dj, dk) reads the two row pairs it needs (36 values live, not the 81
-    // of the whole neighbourhood: fewer registers outweigh the extra shared-memory loads)
-    static __device__ __forceinline__ void general(const LevelView& L, const Coefs<T>& C, const T* xs, const uint32_t* vs, int cx, int cy,
-                                                   int cz, T acc[3], const T own[3]) {
-        acc[0] = acc[1] = acc[2] = T(0);
-        T A[2][3][3], B[2][3][3];
-        rowPair(xs, cx, cy, cz, -1, -1, own, A);
-        rowPair(xs, cx, cy, cz, -1, 0, own, B);
-        voxel<0>(L, C, vs, cx, cy, cz, A, B, acc);
-        voxel<1>(L, C, vs, cx, cy, cz, A, B, acc);
-        rowPair(xs, cx, cy, cz, 0, -1, own, A);
-        rowPair(xs, cx, cy, cz, 0, 0, own, B);
-        voxel<2>(L, C, vs, cx, cy, cz, A, B, acc);
-        voxel<3>(L, C, vs, cx, cy, cz, A, B, acc);
-        rowPair(xs, cx, cy, cz, -1, 0, own, A);
-        rowPair(xs, cx, cy, cz, -1, 1, own, B);
-        voxel<4>(L, C, vs, cx, cy, cz, A, B, acc);
-        voxel<5>(L, C, vs, cx, cy, cz, A, B, acc);
-        rowPair(xs, cx, cy, cz, 0, 0, own, A);
-        rowPair(xs, cx, cy, cz, 0, 1, own, B);
-        voxel<6>(L, C, vs, cx, cy, cz, A, B, acc);
-        voxel<7>(L, C, vs, cx, cy, cz, A, B, acc);
-    }
-
-    // unscaled stencil sums of the thread's whole column (cz = 0..TZ-1) at once: every plane of the
-    // 3x3 neighbourhood is read from shared memory once and feeds the (up to) three column nodes it
-    // neighbours. With DIFF every value enters as its difference from the output node's own value.
-    static __device__ __forceinline__ void column(const Coefs<T>& C, const T* xs, int cx, int cy, T acc[TZ][3]) {
-#pragma unroll
-        for (int z = 0; z < TZ; z++) acc[z][0] = acc[z][1] = acc[z][2] = T(0);
-        T own[TZ][3];
-#pragma unroll
-        for (int z = 0; z < TZ; z++) {
-            const T* xr = xs + xOff(cx, cy, z);
-            own[z][0] = DIFF ? xr[0] : T(0);
-            own[z][1] = DIFF ? xr[1] : T(0);
-            own[z][2] = DIFF ? xr[2] : T(0);
-        }
-#pragma unroll
-        for (int p = -1; p <= TZ; p++) {
-            T v[9][3];
-#pragma unroll
-            for (int b = 0; b < 9; b++) {
-                const T* xp = xs + xOff(cx + b % 3 - 1, cy + b / 3 - 1, p);
-                v[b][0] = xp[0];
-                v[b][1] = xp[1];
-                v[b][2] = xp[2];
-            }
-#pragma unroll
-            for (int z = p - 1; z <= p + 1; z++) {
-                if (z < 0 || z >= TZ) continue;
-                const int oz = p - z;
-#pragma unroll
-                for (int b = 0; b < 9; b++) {
-                    const int ox = b % 3 - 1, oy = b / 3 - 1, m = (ox + 1) + 3 * (oy + 1) + 9 * (oz + 1);
-                    if (DIFF && m == 13) continue;  // the node itself: a zero difference
-                    const T x0 = v[b][0] - own[z][0], x1 = v[b][1] - own[z][1], x2 = v[b][2] - own[z][2];
-                    T* a = acc[z];
-                    a[0] += C.S[m * 9 + 0] * x0;
-                    a[1] += C.S[m * 9 + 4] * x1;
-                    a[2] += C.S[m * 9 + 8] * x2;
-                    if (ox && oy) { a[0] += C.S[m * 9 + 1] * x1; a[1] += C.S[m * 9 + 3] * x0; }
-                    if (ox && oz) { a[0] += C.S[m * 9 + 2] * x2; a[2] += C.S[m * 9 + 6] * x0; }
-                    if (oy && oz) { a[1] += C.S[m * 9 + 5] * x2; a[2] += C.S[m * 9 + 7] * x1; }
-                }
-            }
-        }
-    }
-
-    // the same column sums with paired FMAs (__ffma2_rn, two nodes per instruction; each lane of
-    // the pair rounds exactly like fmaf): nodes (0, 1) and (2, 3) of the column advance together,
-    // fed by the pair of planes (p, p + 1) that the two nodes see at the same offset
-    static __device__ __forceinline__ void column2(const Coefs32& C, const float* xs, int cx, int cy, float acc[TZ][3]) {
-        static_assert(TZ == 4, "node pairs (0, 1) and (2, 3)");
-        float2 A[2][3];
-#pragma unroll
-        for (int h = 0; h < 2; h++) A[h][0] = A[h][1] = A[h][2] = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int p = -1; p <= 3; p++) {
-            float2 v[9][3];
-#pragma unroll
-            for (int b = 0; b < 9; b++) {
-                const float* x0 = xs + xOff(cx + b % 3 - 1, cy + b / 3 - 1, p);
-                const float* x1 = xs + xOff(cx + b % 3 - 1, cy + b / 3 - 1, p + 1);
-                v[b][0] = make_float2(x0[0], x1[0]);
-                v[b][1] = make_float2(x0[1], x1[1]);
-                v[b][2] = make_float2(x0[2], x1[2]);
-            }
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int oz = p - 2 * h;  // pair h = nodes (2h, 2h + 1) sees planes (p, p + 1) at offset oz
-                if (oz < -1 || oz > 1) continue;
-#pragma unroll
-                for (int b = 0; b < 9; b++) {
-                    const int ox = b % 3 - 1, oy = b / 3 - 1, m = (ox + 1) + 3 * (oy + 1) + 9 * (oz + 1);
-                    float2* a = A[h];
-                    a[0] = __ffma2_rn(C.S2[m * 9 + 0], v[b][0], a[0]);
-                    a[1] = __ffma2_rn(C.S2[m * 9 + 4], v[b][1], a[1]);
-                    a[2] = __ffma2_rn(C.S2[m * 9 + 8], v[b][2], a[2]);
-                    if (ox && oy) { a[0] = __ffma2_rn(C.S2[m * 9 + 1], v[b][1], a[0]); a[1] = __ffma2_rn(C.S2[m * 9 + 3], v[b][0], a[1]); }
-                    if (ox && oz) { a[0] = __ffma2_rn(C.S2[m * 9 + 2], v[b][2], a[0]); a[2] = __ffma2_rn(C.S2[m * 9 + 6], v[b][0], a[2]); }
-                    if (oy && oz) { a[1] = __ffma2_rn(C.S2[m * 9 + 5], v[b][2], a[1]); a[2] = __ffma2_rn(C.S2[m * 9 + 7], v[b][1], a[2]); }
-                }
-            }
-        }
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            acc[0][d] = A[0][d].x;
-            acc[1][d] = A[0][d].y;
-            acc[2][d] = A[1][d].x;
-            acc[3][d] = A[1][d].y;
-        }
-    }
-};
 
 }  // namespace dev
 }  // namespace psfea

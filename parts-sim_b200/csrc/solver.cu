@@ -26,7 +26,6 @@
 #include <chrono>
 #include <map>
 #include <memory>
-#include <tuple>
 #include <type_traits>
 #include <mutex>
 #include <thread>
@@ -260,257 +259,10 @@ __global__ void __launch_bounds__(256) k_op8(LevelView L, Coefs<T> C, const T* _
     }
 }
 
-// ---------------------------------------------------------------- tiled operator kernel
-
-// The level's operator over its active tiles with a per-node epilogue:
-//   TOP_APPLY  y = K x (held DOFs 0 unless raw)
-//   TOP_CHEB   d = c1 d + c2 D^-1 (r - K x); y = x + d      (Chebyshev / Jacobi step, 32-bit)
-//   TOP_RESID  y = r - K x
-//   TOP_DOT    y = K x (held 0) and the CG step alpha = rz / (x . y); x . y <= 0 is a breakdown
-//              (voxel_fea.cpp:902-905)
-// A staging barrier that never completes (it cannot in a correct launch) is given up after a
-// bounded wait: the CTA records ST_ERR_STAGING in st->err and ends the solve.
-constexpr unsigned TILE_WAIT_POLLS = 1u << 22;
-constexpr int ST_ERR_STAGING = 1, ST_ERR_ALIGN = 2;
-
-// the epilogue of tile node (cx, cy, cz) with its K x: results into the output tile (and d)
-template <class T, int MODE>
-__device__ __forceinline__ void tileFinish(const LevelView& L, const TileIO<T>& io, int i0, int j0, int k0, int cx, int cy, int cz, uint8_t mask,
-                                           const T kxIn[3], const float* is, const T* xs, T* ys, float* rs, float* ds, double& dot) {
-    const int base = (cz * TY + cy) * TROW + 3 * cx, xb = xOff(cx, cy, cz);
-    const bool act = mask & NM_ACTIVE;
-#pragma unroll
-    for (int comp = 0; comp < 3; comp++) {
-        const int e = base + comp;
-        const bool fx = fixedDof(mask, comp);
-        const T xv = xs[xb + comp];
-        T kx = act ? kxIn[comp] : T(0);
-        if (act && L.dadd) {
-            const long long id = 3 * ((long long)(i0 + cx) + (long long)L.PX * ((j0 + cy) + (long long)L.NY * (k0 + cz))) + comp;
-            kx += (sizeof(T) == 8 ? T(L.dadd[id]) : T(L.dadd32[id])) * xv;
-        }
-        if constexpr (MODE == TOP_APPLY) {
-            ys[e] = (!io.raw && fx) ? T(0) : kx;
-        } else if constexpr (MODE == TOP_DOT) {
-            const T yv = fx ? T(0) : kx;
-            ys[e] = yv;
-            dot += double(xv) * double(yv);
-        } else if constexpr (MODE == TOP_RESID) {
-            rs[e] = fx ? 0.f : rs[e] - float(kx);
-        } else {
-            if (fx) {
-                ds[e] = 0.f;
-                rs[e] = 0.f;
-            } else {
-                const float dn = io.c1 * ds[e] + io.c2 * is[e] * (rs[e] - float(kx));
-                ds[e] = dn;
-                rs[e] = float(xv) + dn;
-            }
-        }
-    }
-}
-
-// resident CTAs per SM the register budget is cut for (32-bit / 64-bit values)
-#ifndef PSFEA_TILE_CTAS32
-#define PSFEA_TILE_CTAS32 3
-#endif
-#ifndef PSFEA_TILE_CTAS64
-#define PSFEA_TILE_CTAS64 2
-#endif
-
-template <class T> struct CoefsFor { using type = Coefs<T>; };
-template <> struct CoefsFor<float> { using type = Coefs32; };
-
-template <class T, int MODE, bool OWN16, bool DIFF, bool INNER = (sizeof(T) == 4)>
-__global__ void __launch_bounds__(TILE_THREADS, sizeof(T) == 8 ? PSFEA_TILE_CTAS64 : PSFEA_TILE_CTAS32)
-    k_tile(LevelView L, typename CoefsFor<T>::type C, const uint32_t* __restrict__ tiles, const __grid_constant__ TileMaps maps, TileIO<T> io, SolveState* st,
-           double* partials, unsigned* ticket, Ctl ctl) {
-    if (skipped(ctl)) return;
-    using Op = TileOp<T, OWN16, DIFF>;
-    extern __shared__ __align__(128) unsigned char smem[];
-    if (smemAddr(smem) & 127u) {  // the layout's TMA alignment (never expected to fail)
-        if (threadIdx.x == 0) {
-            atomicExch(&st->err, ST_ERR_ALIGN);
-            st->done = 1;
-        }
-        return;
-    }
-    T* xs = reinterpret_cast<T*>(smem);
-    uint32_t* vs = reinterpret_cast<uint32_t*>(smem + tileOffW<T>());
-    T* ys = reinterpret_cast<T*>(smem + tileOffY<T>());        // y tile (APPLY / DOT)
-    float* rs = reinterpret_cast<float*>(smem + tileOffY<T>()); // r tile, then y in place (CHEB / RESID)
-    float* ds = reinterpret_cast<float*>(smem + tileOffD<T, MODE>());
-    const float* is = reinterpret_cast<const float*>(smem + tileOffI<T, MODE>());
-    uint8_t* ms = smem + tileOffM<T, MODE>();
-    uint16_t* blist = reinterpret_cast<uint16_t*>(smem + tileOffB<T, MODE, INNER>());
-    int* wsum = reinterpret_cast<int*>(blist + TILE_NODES);
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + tileOffBar<T, MODE, INNER>());  // [0] x and words, [1] r and d
-    const uint32_t tw = tiles[blockIdx.x];
-    const int i0 = int(tw & 2047u) * TX, j0 = int((tw >> 11) & 2047u) * TY, k0 = int(tw >> 22) * TZ;
-    const int tid = threadIdx.x, cx = tid & 31, cy = tid >> 5;
-    const long long PXY = (long long)L.PX * L.NY;
-
-    // stage: one thread issues every copy, on two barriers
-    if (tid == 0) {
-        mbarInit(bar, 1);
-        mbarInit(bar + 1, 1);
-        mbarExpectTx(bar, tileStage0Bytes<T>());
-        tmaLoad3d(xs, &maps.x, 3 * (i0 - XLEFT), j0 - 1, k0 - 1, bar);
-        tmaLoad3d(vs, &maps.w, i0 - XLEFT, j0 - 1, k0 - 1, bar);
-        if (tileHasR(MODE)) {
-            mbarExpectTx(bar + 1, tileStage1Bytes<MODE>());
-            tmaLoad3d(rs, &maps.r, 3 * i0, j0, k0, bar + 1);
-            if (tileHasD(MODE)) {
-                tmaLoad3d(ds, &maps.d, 3 * i0, j0, k0, bar + 1);
-                tmaLoad3d(const_cast<float*>(is), &maps.inv, 3 * i0, j0, k0, bar + 1);
-            }
-        }
-    }
-    // the column's node masks (padding nodes i >= NX hold 7: inactive, all held) meanwhile
-    const int i = i0 + cx, j = j0 + cy;
-    const bool col = i < L.PX && j < L.NY;
-    uint8_t mk[TZ];
-    bool anyUniform = false;
-    unsigned bmask = 0;  // the column's boundary nodes (active, not uniform)
-#pragma unroll
-    for (int z = 0; z < TZ; z++) {
-        const int k = k0 + z;
-        mk[z] = (col && k < L.NZ) ? __ldg(L.nmask + i + (long long)L.PX * j + PXY * k) : uint8_t(0);
-        if (INNER) ms[(z * TY + cy) * TX + cx] = mk[z];
-        anyUniform = anyUniform || (mk[z] & NM_UNIFORM);
-        if ((mk[z] & NM_ACTIVE) && !(mk[z] & NM_UNIFORM)) bmask |= 1u << z;
-    }
-    int total = 0;
-    if constexpr (INNER) {
-        // the boundary nodes compacted in a fixed order (thread order, then z) while the copies land
-        const int cnt = __popc(bmask);
-        int incl = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (cx >= o) incl += v;
-        }
-        if (cx == 31) wsum[cy] = incl;
-        if (tid == 0) wsum[TILE_THREADS / 32] = 0;  // the counter of handed-out boundary chunks
-        __syncthreads();
-        int off = incl - cnt;
-#pragma unroll
-        for (int w = 0; w < TILE_THREADS / 32; w++) {
-            const int c = wsum[w];
-            off += (w < cy) ? c : 0;
-            total += c;
-        }
-        for (unsigned b = bmask; b; b &= b - 1) blist[off++] = uint16_t((tid << 4) | (__ffs(b) - 1));
-    }
-    __syncthreads();  // barriers initialised; masks and the boundary list in place
-    // each warp goes on as soon as its own wait ends; the outcome is combined before the stores
-    bool ok = mbarWait(bar, TILE_WAIT_POLLS);
-    double dot = 0.0;
-    // pass 1: the thread's column, all four nodes from one sweep of the planes (uniform nodes)
-    T acc[TZ][3];
-    if (ok && anyUniform) {
-        if constexpr (sizeof(T) == 4) Op::column2(C, xs, cx, cy, acc);
-        else Op::column(C, xs, cx, cy, acc);
-    }
-    if (tileHasR(MODE)) ok = ok && mbarWait(bar + 1, TILE_WAIT_POLLS);
-    if (ok) {
-        // epilogue of the column's nodes except the boundary ones. An inactive node (all its DOFs
-        // held; r, d and x are 0 there) gives y = 0: with r staged in place of the output
-        // (smoother, residual) its slots already hold that, a separate output tile gets zeros
-#pragma unroll
-        for (int z = 0; z < TZ; z++) {
-            if ((bmask >> z) & 1u) continue;
-            if (!(mk[z] & NM_ACTIVE)) {
-                if (!tileHasR(MODE)) {  // a separate output tile: its slots are zeros
-                    T* yn = ys + (z * TY + cy) * TROW + 3 * cx;
-                    yn[0] = yn[1] = yn[2] = T(0);
-                }
-                continue;
-            }
-            T kx[3] = {T(0), T(0), T(0)};
-            if (mk[z] & NM_UNIFORM) {
-                const T s = T(__uint_as_float(vs[vOff(cx, cy, z)]));
-                kx[0] = s * acc[z][0];
-                kx[1] = s * acc[z][1];
-                kx[2] = s * acc[z][2];
-            }
-            tileFinish<T, MODE>(L, io, i0, j0, k0, cx, cy, z, mk[z], kx, is, xs, ys, rs, ds, dot);
-        }
-    }
-    if constexpr (INNER) {
-        // pass 2: the listed nodes in chunks of 32 to whichever warp is free first, one thread a node
-        // (per-voxel gather); a node's result does not depend on the warp that computes it, and its
-        // share of x.y is added below by the thread owning its column, in a fixed order
-        for (;;) {
-            int c = 0;
-            if (cx == 0) c = atomicAdd(&wsum[TILE_THREADS / 32], 32);
-            c = __shfl_sync(0xffffffffu, c, 0);
-            if (c >= total) break;
-            const int q = c + cx;
-            if (ok && q < total) {
-                const int e = blist[q], bt = e >> 4, bz = e & 15, bx = bt & 31, by = bt >> 5;
-                T own[3] = {T(0), T(0), T(0)};
-                if (DIFF) {
-                    const T* xn = xs + xOff(bx, by, bz);
-                    own[0] = xn[0]; own[1] = xn[1]; own[2] = xn[2];
-                }
-                T a[3];
-                Op::general(L, C, xs, vs, bx, by, bz, a, own);
-                double unused = 0.0;
-                tileFinish<T, MODE>(L, io, i0, j0, k0, bx, by, bz, ms[(bz * TY + by) * TX + bx], a, is, xs, ys, rs, ds, unused);
-            }
-        }
-    }
-    // results out
-    fenceAsyncShared();
-    const bool staged = __syncthreads_and(ok) != 0;
-    if (INNER && MODE == TOP_DOT && staged) {
-        // the column's boundary nodes' share of x.y, from the y tile
-#pragma unroll
-        for (int z = 0; z < TZ; z++) {
-            if (!((bmask >> z) & 1u)) continue;
-            const T* xn = xs + xOff(cx, cy, z);
-            const T* yn = ys + (z * TY + cy) * TROW + 3 * cx;
-#pragma unroll
-            for (int c = 0; c < 3; c++) dot += double(xn[c]) * double(yn[c]);
-        }
-    }
-    if (staged && tid == 0) {
-        if (tileHasR(MODE)) tmaStore3d(&maps.y, rs, 3 * i0, j0, k0);
-        else tmaStore3d(&maps.y, ys, 3 * i0, j0, k0);
-        if (tileHasD(MODE)) tmaStore3d(&maps.d, ds, 3 * i0, j0, k0);
-        tmaStoreCommitWait();
-    }
-    if (!staged && tid == 0) {
-        atomicExch(&st->err, ST_ERR_STAGING);
-        st->done = 1;
-    }
-    if (MODE == TOP_DOT) {
-        double vv[1] = {dot};
-        double tot[1];
-        if (gridReduce<1>(vv, 0u, partials, ticket, tot) && threadIdx.x == 0) {
-            const double pq = tot[0];
-            if (io.partial) {  // the boundary-node kernel adds its share and finishes the step
-                st->pqPart = pq;
-                return;
-            }
-            st->pq = pq;
-            if (!(pq > 0)) {
-                st->status = ST_BREAKDOWN;
-                if (st->mixed) st->fold = 1;  // fold what there is, then stop
-                else st->done = 1;
-            } else {
-                st->alpha = st->rz / pq;
-            }
-        }
-    }
-}
-
-// The boundary nodes of a tiled level (active, not uniform: next to an empty voxel, a voxel of
-// another scale or an own matrix) from their list, one thread each, with the per-voxel gather and
-// the tiled kernel's epilogues (TOP_*); runs after the tiled kernel on the same vectors and
-// overwrites the boundary nodes' output slots. TOP_DOT adds its p.q share to the tiled one
-// (fixed order: tiles, then boundary nodes) and takes the CG step.
+// The listed nodes of a marched level (those that touch an own matrix, or every node that is not
+// uniform on a split level), one thread each, with the per-voxel gather and the marching kernel's
+// epilogues (TOP_*); runs after the marching kernel, which leaves these nodes out, on the same vectors.
+// TOP_DOT adds its p.q share to the marched one (fixed order) and takes the CG step.
 template <class T, int MODE, bool OWN16, bool DIFF>
 __global__ void __launch_bounds__(NODE_THREADS) k_bnd(LevelView L, Coefs<T> C, const int* __restrict__ list, int count, const T* __restrict__ x,
                                                       T* __restrict__ y, const float* __restrict__ r, float* __restrict__ d, float c1, float c2,
@@ -1284,6 +1036,7 @@ __global__ void k_reactions(long long nNodes, const uint8_t* __restrict__ nmask,
 }  // namespace dev
 }  // namespace psfea
 
+#include "march_kernels.cuh"  // the marched operator of large levels
 #include "block_kernels.cuh"  // the multi-RHS kernels (they use the control helpers above)
 #include "ebe_kernels.cuh"    // the tensor-core element-block operator
 #include "block_tc.cuh"       // the block operator on the tensor cores
@@ -1445,70 +1198,124 @@ int gridFor(int64_t n, int threads, int cap) {
 
 }  // namespace
 
-// ---- tensor maps of the tiled kernels (cuTensorMapEncodeTiled through the runtime's driver entry
-// point, so the library needs no link to the driver library)
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                   const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+// ---- the marched operator's host side
 
-EncodeTiledFn encodeTiled() {
-    static EncodeTiledFn fn = nullptr;
-    static std::once_flag once;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q{};
-        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-        else
-            cudaGetLastError();
-    });
-    if (!fn) throw Error(PS_ECUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    return fn;
+// The element in the reflection basis: block entries (1/64) h_a^T K h_b over the modes h_a = product of (2 x - 1)^a,
+// which vanish outside the blocks of march_kernels.cuh for the element of an isotropic cube and its Galerkin sums
+// over uniform children (checked: ok is false if Kb is anything else).
+template <class T>
+dev::ModeCoefs<T> marchCoefs(const double Kb[576], bool& ok) {
+    double B[24][24];  // [3 a + c][3 b + e], a = ax + 2 ay + 4 az
+    auto sign = [](int a, int corner) {
+        double v = 1;
+        for (int d = 0; d < 3; d++)
+            if ((a >> d) & 1) v *= 2.0 * CORNER_XYZ[corner][d] - 1;
+        return v;
+    };
+    double big = 0;
+    for (int a = 0; a < 8; a++)
+        for (int b = 0; b < 8; b++)
+            for (int c = 0; c < 3; c++)
+                for (int e = 0; e < 3; e++) {
+                    double v = 0;
+                    for (int p = 0; p < 8; p++)
+                        for (int q = 0; q < 8; q++) v += sign(a, p) * sign(b, q) * Kb[(3 * p + c) * 24 + 3 * q + e];
+                    B[3 * a + c][3 * b + e] = v / 64;
+                    big = std::max(big, std::fabs(v / 64));
+                }
+    double M[24][24] = {};
+    // normal strains a_c = e_c (parity 000) and twists a_c = 111 - e_c (parity 111)
+    const double b0 = B[3 * 1 + 0][3 * 2 + 1], a0 = B[3 * 1 + 0][3 * 1 + 0] - b0, b3 = B[3 * 6 + 0][3 * 5 + 1], a3 = B[3 * 6 + 0][3 * 6 + 0] - b3;
+    for (int c = 0; c < 3; c++)
+        for (int e = 0; e < 3; e++) {
+            M[3 * (1 << c) + c][3 * (1 << e) + e] = b0 + (c == e ? a0 : 0);
+            M[3 * (7 ^ (1 << c)) + c][3 * (7 ^ (1 << e)) + e] = b3 + (c == e ? a3 : 0);
+        }
+    // bending: the two components other than p, modes e_p + e_c
+    const double a1 = B[3 * 3 + 1][3 * 3 + 1], b1 = B[3 * 3 + 1][3 * 5 + 2];
+    // shear: components c, e with modes e_e, e_c; the third component's hourglass mode 111
+    const double c2 = B[3 * 2 + 0][3 * 1 + 1], e2 = B[3 * 7 + 2][3 * 7 + 2];
+    for (int p = 0; p < 3; p++) {
+        const int c = (p + 1) % 3, e = (p + 2) % 3;
+        const int mc = 3 * ((1 << p) | (1 << c)) + c, me = 3 * ((1 << p) | (1 << e)) + e;
+        M[mc][mc] = M[me][me] = a1;
+        M[mc][me] = M[me][mc] = b1;
+        const int sc = 3 * (1 << e) + c, se = 3 * (1 << c) + e;
+        M[sc][sc] = M[se][se] = M[sc][se] = M[se][sc] = c2;
+        M[3 * 7 + p][3 * 7 + p] = e2;
+    }
+    ok = true;
+    for (int r = 0; r < 24; r++)
+        for (int q = 0; q < 24; q++) ok = ok && std::fabs(M[r][q] - B[r][q]) <= 1e-12 * big;
+    return {T(b0), T(a0), T(a1), T(b1), T(c2), T(e2), T(b3), T(a3)};
 }
 
-enum MapKind { MAP_HALO = 0, MAP_TILE = 1, MAP_WORDS = 2 };
-
-// x halo boxes (PROW x HY x HZ values), tile boxes (TROW x TY x TZ) over a level's pitched DOF
-// vector, or voxel-word boxes (WROW x VY x VZ); outside the tensor loads read 0 and stores are dropped
-CUtensorMap makeMap(const void* base, MapKind kind, bool f64, const dev::LevelView& v) {
-    CUtensorMap m;
-    cuuint64_t dims[3];
-    cuuint32_t box[3];
-    const cuuint32_t es[3] = {1, 1, 1};
-    CUtensorMapDataType dt;
-    size_t esz;
-    if (kind == MAP_WORDS) {
-        dt = CU_TENSOR_MAP_DATA_TYPE_UINT32;
-        esz = 4;
-        dims[0] = cuuint64_t(v.px); dims[1] = cuuint64_t(v.ny); dims[2] = cuuint64_t(v.nz);
-        box[0] = dev::WROW; box[1] = dev::VY; box[2] = dev::VZ;
-    } else {
-        dt = f64 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-        esz = f64 ? 8 : 4;
-        dims[0] = cuuint64_t(3) * v.PX; dims[1] = cuuint64_t(v.NY); dims[2] = cuuint64_t(v.NZ);
-        if (kind == MAP_HALO) { box[0] = dev::PROW; box[1] = dev::HY; box[2] = dev::HZ; }
-        else { box[0] = dev::TROW; box[1] = dev::TY; box[2] = dev::TZ; }
+// The tiles of a marched level: columns of 30 x ny nodes cut into chunks of planes, trimmed to the planes with an
+// active node. A CTA of n planes takes about n + 4 steps (one plane of halo below and above, two to fill and
+// drain), so the chunk length is the one with the least waves x steps on `slots` resident CTAs: long chunks where
+// the level has many columns, short ones where it would leave SMs idle.
+std::vector<dev::MarchTile> marchTiles(const HostLevel& h, int ny, int slots) {
+    const int ntx = (h.NX + dev::MARCH_NX - 1) / dev::MARCH_NX, nty = (h.NY + ny - 1) / ny;
+    const size_t cols = size_t(ntx) * nty;
+    std::vector<uint8_t> act(cols * h.NZ, 0);  // [k][ty][tx]
+    parallelFor(h.NZ, [&](int64_t ka, int64_t kb) {
+        for (int64_t k = ka; k < kb; k++)
+            for (int j = 0; j < h.NY; j++) {
+                const uint8_t* row = h.nmask.data() + h.node(0, j, int(k));
+                uint8_t* a = act.data() + size_t(k) * cols + size_t(j / ny) * ntx;
+                for (int i = 0; i < h.NX; i++) a[i / dev::MARCH_NX] |= (row[i] & NM_ACTIVE) ? 1 : 0;
+            }
+    }, 8);
+    size_t live = 0;
+    for (size_t c = 0; c < cols; c++) {
+        bool any = false;
+        for (int k = 0; k < h.NZ && !any; k++) any = act[size_t(k) * cols + c] != 0;
+        live += any;
     }
-    const cuuint64_t strides[2] = {dims[0] * esz, dims[0] * dims[1] * esz};
-    const CUresult r = encodeTiled()(&m, dt, 3, const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) throw Error(PS_ECUDA, "cuTensorMapEncodeTiled failed (" + std::to_string(int(r)) + ")");
-    return m;
+    int best = 1;
+    int64_t bestCost = INT64_MAX;
+    for (int tz = 1; tz <= std::min(h.NZ, 96); tz++) {
+        const int64_t ctas = int64_t(live) * ((h.NZ + tz - 1) / tz), cost = ((ctas + slots - 1) / slots) * (tz + 4);
+        if (cost < bestCost) {
+            bestCost = cost;
+            best = tz;
+        }
+    }
+    std::vector<dev::MarchTile> out;
+    for (int kz = 0; kz < h.NZ; kz += best)
+        for (size_t c = 0; c < cols; c++) {
+            int lo = -1, hi = -1;
+            for (int k = kz; k < std::min(h.NZ, kz + best); k++)
+                if (act[size_t(k) * cols + c]) {
+                    if (lo < 0) lo = k;
+                    hi = k + 1;
+                }
+            if (lo >= 0) out.push_back({uint16_t(c % ntx), uint16_t(c / ntx), uint16_t(lo), uint16_t(hi)});
+        }
+    return out;
 }
 
 // Read-only device data of one level, shared by every solve context of a handle.
 struct DevLevel {
     dev::LevelView view{};
     dev::Coefs<double> c64{};
-    dev::Coefs32 c32{};
+    dev::Coefs<float> c32{};
+    dev::ModeCoefs<double> m64{};
+    dev::ModeCoefs<float> m32{};
     DevMem word, nmask, own, own16, invD, dadd, dadd32, bc;
-    DevMem tiles;      // packed (tx, ty, tz) of the 32 x 8 x 4 node tiles with an active node
-    int nTiles = 0;
-    DevMem blist;      // tiled levels: the boundary nodes (pitched indices, increasing)
-    int nBnd = 0;
-    bool inner64 = false;  // 64-bit tiles compute their boundary nodes themselves (else k_bnd does)
-    bool split32 = false;  // 32-bit tiles leave their boundary nodes to k_bnd (else they compute them)
-    bool useTiles = false;  // tiled kernel (large levels) or one thread per node (small ones)
+    DevMem tiles32, tiles64;  // marched levels: the 32- and 64-bit tiles with an active node
+    int nTiles32 = 0, nTiles64 = 0;
+    int nActive = 0;   // active nodes
+    // marched levels: the boundary nodes (active, not uniform) and those of them that touch an own
+    // matrix (pitched indices, increasing); the marching kernel leaves one of the two lists out
+    DevMem blist, olist;
+    int nBnd = 0, nOwnNodes = 0;
+    bool inner64 = false;  // 64-bit marches compute the boundary nodes without own matrices too (else k_bnd does)
+    bool split32 = false;  // 32-bit marches leave all boundary nodes to the list kernels
+    bool useTiles = false;  // marched (large levels) or one thread per node (small ones)
+    const int* list(bool split) const { return (split ? blist : olist).as<int>(); }
+    int listCount(bool split) const { return split ? nBnd : nOwnNodes; }
+    static unsigned outBit(bool split) { return split ? NM_UNIFORM : NM_PLAIN; }
     bool use8 = false;      // eight lanes per node (the smallest levels)
     float cf0 = 0, cf1 = 0, cf2 = 0, omega = 0.5f;
     std::vector<float> chebC1, chebC2;  // steps 1 .. degree-1 of the Chebyshev smoother: d = c1 d + c2 D^-1 (r - K z)
@@ -1526,7 +1333,7 @@ struct DevLevel {
     DevMem stn32, stn16;
     float stnScale = 1.f;
     void release() {
-        for (DevMem* b : {&word, &nmask, &own, &own16, &invD, &dadd, &dadd32, &bc, &tiles, &blist, &ebeTiles, &stn32, &stn16}) b->release();
+        for (DevMem* b : {&word, &nmask, &own, &own16, &invD, &dadd, &dadd32, &bc, &tiles32, &tiles64, &blist, &olist, &ebeTiles, &stn32, &stn16}) b->release();
     }
 };
 
@@ -1661,27 +1468,16 @@ void SharedModel::adopt(Hierarchy&& h) {
     check(cudaEventCreateWithFlags(&readyEv, cudaEventDisableTiming), "event");
     static std::once_flag attrOnce;
     std::call_once(attrOnce, [] {
-        // the tiled operator stages more than the default 48 KB of shared memory
+        // kernels that use more than the default 48 KB of shared memory
         auto set = [](auto kernel, size_t bytes) {
             check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)), "attr");
         };
-        set(dev::k_tile<double, dev::TOP_APPLY, false, false>, dev::tileSmemBytes<double, dev::TOP_APPLY, false>());
-        set(dev::k_tile<double, dev::TOP_DOT, false, false>, dev::tileSmemBytes<double, dev::TOP_DOT, false>());
-        set(dev::k_tile<double, dev::TOP_APPLY, false, false, true>, dev::tileSmemBytes<double, dev::TOP_APPLY, true>());
-        set(dev::k_tile<double, dev::TOP_DOT, false, false, true>, dev::tileSmemBytes<double, dev::TOP_DOT, true>());
-        set(dev::k_tile<float, dev::TOP_CHEB, false, false>, dev::tileSmemBytes<float, dev::TOP_CHEB, true>());
-        set(dev::k_tile<float, dev::TOP_CHEB, true, false>, dev::tileSmemBytes<float, dev::TOP_CHEB, true>());
-        set(dev::k_tile<float, dev::TOP_CHEB, true, true>, dev::tileSmemBytes<float, dev::TOP_CHEB, true>());
-        set(dev::k_tile<float, dev::TOP_RESID, false, false>, dev::tileSmemBytes<float, dev::TOP_RESID, true>());
-        set(dev::k_tile<float, dev::TOP_RESID, true, false>, dev::tileSmemBytes<float, dev::TOP_RESID, true>());
-        set(dev::k_tile<float, dev::TOP_RESID, true, true>, dev::tileSmemBytes<float, dev::TOP_RESID, true>());
-        set(dev::k_tile<float, dev::TOP_DOT, false, true>, dev::tileSmemBytes<float, dev::TOP_DOT, true>());
-        set(dev::k_tile<float, dev::TOP_CHEB, false, false, false>, dev::tileSmemBytes<float, dev::TOP_CHEB, false>());
-        set(dev::k_tile<float, dev::TOP_CHEB, true, false, false>, dev::tileSmemBytes<float, dev::TOP_CHEB, false>());
-        set(dev::k_tile<float, dev::TOP_CHEB, true, true, false>, dev::tileSmemBytes<float, dev::TOP_CHEB, false>());
-        set(dev::k_tile<float, dev::TOP_RESID, false, false, false>, dev::tileSmemBytes<float, dev::TOP_RESID, false>());
-        set(dev::k_tile<float, dev::TOP_RESID, true, false, false>, dev::tileSmemBytes<float, dev::TOP_RESID, false>());
-        set(dev::k_tile<float, dev::TOP_RESID, true, true, false>, dev::tileSmemBytes<float, dev::TOP_RESID, false>());
+        set(dev::k_march<double, dev::TOP_APPLY>, dev::marchSmemBytes<double>());
+        set(dev::k_march<double, dev::TOP_DOT>, dev::marchSmemBytes<double>());
+        set(dev::k_march<float, dev::TOP_APPLY>, dev::marchSmemBytes<float>());
+        set(dev::k_march<float, dev::TOP_CHEB>, dev::marchSmemBytes<float>());
+        set(dev::k_march<float, dev::TOP_RESID>, dev::marchSmemBytes<float>());
+        set(dev::k_march<float, dev::TOP_DOT>, dev::marchSmemBytes<float>());
         set(dev::k_ebe<dev::TOP_APPLY, 1>, dev::ebeSmemBytes<1>());
         set(dev::k_ebe<dev::TOP_CHEB, 1>, dev::ebeSmemBytes<1>());
         set(dev::k_ebe<dev::TOP_RESID, 1>, dev::ebeSmemBytes<1>());
@@ -1717,7 +1513,7 @@ void SharedModel::adopt(Hierarchy&& h) {
         upload(cDof, dofs, bytes, ms);
         upload(cInv, H.coarseInv, bytes, ms);
     }
-    for (auto& D : L) maxTiles = std::max(maxTiles, D.nTiles);
+    for (auto& D : L) maxTiles = std::max({maxTiles, D.nTiles32, D.nTiles64});
     // delta_l = 2^(round(log2(median diagonal of level l)) - 4): the FP16 iterates then sit near
     // 1/16 of the residuals' order one, leaving room for the coarse corrections' growth
     // (one scale per level cannot hold graded stiffness in FP16: when a level's diagonal spans more
@@ -1810,22 +1606,20 @@ void SharedModel::uploadLevel(int l) {
     }
     if (l == 0) upload(D.bc, pitched<uint8_t>(h.bc, 3, h, PX, uint8_t(0)), bytes, ms);
     {
-        const int ntx = (h.NX + dev::TX - 1) / dev::TX, nty = (h.NY + dev::TY - 1) / dev::TY, ntz = (h.NZ + dev::TZ - 1) / dev::TZ;
-        if (ntx > 2047 || nty > 2047 || ntz > 1023) throw Error(PS_EINVAL, "grid too large for the tile index");
-        std::vector<uint8_t> act(size_t(ntx) * nty * ntz, 0);
-        for (int k = 0; k < h.NZ; k++)
-            for (int j = 0; j < h.NY; j++) {
-                const uint8_t* row = h.nmask.data() + h.node(0, j, k);
-                for (int i = 0; i < h.NX; i++)
-                    if (row[i] & NM_ACTIVE) act[size_t((i / dev::TX) + ntx * ((j / dev::TY) + size_t(nty) * (k / dev::TZ)))] = 1;
+        // (the largest grids the 64-bit tile indices of the element-block lists hold)
+        if ((h.NX + 31) / 32 > 2047 || (h.NY + 7) / 8 > 2047 || (h.NZ + 3) / 4 > 1023) throw Error(PS_EINVAL, "grid too large for the tile index");
+        std::vector<int64_t> planeActive(size_t(h.NZ), 0);
+        parallelFor(h.NZ, [&](int64_t k0, int64_t k1) {
+            for (int64_t k = k0; k < k1; k++) {
+                const uint8_t* mk = h.nmask.data() + h.node(0, 0, int(k));
+                int64_t n = 0;
+                for (int64_t q = 0; q < int64_t(h.NX) * h.NY; q++) n += (mk[q] & NM_ACTIVE) ? 1 : 0;
+                planeActive[size_t(k)] = n;
             }
-        std::vector<uint32_t> list;
-        for (int tz = 0; tz < ntz; tz++)
-            for (int ty = 0; ty < nty; ty++)
-                for (int tx = 0; tx < ntx; tx++)
-                    if (act[size_t(tx + ntx * (ty + size_t(nty) * tz))]) list.push_back(dev::packTile(tx, ty, tz));
-        D.nTiles = int(list.size());
-        upload(D.tiles, list, bytes, ms);
+        }, 8);
+        int64_t active = 0;
+        for (int64_t n : planeActive) active += n;
+        D.nActive = int(active);
         if (h.nOwn == 0 && l < 63 && ((ebeLevels >> l) & 1)) {
             // the element-block tiles (8 x 8 x 4 nodes) with an active node
             const int ex = (h.NX + dev::EX - 1) / dev::EX, ey = (h.NY + dev::EY - 1) / dev::EY, ez = (h.NZ + dev::EZ - 1) / dev::EZ;
@@ -1849,34 +1643,34 @@ void SharedModel::uploadLevel(int l) {
         // lanes per node on the smallest ones
         int64_t minNodes = 400000;
         if (const char* e = std::getenv("PSFEA_TILE_MIN_NODES")) minNodes = std::atoll(e);
-        // (and grids no smaller than the staging boxes of 116 x 10 x 6 values and 36 x 9 x 5 words)
-        D.useTiles = h.nNodes >= minNodes && h.NY >= dev::HY && h.NZ >= dev::HZ && 3 * PX >= dev::PROW && px >= dev::WROW;
+        D.m64 = marchCoefs<double>(h.Kb, D.useTiles);
+        D.m32 = marchCoefs<float>(h.Kb, D.useTiles);
+        D.useTiles = D.useTiles && h.nNodes >= minNodes;
         int64_t max8 = 30000;
         if (const char* e = std::getenv("PSFEA_OP8_MAX_NODES")) max8 = std::atoll(e);
         D.use8 = !D.useTiles && l > 0 && h.nNodes <= max8;
-        if (D.useTiles) {  // for the 64-bit tiled kernels
-            std::vector<int32_t> bl(h.boundary.size());
+        if (D.useTiles) {
+            const std::vector<dev::MarchTile> t32 = marchTiles(h, dev::marchNY<float>(), smCount), t64 = marchTiles(h, dev::marchNY<double>(), smCount);
+            D.nTiles32 = int(t32.size());
+            D.nTiles64 = int(t64.size());
+            upload(D.tiles32, t32, bytes, ms);
+            upload(D.tiles64, t64, bytes, ms);
+            std::vector<int32_t> bl(h.boundary.size()), ol;
             for (size_t q = 0; q < bl.size(); q++) {
                 const int64_t nd = h.boundary[q], row = nd / h.NX;
                 bl[q] = int32_t((nd - row * h.NX) + int64_t(PX) * row);
+                if (!(h.nmask[size_t(nd)] & NM_PLAIN)) ol.push_back(bl[q]);
             }
             D.nBnd = int(bl.size());
+            D.nOwnNodes = int(ol.size());
             upload(D.blist, bl, bytes, ms);
-            // in the tile once boundary nodes are a large share of the level (graded grids, thin
-            // walls); PSFEA_TILE_INNER64: 0 never, 1 always
-            int64_t active = 0;
-            for (uint8_t mk : h.nmask) active += (mk & NM_ACTIVE) ? 1 : 0;
-            D.inner64 = active > 0 && double(bl.size()) >= 0.3 * double(active);
-            if (const char* e = std::getenv("PSFEA_TILE_INNER64")) {
-                const int v = std::atoi(e);
-                if (v == 0 || v == 1) D.inner64 = v == 1;
-            }
-            // 32-bit tiles of the Galerkin levels (l >= 1) leave their boundary nodes to k_bnd: there
-            // the boundary nodes gather own matrices, and the few hundred tiles of such a level wait
-            // on their heaviest ones (L-bracket level 1: 495 tiles, 36 % boundary nodes; FP64-form
-            // solves 7-10 % faster on the L-bracket and the gyroid, the finest level slower split).
-            // PSFEA_TILE_SPLIT32: bit l set = level l split
-            D.split32 = l > 0;
+            upload(D.olist, ol, bytes, ms);
+            // the marches compute every node that touches no own matrix: a boundary node costs them no more
+            // than a uniform one. PSFEA_TILE_INNER64=0 and PSFEA_TILE_SPLIT32 (bit l set = level l) leave all
+            // boundary nodes to the list kernels instead
+            D.inner64 = true;
+            if (const char* e = std::getenv("PSFEA_TILE_INNER64")) D.inner64 = std::atoi(e) != 0;
+            D.split32 = false;
             if (const char* e = std::getenv("PSFEA_TILE_SPLIT32")) D.split32 = l < 63 && ((std::atoll(e) >> l) & 1);
         }
     }
@@ -1900,7 +1694,6 @@ void SharedModel::uploadLevel(int l) {
         for (int e = 0; e < 9; e++) {
             D.c64.S[m * 9 + e] = h.S[m][e];
             D.c32.S[m * 9 + e] = float(h.S[m][e]);
-            D.c32.S2[m * 9 + e] = make_float2(float(h.S[m][e]), float(h.S[m][e]));
         }
 }
 
@@ -1911,9 +1704,14 @@ void SharedModel::ensureStencils(bool half) {
     bool built = false;
     for (size_t l = 1; l < L.size() && l < 63; l++) {
         DevLevel& D = L[l];
-        const int cnt = D.useTiles ? (D.split32 ? D.nBnd : 0) : nAct[l];
+        const int cnt = D.useTiles ? D.listCount(D.split32) : nAct[l];
         if (!((stencilLevels >> l) & 1) || cnt <= 0 || cnt < stencilMinNodes) continue;
-        D.stnNodes = D.useTiles ? D.blist.as<int>() : act[l].as<int>();
+        const int* nodes = D.useTiles ? D.list(D.split32) : act[l].as<int>();
+        if (D.stnNodes != nodes) {  // (the autotuner may switch a level's list)
+            D.stn32.release();
+            D.stn16.release();
+        }
+        D.stnNodes = nodes;
         D.nStn = cnt;
         const int grid = gridFor(int64_t(cnt) * 27, 256, smCount * 32);
         if (!half && !D.stn32.p) {
@@ -2076,15 +1874,6 @@ struct SolverImpl {
     // node and DOF counts of level l in the pitched device layout (every device vector's length)
     int64_t pn(int l) const { return L[size_t(l)].view.nNodes; }
     int64_t pd(int l) const { return 3 * pn(l); }
-    // tensor maps by (base, kind, level); a base address can only be reused for the same level's
-    // vector of the same kind, which has the same map
-    std::map<std::tuple<const void*, int, int>, CUtensorMap> mapCache;
-    const CUtensorMap& mapOf(const void* base, MapKind kind, bool f64, int l) {
-        const auto key = std::make_tuple(base, int(kind) * 2 + (f64 ? 1 : 0), l);
-        auto it = mapCache.find(key);
-        if (it == mapCache.end()) it = mapCache.emplace(key, makeMap(base, kind, f64, L[size_t(l)].view)).first;
-        return it->second;
-    }
     // dense reference layout <-> pitched device layout of a level-l DOF vector (device to device)
     void pitch(const double* src, double* dst, int l, bool toPitched) {
         const dev::LevelView& v = L[size_t(l)].view;
@@ -2139,6 +1928,15 @@ struct SolverImpl {
     void op16(int l, const __half* x, __half* y, float c1, float c2, dev::Ctl ctl, bool own16);
     float* vcycleHalf(dev::Ctl ctl, bool own16, bool firstDone);
     __half* vcycle16(int l, dev::Ctl ctl, bool own16, bool firstDone);
+    // the FP16 V-cycle keeps its coarse vectors in the FP32 ones' storage: an FP32 V-cycle after it starts from
+    // zeros again (the kernels write a level's active nodes only and read inactive ones as 0)
+    bool halfLeft = false;
+    void clearHalf() {
+        if (!halfLeft) return;
+        for (size_t l = 1; l < W.size(); l++)
+            for (DevMem* b : {&W[l].r, &W[l].z, &W[l].t, &W[l].d}) check(cudaMemsetAsync(b->p, 0, b->bytes, stream), "memset");
+        halfLeft = false;
+    }
     float* vcycleFor(bool half, dev::Ctl ctl, bool own16, bool firstDone = false) {
         return half ? vcycleHalf(ctl, own16, firstDone) : vcycle(0, ctl, own16, firstDone);
     }
@@ -2218,7 +2016,7 @@ void SolverImpl::allocate() {
 
 void SolverImpl::op64(int l, const double* xin, double* y, bool raw, dev::Ctl ctl) {
     DevLevel& D = L[size_t(l)];
-    if (!D.nTiles) return;
+    if (!D.nActive) return;
     if (!D.useTiles) {
         if (D.use8)
             launch(dev::k_op8<double, dev::OP_APPLY, false, false>, gridFor(D.view.nNodes * 8, 256, smCount * 32), 256, 0, stream, D.view, D.c64, xin,
@@ -2228,28 +2026,18 @@ void SolverImpl::op64(int l, const double* xin, double* y, bool raw, dev::Ctl ct
                    nullptr, 0.f, 0.f, raw ? 1 : 0, ctl);
         return;
     }
-    dev::TileIO<double> io{0.f, 0.f, raw ? 1 : 0, 0};
-    dev::TileMaps mp;
-    mp.x = mapOf(xin, MAP_HALO, true, l);
-    mp.w = mapOf(D.word.p, MAP_WORDS, false, l);
-    mp.y = mapOf(y, MAP_TILE, true, l);
-    mp.r = mp.d = mp.inv = mp.y;  // not read by this epilogue
-    if (D.inner64) {
-        launch(dev::k_tile<double, dev::TOP_APPLY, false, false, true>, D.nTiles, dev::TILE_THREADS, dev::tileSmemBytes<double, dev::TOP_APPLY, true>(),
-               stream, D.view, D.c64, D.tiles.as<uint32_t>(), mp, io, st(), part(), tick(), ctl);
-        return;
-    }
-    launch(dev::k_tile<double, dev::TOP_APPLY, false, false>, D.nTiles, dev::TILE_THREADS, dev::tileSmemBytes<double, dev::TOP_APPLY, false>(), stream,
-           D.view, D.c64, D.tiles.as<uint32_t>(), mp, io, st(), part(), tick(), ctl);
-    if (D.nBnd)
-        launch(dev::k_bnd<double, dev::TOP_APPLY, false, false>, nodeGrid(D.nBnd), dev::NODE_THREADS, 0, stream, D.view, D.c64,
-               D.blist.as<int>(), D.nBnd, xin, y, nullptr, nullptr, 0.f, 0.f, raw ? 1 : 0, st(), part(), tick(), ctl);
+    const bool split = !D.inner64;
+    launch(dev::k_march<double, dev::TOP_APPLY>, D.nTiles64, dev::marchThreads<double>(), dev::marchSmemBytes<double>(), stream, D.view, D.m64,
+           D.tiles64.as<dev::MarchTile>(), xin, y, nullptr, nullptr, dev::MarchIO{0.f, 0.f, raw ? 1 : 0, 0, D.outBit(split)}, st(), part(), tick(), ctl);
+    if (const int nl = D.listCount(split))
+        launch(dev::k_bnd<double, dev::TOP_APPLY, false, false>, nodeGrid(nl), dev::NODE_THREADS, 0, stream, D.view, D.c64, D.list(split), nl, xin,
+               y, nullptr, nullptr, 0.f, 0.f, raw ? 1 : 0, st(), part(), tick(), ctl);
 }
 
 template <int MODE>
 void SolverImpl::op32(int l, const float* xin, float* y, float c1, float c2, dev::Ctl ctl, bool own16) {
     DevLevel& D = L[size_t(l)];
-    if (!D.nTiles) return;
+    if (!D.nActive) return;
     float* rr = W[size_t(l)].r.as<float>();
     float* dd = W[size_t(l)].d.as<float>();
     if (own16 && D.ebe) {
@@ -2280,7 +2068,8 @@ void SolverImpl::op32(int l, const float* xin, float* y, float c1, float c2, dev
             launch(dev::k_stn<SM_, float, float>, g, 256, 0, stream, D.view, D.stnNodes, D.nStn, D.stn32.as<float>(), 1.f, xin, y, rr, dd, c1, c2,
                    1.f, 0, ctl);
     };
-    const bool stn = l > 0 && !diff && D.nStn > 0 && (s16 ? D.stn16.p != nullptr : D.stn32.p != nullptr);
+    const bool stn = l > 0 && !diff && D.nStn > 0 && (s16 ? D.stn16.p != nullptr : D.stn32.p != nullptr) &&
+                     (!D.useTiles || D.stnNodes == D.list(D.split32));
     if (stn && !D.useTiles) {
         stencilPass();
         return;
@@ -2316,50 +2105,31 @@ void SolverImpl::op32(int l, const float* xin, float* y, float c1, float c2, dev
         else launch(dev::k_op<float, MODE, false>, g, dev::NODE_THREADS, 0, stream, D.view, D.c32, xin, y, rr, dd, c1, c2, 0, ctl);
         return;
     }
-    constexpr int TM = MODE == dev::OP_CHEB ? dev::TOP_CHEB : (MODE == dev::OP_RESID ? dev::TOP_RESID : dev::TOP_APPLY);
-    dev::TileIO<float> io{c1, c2, 0, 0};
-    dev::TileMaps mp;
-    mp.x = mapOf(xin, MAP_HALO, false, l);
-    mp.w = mapOf(D.word.p, MAP_WORDS, false, l);
-    mp.y = mapOf(y, MAP_TILE, false, l);
-    mp.r = dev::tileHasR(TM) ? mapOf(rr, MAP_TILE, false, l) : mp.y;
-    mp.d = dev::tileHasD(TM) ? mapOf(dd, MAP_TILE, false, l) : mp.y;
-    mp.inv = dev::tileHasD(TM) ? mapOf(D.invD.p, MAP_TILE, false, l) : mp.y;
-    const uint32_t* tl = D.tiles.as<uint32_t>();
-    if (D.split32) {
-        // uniform nodes in the tiles, boundary nodes from the list at full occupancy (the tiles
-        // store a boundary node's staged d unchanged, and k_bnd overwrites its d and y)
-        const size_t sm = dev::tileSmemBytes<float, TM, false>();
-        const dev::Coefs<float>& c = D.c32;
-        if (diff) launch(dev::k_tile<float, TM, true, true, false>, D.nTiles, dev::TILE_THREADS, sm, stream, D.view, D.c32, tl, mp, io, st(), part(), tick(), ctl);
-        else if (o16) launch(dev::k_tile<float, TM, true, false, false>, D.nTiles, dev::TILE_THREADS, sm, stream, D.view, D.c32, tl, mp, io, st(), part(), tick(), ctl);
-        else launch(dev::k_tile<float, TM, false, false, false>, D.nTiles, dev::TILE_THREADS, sm, stream, D.view, D.c32, tl, mp, io, st(), part(), tick(), ctl);
-        if (!D.nBnd) return;
-        if (stn) {
-            stencilPass();
-            return;
-        }
-        const int* bl = D.blist.as<int>();
-        if (!diff && D.hasOwn) {
-            // few Galerkin classes: the boundary pass gathers from a shared-memory copy of them
-            const size_t cls = size_t(D.nOwnDev) * 576 * (o16 ? 2 : 4);
-            if (cls <= M->clsSmemMax) {
-                const int gc = std::min(smCount, (D.nBnd + 511) / 512);
-                if (o16) launch(dev::k_list<TM, true, true>, gc, 512, cls, stream, D.view, c, bl, D.nBnd, D.nOwnDev, xin, y, rr, dd, c1, c2, 1.f, 0, ctl);
-                else launch(dev::k_list<TM, false, true>, gc, 512, cls, stream, D.view, c, bl, D.nBnd, D.nOwnDev, xin, y, rr, dd, c1, c2, 1.f, 0, ctl);
-                return;
-            }
-        }
-        const int g = gridFor(D.nBnd, dev::NODE_THREADS, smCount * 16);
-        if (diff) launch(dev::k_bnd<float, TM, true, true>, g, dev::NODE_THREADS, 0, stream, D.view, c, bl, D.nBnd, xin, y, rr, dd, c1, c2, 0, st(), part(), tick(), ctl);
-        else if (o16) launch(dev::k_bnd<float, TM, true, false>, g, dev::NODE_THREADS, 0, stream, D.view, c, bl, D.nBnd, xin, y, rr, dd, c1, c2, 0, st(), part(), tick(), ctl);
-        else launch(dev::k_bnd<float, TM, false, false>, g, dev::NODE_THREADS, 0, stream, D.view, c, bl, D.nBnd, xin, y, rr, dd, c1, c2, 0, st(), part(), tick(), ctl);
+    // marched: the nodes of one scale per voxel; then the list kernels' nodes (those that touch an own matrix)
+    const int* bl = D.list(D.split32);
+    const int nl = D.listCount(D.split32);
+    launch(dev::k_march<float, SM_>, D.nTiles32, dev::marchThreads<float>(), dev::marchSmemBytes<float>(), stream, D.view, D.m32,
+           D.tiles32.as<dev::MarchTile>(), xin, y, rr, dd, dev::MarchIO{c1, c2, 0, 0, D.outBit(D.split32)}, st(), part(), tick(), ctl);
+    if (!nl) return;
+    if (stn) {
+        stencilPass();
         return;
     }
-    const size_t sm = dev::tileSmemBytes<float, TM, true>();
-    if (diff) launch(dev::k_tile<float, TM, true, true>, D.nTiles, dev::TILE_THREADS, sm, stream, D.view, D.c32, tl, mp, io, st(), part(), tick(), ctl);
-    else if (o16) launch(dev::k_tile<float, TM, true, false>, D.nTiles, dev::TILE_THREADS, sm, stream, D.view, D.c32, tl, mp, io, st(), part(), tick(), ctl);
-    else launch(dev::k_tile<float, TM, false, false>, D.nTiles, dev::TILE_THREADS, sm, stream, D.view, D.c32, tl, mp, io, st(), part(), tick(), ctl);
+    const dev::Coefs<float>& c = D.c32;
+    if (!diff && D.hasOwn) {
+        // few Galerkin classes: the list pass gathers from a shared-memory copy of them
+        const size_t cls = size_t(D.nOwnDev) * 576 * (o16 ? 2 : 4);
+        if (cls <= M->clsSmemMax) {
+            const int gc = std::min(smCount, (nl + 511) / 512);
+            if (o16) launch(dev::k_list<SM_, true, true>, gc, 512, cls, stream, D.view, c, bl, nl, D.nOwnDev, xin, y, rr, dd, c1, c2, 1.f, 0, ctl);
+            else launch(dev::k_list<SM_, false, true>, gc, 512, cls, stream, D.view, c, bl, nl, D.nOwnDev, xin, y, rr, dd, c1, c2, 1.f, 0, ctl);
+            return;
+        }
+    }
+    const int g = gridFor(nl, dev::NODE_THREADS, smCount * 16);
+    if (diff) launch(dev::k_bnd<float, SM_, true, true>, g, dev::NODE_THREADS, 0, stream, D.view, c, bl, nl, xin, y, rr, dd, c1, c2, 0, st(), part(), tick(), ctl);
+    else if (o16) launch(dev::k_bnd<float, SM_, true, false>, g, dev::NODE_THREADS, 0, stream, D.view, c, bl, nl, xin, y, rr, dd, c1, c2, 0, st(), part(), tick(), ctl);
+    else launch(dev::k_bnd<float, SM_, false, false>, g, dev::NODE_THREADS, 0, stream, D.view, c, bl, nl, xin, y, rr, dd, c1, c2, 0, st(), part(), tick(), ctl);
 }
 
 // pre-smoothing from zero, residual, restriction, coarse correction, prolongation, post-smoothing
@@ -2655,21 +2425,14 @@ void SolverImpl::recordPlainIteration(dev::Ctl ctl, bool own16) {
         launch(dev::k_apply_alpha<double, false>, nodeGrid(pn(0)), dev::NODE_THREADS, 0, stream, D.view, D.c64, p.as<double>(), q.as<double>(),
                st(), part(), tick(), ctl);
     } else {
-        dev::TileIO<double> io{0.f, 0.f, 0, (D.nBnd && !D.inner64) ? 1 : 0};
-        dev::TileMaps mp;
-        mp.x = mapOf(p.p, MAP_HALO, true, 0);
-        mp.w = mapOf(D.word.p, MAP_WORDS, false, 0);
-        mp.y = mapOf(q.p, MAP_TILE, true, 0);
-        mp.r = mp.d = mp.inv = mp.y;
-        if (D.inner64)
-            launch(dev::k_tile<double, dev::TOP_DOT, false, false, true>, D.nTiles, dev::TILE_THREADS, dev::tileSmemBytes<double, dev::TOP_DOT, true>(),
-                   stream, D.view, D.c64, D.tiles.as<uint32_t>(), mp, io, st(), part(), tick(), ctl);
-        else
-            launch(dev::k_tile<double, dev::TOP_DOT, false, false>, D.nTiles, dev::TILE_THREADS, dev::tileSmemBytes<double, dev::TOP_DOT, false>(),
-                   stream, D.view, D.c64, D.tiles.as<uint32_t>(), mp, io, st(), part(), tick(), ctl);
-        if (D.nBnd && !D.inner64)
-            launch(dev::k_bnd<double, dev::TOP_DOT, false, false>, nodeGrid(D.nBnd), dev::NODE_THREADS, 0, stream, D.view, D.c64,
-                   D.blist.as<int>(), D.nBnd, p.as<double>(), q.as<double>(), nullptr, nullptr, 0.f, 0.f, 0, st(), part(), tick(), ctl);
+        const bool split = !D.inner64;
+        const int nl = D.listCount(split);
+        launch(dev::k_march<double, dev::TOP_DOT>, D.nTiles64, dev::marchThreads<double>(), dev::marchSmemBytes<double>(), stream, D.view, D.m64,
+               D.tiles64.as<dev::MarchTile>(), p.as<double>(), q.as<double>(), nullptr, nullptr, dev::MarchIO{0.f, 0.f, 0, nl ? 1 : 0, D.outBit(split)},
+               st(), part(), tick(), ctl);
+        if (nl)
+            launch(dev::k_bnd<double, dev::TOP_DOT, false, false>, nodeGrid(nl), dev::NODE_THREADS, 0, stream, D.view, D.c64, D.list(split), nl,
+                   p.as<double>(), q.as<double>(), nullptr, nullptr, 0.f, 0.f, 0, st(), part(), tick(), ctl);
     }
     const bool one = exactOneLevel();
     launch(dev::k_cg_update, vecGrid(pn(0)), dev::VEC_THREADS, 0, stream, pn(0), D.view.nmask, x.as<double>(), r.as<double>(), p.as<double>(),
@@ -2699,14 +2462,9 @@ void SolverImpl::recordMixedIteration(dev::Ctl ctl, bool refine, bool half) {
         launch(dev::k_apply_alpha<float, true>, nodeGrid(pn(0)), dev::NODE_THREADS, 0, stream, D.view, D.c32, p32.as<float>(), q32.as<float>(),
                st(), part(), tick(), dev::Ctl{ctl.skipIf, nullptr});
     } else {
-        dev::TileIO<float> io{0.f, 0.f, 0, 0};
-        dev::TileMaps mp;
-        mp.x = mapOf(p32.p, MAP_HALO, false, 0);
-        mp.w = mapOf(D.word.p, MAP_WORDS, false, 0);
-        mp.y = mapOf(q32.p, MAP_TILE, false, 0);
-        mp.r = mp.d = mp.inv = mp.y;
-        launch(dev::k_tile<float, dev::TOP_DOT, false, true>, D.nTiles, dev::TILE_THREADS, dev::tileSmemBytes<float, dev::TOP_DOT, true>(), stream, D.view,
-               D.c32, D.tiles.as<uint32_t>(), mp, io, st(), part(), tick(), dev::Ctl{ctl.skipIf, nullptr});
+        launch(dev::k_march<float, dev::TOP_DOT>, D.nTiles32, dev::marchThreads<float>(), dev::marchSmemBytes<float>(), stream, D.view, D.m32,
+               D.tiles32.as<dev::MarchTile>(), p32.as<float>(), q32.as<float>(), nullptr, nullptr, dev::MarchIO{0.f, 0.f, 0, 0, NM_PLAIN}, st(), part(),
+               tick(), dev::Ctl{ctl.skipIf, nullptr});
     }
     // the fold (u += x32, the FP64 defect as the new r32) is due every few iterations only: it sits
     // in a conditional branch that the update kernel opens, so that iterations without it launch
@@ -2819,7 +2577,9 @@ void SolverImpl::startIterations() {
         check(cudaStreamWaitEvent(stream, M->readyEv, 0), "wait");
         listsWaited = listsWaited || ready;
     }
+    if (!half) clearHalf();
     if (half) {
+        halfLeft = true;
         M->ensureActiveLists();
         check(cudaStreamWaitEvent(stream, M->readyEv, 0), "wait");
         // the list kernels write active nodes only: the FP16 views of the levels' second iterate
@@ -3657,6 +3417,7 @@ void Solver::precondition(const double* rHost, double* zHost) {
     const int64_t n = I.pd(0), nn = I.pn(0);
     I.setDegree(2);  // the reference's preconditioner
     I.prepareSmoothers();
+    I.clearHalf();
     I.uploadPitched(rHost, I.r.as<double>(), 0, I.q.as<double>());
     const dev::Ctl none{nullptr, nullptr};
     if (I.exactOneLevel()) {
