@@ -341,6 +341,8 @@ struct MarchIO {
     int raw;           // APPLY: keep held DOFs
     int partial;       // DOT: leave the step to the list kernel (st->pqPart holds the marched share)
     unsigned outBit;   // the mask bit of the nodes to compute
+    int nTiles;        // DENSE: the tiles of the list, and where x . y goes
+    double* dotOut;
 };
 
 __host__ __device__ constexpr uint32_t packTile(int tx, int ty, int tz) { return uint32_t(tx) | (uint32_t(ty) << 11) | (uint32_t(tz) << 22); }

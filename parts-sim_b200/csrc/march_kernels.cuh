@@ -62,6 +62,7 @@ struct ModeCoefs {
 };
 
 // a tile: its (tx, ty) and the output planes [k0, k1)
+constexpr uint16_t MARCH_EMPTY = 0x8000;  // in tx: no active node (lists over the whole grid)
 struct MarchTile {
     uint16_t tx, ty, k0, k1;
 };
@@ -158,176 +159,197 @@ __device__ __forceinline__ void marchLayer(const ModeCoefs<T>& K, T s, const Fac
 //              (voxel_fea.cpp:902-905); held DOFs of y, where x is 0, are left with K x
 // at the nodes whose mask has the bit `outBit`; the other nodes' y and d are not touched. Held DOFs have
 // x = r = d = 1/diag = 0, so the smoother leaves zeros there.
-template <class T, int MODE>
+// DENSE (TOP_DOT, 64-bit): the caller's vectors instead, in the reference's layout (rows of NX nodes): y is written at
+// every node of the grid (0 at held DOFs and inactive nodes; a tile of the list with MARCH_EMPTY set has only those),
+// x . y goes to io.dotOut, and the CTAs take the tiles in turn.
+template <class T, int MODE, bool DENSE = false>
 __global__ void __launch_bounds__(marchThreads<T>(), 1)
     k_march(LevelView L, ModeCoefs<T> K, const MarchTile* __restrict__ tiles, const T* __restrict__ x, T* __restrict__ y,
             const float* __restrict__ r, float* __restrict__ d, MarchIO io, SolveState* st, double* partials, unsigned* ticket, Ctl ctl) {
     if (skipped(ctl)) return;
     constexpr int ROWS = marchRows<T>(), PLANE = ROWS * MARCH_ROW;
     constexpr bool CHEB = MODE == TOP_CHEB, RESID = MODE == TOP_RESID, DOT = MODE == TOP_DOT, APPLY = MODE == TOP_APPLY;
-    constexpr bool MASKED = RESID || APPLY;  // held DOFs of the result set to 0 by the masks
+    constexpr bool MASKED = RESID || APPLY || DENSE;  // held DOFs of the result set to 0 by the masks
     extern __shared__ __align__(16) unsigned char marchSmem[];
     T* ring = reinterpret_cast<T*>(marchSmem);                       // [STAGES][ROWS][96]
     T* sums = ring + MARCH_STAGES * PLANE;                           // [2][own row, share of the next row][ROWS][96]
     unsigned* bits = reinterpret_cast<unsigned*>(sums + 4 * PLANE);  // [BITS][ROWS]
-    const MarchTile tile = tiles[blockIdx.x];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int k0 = tile.k0, k1 = tile.k1;
-    const int i = MARCH_NX * int(tile.tx) - 1 + lane;      // the lane's node and voxel along x
-    const int j = marchNY<T>() * int(tile.ty) - 1 + warp;  // the warp's node row
-    const long long PXY = (long long)L.PX * L.NY, WXY = (long long)L.px * L.ny;  // node and word planes
-    const bool nodeIn = i >= 0 && i < L.NX && j >= 0 && j < L.NY, nextIn = i >= 0 && i < L.NX && j + 1 >= 0 && j + 1 < L.NY;
-    // the last lane's and the last row's voxels lack a corner: they count as empty (and shape halo nodes only)
-    const bool voxIn = i >= 0 && i < L.nx && lane < 31 && j >= 0 && j < L.ny && warp < ROWS - 1;
-    const bool outRow = warp > 0 && warp < ROWS - 1;
-    // offsets within a plane: the lane's node, its voxel, and the row's value `lane` in DOF order; the row's values
-    // lane + 32 q belong to the nodes at bits mq[q]
-    const int nodeAt = i + L.PX * j, wordAt = i + L.px * j, valueAt = 3 * (nodeAt - lane) + lane;
-    unsigned mq[3];
-#pragma unroll
-    for (int q = 0; q < 3; q++) mq[q] = 1u << ((lane + 32 * q) / 3);
-    auto maskAt = [&](bool in, int at, int k) -> unsigned {  // of a node of plane k, 0 outside the grid
-        const uint8_t* m = L.nmask + k * PXY;
-        return (in && unsigned(k) < unsigned(L.NZ)) ? unsigned(__ldg(m + at)) : 0u;
-    };
-    auto stage = [&](int k, unsigned mk) {
-        T* dst = ring + ((k + 1) & (MARCH_STAGES - 1)) * PLANE + warp * MARCH_ROW + lane;
-        const unsigned act = __ballot_sync(0xffffffffu, mk & NM_ACTIVE), out = __ballot_sync(0xffffffffu, mk & io.outBit);
-        if (lane == 0) bits[((k + 1) & (MARCH_BITS - 1)) * ROWS + warp] = (outRow && k >= k0 && k < k1) ? out & 0x7ffffffeu : 0u;
-        const T* src = x + 3 * k * PXY + valueAt;  // (read at the active nodes only)
-#pragma unroll
-        for (int q = 0; q < 3; q++) cpAsyncOr0(dst + 32 * q, src + 32 * q, act & mq[q]);
-        cpAsyncCommit();
-    };
-
-    T F[3][4] = {};
-    float er[3], ed[3], ei[3];  // epilogue operands of the plane being completed, loaded a step ahead
-    unsigned eb = 0, mkNext;
-    uint32_t wNext = 0;  // the voxel word above the plane, a step ahead; used as loaded only then
     double dot = 0.0;
-
-    // the finished sums of plane k (in shared memory) through the epilogue
-    auto finish = [&](int k) {
-        const T* sm = sums + ((k + 1) & 1) * 2 * PLANE + warp * MARCH_ROW + lane;
-        const T* own = ring + ((k + 1) & (MARCH_STAGES - 1)) * PLANE + warp * MARCH_ROW + lane;
-        T kx[3], xv[3];
+    // (one tile a CTA, or, DENSE, every gridDim.x-th)
+    for (unsigned tileAt = blockIdx.x; tileAt == blockIdx.x || (DENSE && tileAt < unsigned(io.nTiles)); tileAt += gridDim.x) {
+        if (DENSE) __syncthreads();  // the tile before is done with the shared memory
+        const MarchTile tile = tiles[tileAt];
+        const int k0 = tile.k0, k1 = tile.k1;
+        const int i = MARCH_NX * int(tile.tx & ~MARCH_EMPTY) - 1 + lane;      // the lane's node and voxel along x
+        const int j = marchNY<T>() * int(tile.ty) - 1 + warp;  // the warp's node row
+        const int XROW = DENSE ? L.NX : L.PX;  // the vectors' row pitch
+        const long long PXY = (long long)L.PX * L.NY, XXY = (long long)XROW * L.NY, WXY = (long long)L.px * L.ny;  // mask, vector and word planes
+        const bool nodeIn = i >= 0 && i < L.NX && j >= 0 && j < L.NY, nextIn = i >= 0 && i < L.NX && j + 1 >= 0 && j + 1 < L.NY;
+        // the last lane's and the last row's voxels lack a corner: they count as empty (and shape halo nodes only)
+        const bool voxIn = i >= 0 && i < L.nx && lane < 31 && j >= 0 && j < L.ny && warp < ROWS - 1;
+        const bool outRow = warp > 0 && warp < ROWS - 1;
+        // offsets within a plane: the lane's node, its voxel, and the row's value `lane` in DOF order; the row's values
+        // lane + 32 q belong to the nodes at bits mq[q]
+        const int nodeAt = i + L.PX * j, wordAt = i + L.px * j, valueAt = 3 * (i - lane + XROW * j) + lane;
+        unsigned mq[3];
 #pragma unroll
-        for (int q = 0; q < 3; q++) {
-            kx[q] = sm[32 * q];
-            xv[q] = own[32 * q];
-        }
-        if (warp > 0)
+        for (int q = 0; q < 3; q++) mq[q] = 1u << ((lane + 32 * q) / 3);
+        auto maskAt = [&](bool in, int at, int k) -> unsigned {  // of a node of plane k, 0 outside the grid
+            const uint8_t* m = L.nmask + k * PXY;
+            return (in && unsigned(k) < unsigned(L.NZ)) ? unsigned(__ldg(m + at)) : 0u;
+        };
+        auto stage = [&](int k, unsigned mk) {
+            T* dst = ring + ((k + 1) & (MARCH_STAGES - 1)) * PLANE + warp * MARCH_ROW + lane;
+            const unsigned act = __ballot_sync(0xffffffffu, mk & NM_ACTIVE), out = __ballot_sync(0xffffffffu, DENSE ? nodeIn : (mk & io.outBit) != 0);
+            if (lane == 0) bits[((k + 1) & (MARCH_BITS - 1)) * ROWS + warp] = (outRow && k >= k0 && k < k1) ? out & 0x7ffffffeu : 0u;
+            const T* src = x + 3 * k * XXY + valueAt;  // (read at the active nodes only)
 #pragma unroll
-            for (int q = 0; q < 3; q++) kx[q] += sm[PLANE - MARCH_ROW + 32 * q];  // the warp below's share
-        if (L.dadd) {
-#pragma unroll
-            for (int q = 0; q < 3; q++)
-                if (eb & mq[q]) {
-                    const long long id = 3 * k * PXY + valueAt + 32 * q, n = id / 3;
-                    // (a held DOF keeps its 0: x is 0 there in every mode but APPLY)
-                    if (!(APPLY && !io.raw && fixedDof(__ldg(L.nmask + n), int(id - 3 * n))))
-                        kx[q] += (sizeof(T) == 8 ? T(L.dadd[id]) : T(L.dadd32[id])) * xv[q];
-                }
-        }
-        T* yr = y + 3 * k * PXY + valueAt;
-        float* dr = d + 3 * k * PXY + valueAt;
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            const bool p = eb & mq[q];
-            if constexpr (CHEB) {
-                const float dn = io.c1 * ed[q] + io.c2 * ei[q] * (er[q] - float(kx[q]));
-                if (p) dr[32 * q] = dn;
-                if (p) yr[32 * q] = xv[q] + T(dn);
-            } else if constexpr (RESID) {
-                if (p) yr[32 * q] = T(er[q]) - kx[q];
-            } else {
-                if (p) yr[32 * q] = kx[q];
-                if (DOT && p) dot += double(xv[q]) * double(kx[q]);
-            }
-        }
-    };
-
-    // planes k0 - 1 .. k1, PREFETCH of them in flight
-#pragma unroll
-    for (int p = 0; p < MARCH_PREFETCH; p++) stage(k0 - 1 + p, maskAt(nodeIn, nodeAt, k0 - 1 + p));
-    mkNext = maskAt(nodeIn, nodeAt, k0 - 1 + MARCH_PREFETCH);
-    FaceModes<T> P, Q;  // the modes of planes k - 1 and k
-    for (int k = k0 - 1; k <= k1; k++) {
-        cpAsyncWait<MARCH_PREFETCH - 1>();
-        __syncthreads();
-        if (k > k0 + 1) finish(k - 2);
-        __syncwarp();
-        if (k + MARCH_PREFETCH <= k1) {  // into the slot of plane k - 2, whose last reader was this warp, just now
-            stage(k + MARCH_PREFETCH, mkNext);
-            mkNext = maskAt(nodeIn, nodeAt, k + MARCH_PREFETCH + 1);
-        } else {
+            for (int q = 0; q < 3; q++) cpAsyncOr0(dst + 32 * q, src + 32 * q, act & mq[q]);
             cpAsyncCommit();
-        }
-        unsigned hold = 0, holdNext = 0;  // the masks of the warp's own row and the next, plane k - 1
-        if (k > k0) {
-            eb = bits[(k & (MARCH_BITS - 1)) * ROWS + warp];
-            const long long at = 3 * (k - 1) * PXY + valueAt;
-            if (CHEB || RESID)
+        };
+
+        T F[3][4] = {};
+        float er[3], ed[3], ei[3];  // epilogue operands of the plane being completed, loaded a step ahead
+        unsigned eb = 0, mkNext;
+        uint32_t wNext = 0;  // the voxel word above the plane, a step ahead; used as loaded only then
+
+        // the finished sums of plane k (in shared memory) through the epilogue
+        auto finish = [&](int k) {
+            const T* sm = sums + ((k + 1) & 1) * 2 * PLANE + warp * MARCH_ROW + lane;
+            const T* own = ring + ((k + 1) & (MARCH_STAGES - 1)) * PLANE + warp * MARCH_ROW + lane;
+            T kx[3], xv[3];
 #pragma unroll
-                for (int q = 0; q < 3; q++)
-                    if (eb & mq[q]) er[q] = __ldg(r + at + 32 * q);
-            if (CHEB) {
-#pragma unroll
-                for (int q = 0; q < 3; q++)
-                    if (eb & mq[q]) ed[q] = d[at + 32 * q];
-#pragma unroll
-                for (int q = 0; q < 3; q++)
-                    if (eb & mq[q]) ei[q] = __ldg(L.invD + at + 32 * q);
+            for (int q = 0; q < 3; q++) {
+                kx[q] = sm[32 * q];
+                xv[q] = own[32 * q];
             }
-            if (MASKED && !io.raw) {
-                hold = maskAt(nodeIn, nodeAt, k - 1);
-                holdNext = maskAt(nextIn, nodeAt + L.PX, k - 1);
-            }
-        }
-        const T s = T(fmaxf(__uint_as_float(wNext), 0.f));  // of the layer below (an own matrix's word is a negative float or NaN: 0)
-        if (k < k1) wNext = (voxIn && unsigned(k) < unsigned(L.nz)) ? __ldg(L.word + k * WXY + wordAt) : 0u;
-        const T* pl = ring + ((k + 1) & (MARCH_STAGES - 1)) * PLANE + warp * MARCH_ROW + 3 * lane;
-        const int right = lane < 31 ? 3 : 0, up = warp < ROWS - 1 ? MARCH_ROW : 0;
+            if (warp > 0)
 #pragma unroll
-        for (int c = 0; c < 3; c++) Q.make(c, pl[c], pl[c + right], pl[up + c], pl[up + c + right]);
-        if (k >= k0) {
-            T G[3][4];
-            if (sizeof(T) == 4 || s != T(0)) {
-                marchLayer<T>(K, s, P, Q, F, G);
-            } else {  // an empty voxel (64-bit: whatever x holds at its corners, infinities too, stays out)
+                for (int q = 0; q < 3; q++) kx[q] += sm[PLANE - MARCH_ROW + 32 * q];  // the warp below's share
+            if (L.dadd) {
 #pragma unroll
-                for (int c = 0; c < 3; c++)
-#pragma unroll
-                    for (int m = 0; m < 4; m++) {
-                        G[c][m] = F[c][m];
-                        F[c][m] = T(0);
+                for (int q = 0; q < 3; q++)
+                    if (eb & mq[q]) {
+                        const long long id = 3 * (k * PXY + nodeAt - lane) + lane + 32 * q, n = id / 3;  // (pitched)
+                        // (a held DOF keeps its 0: the solver's x is 0 there)
+                        if (!((APPLY || DENSE) && !io.raw && fixedDof(__ldg(L.nmask + n), int(id - 3 * n))))
+                            kx[q] += (sizeof(T) == 8 ? T(L.dadd[id]) : T(L.dadd32[id])) * xv[q];
                     }
             }
-            if (k > k0) {
-                // plane k - 1 back to its nodes: x neighbours by shuffles, the next row's share to its warp
-                T* sm = sums + (k & 1) * 2 * PLANE + warp * MARCH_ROW + 3 * lane;
+            T* yr = y + 3 * k * XXY + valueAt;
+            float* dr = d + 3 * k * XXY + valueAt;
 #pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    const T s0 = G[c][0] - G[c][2], s1 = G[c][0] + G[c][2], t0 = G[c][1] - G[c][3], t1 = G[c][1] + G[c][3];
-                    T own = s0 - t0 + __shfl_up_sync(0xffffffffu, s0 + t0, 1);
-                    T next = s1 - t1 + __shfl_up_sync(0xffffffffu, s1 + t1, 1);
-                    if (MASKED && !io.raw && ((hold >> c) & 1u)) own = T(0);
-                    if (MASKED && !io.raw && ((holdNext >> c) & 1u)) next = T(0);
-                    sm[c] = own;
-                    sm[PLANE + c] = next;
+            for (int q = 0; q < 3; q++) {
+                const bool p = eb & mq[q];
+                if constexpr (CHEB) {
+                    const float dn = io.c1 * ed[q] + io.c2 * ei[q] * (er[q] - float(kx[q]));
+                    if (p) dr[32 * q] = dn;
+                    if (p) yr[32 * q] = xv[q] + T(dn);
+                } else if constexpr (RESID) {
+                    if (p) yr[32 * q] = T(er[q]) - kx[q];
+                } else {
+                    if (p) yr[32 * q] = kx[q];
+                    if (DOT && p) dot += double(xv[q]) * double(kx[q]);
                 }
             }
+        };
+
+        if (DENSE && (tile.tx & MARCH_EMPTY)) {  // no active node: zeros
+            if (outRow && j < L.NY)
+                for (int k = k0; k < k1; k++)
+#pragma unroll
+                    for (int q = 0; q < 3; q++)
+                        if (__ballot_sync(0xffffffffu, nodeIn) & 0x7ffffffeu & mq[q]) y[3 * k * XXY + valueAt + 32 * q] = T(0);
+            continue;
         }
-        P = Q;
+
+        // planes k0 - 1 .. k1, PREFETCH of them in flight
+#pragma unroll
+        for (int p = 0; p < MARCH_PREFETCH; p++) stage(k0 - 1 + p, maskAt(nodeIn, nodeAt, k0 - 1 + p));
+        mkNext = maskAt(nodeIn, nodeAt, k0 - 1 + MARCH_PREFETCH);
+        FaceModes<T> P, Q;  // the modes of planes k - 1 and k
+        for (int k = k0 - 1; k <= k1; k++) {
+            cpAsyncWait<MARCH_PREFETCH - 1>();
+            __syncthreads();
+            if (k > k0 + 1) finish(k - 2);
+            __syncwarp();
+            if (k + MARCH_PREFETCH <= k1) {  // into the slot of plane k - 2, whose last reader was this warp, just now
+                stage(k + MARCH_PREFETCH, mkNext);
+                mkNext = maskAt(nodeIn, nodeAt, k + MARCH_PREFETCH + 1);
+            } else {
+                cpAsyncCommit();
+            }
+            unsigned hold = 0, holdNext = 0;  // the masks of the warp's own row and the next, plane k - 1
+            if (k > k0) {
+                eb = bits[(k & (MARCH_BITS - 1)) * ROWS + warp];
+                const long long at = 3 * (k - 1) * XXY + valueAt;
+                if (CHEB || RESID)
+#pragma unroll
+                    for (int q = 0; q < 3; q++)
+                        if (eb & mq[q]) er[q] = __ldg(r + at + 32 * q);
+                if (CHEB) {
+#pragma unroll
+                    for (int q = 0; q < 3; q++)
+                        if (eb & mq[q]) ed[q] = d[at + 32 * q];
+#pragma unroll
+                    for (int q = 0; q < 3; q++)
+                        if (eb & mq[q]) ei[q] = __ldg(L.invD + at + 32 * q);
+                }
+                if (MASKED && !io.raw) {
+                    hold = maskAt(nodeIn, nodeAt, k - 1);
+                    holdNext = maskAt(nextIn, nodeAt + L.PX, k - 1);
+                }
+            }
+            const T s = T(fmaxf(__uint_as_float(wNext), 0.f));  // of the layer below (an own matrix's word is a negative float or NaN: 0)
+            if (k < k1) wNext = (voxIn && unsigned(k) < unsigned(L.nz)) ? __ldg(L.word + k * WXY + wordAt) : 0u;
+            const T* pl = ring + ((k + 1) & (MARCH_STAGES - 1)) * PLANE + warp * MARCH_ROW + 3 * lane;
+            const int right = lane < 31 ? 3 : 0, up = warp < ROWS - 1 ? MARCH_ROW : 0;
+#pragma unroll
+            for (int c = 0; c < 3; c++) Q.make(c, pl[c], pl[c + right], pl[up + c], pl[up + c + right]);
+            if (k >= k0) {
+                T G[3][4];
+                if (sizeof(T) == 4 || s != T(0)) {
+                    marchLayer<T>(K, s, P, Q, F, G);
+                } else {  // an empty voxel (64-bit: whatever x holds at its corners, infinities too, stays out)
+#pragma unroll
+                    for (int c = 0; c < 3; c++)
+#pragma unroll
+                        for (int m = 0; m < 4; m++) {
+                            G[c][m] = F[c][m];
+                            F[c][m] = T(0);
+                        }
+                }
+                if (k > k0) {
+                    // plane k - 1 back to its nodes: x neighbours by shuffles, the next row's share to its warp
+                    T* sm = sums + (k & 1) * 2 * PLANE + warp * MARCH_ROW + 3 * lane;
+#pragma unroll
+                    for (int c = 0; c < 3; c++) {
+                        const T s0 = G[c][0] - G[c][2], s1 = G[c][0] + G[c][2], t0 = G[c][1] - G[c][3], t1 = G[c][1] + G[c][3];
+                        T own = s0 - t0 + __shfl_up_sync(0xffffffffu, s0 + t0, 1);
+                        T next = s1 - t1 + __shfl_up_sync(0xffffffffu, s1 + t1, 1);
+                        if (MASKED && !io.raw && ((hold >> c) & 1u)) own = T(0);
+                        if (MASKED && !io.raw && ((holdNext >> c) & 1u)) next = T(0);
+                        sm[c] = own;
+                        sm[PLANE + c] = next;
+                    }
+                }
+            }
+            P = Q;
+        }
+        cpAsyncWait<0>();
+        __syncthreads();
+        finish(k1 - 1);
     }
-    cpAsyncWait<0>();
-    __syncthreads();
-    finish(k1 - 1);
     if (DOT) {
         double vv[1] = {dot};
         double tot[1];
         if (gridReduce<1>(vv, 0u, partials, ticket, tot) && threadIdx.x == 0) {
             const double pq = tot[0];
+            if (DENSE) {
+                *io.dotOut = pq;
+                return;
+            }
             if (io.partial) {  // the list kernel adds its share and finishes the step
                 st->pqPart = pq;
                 return;

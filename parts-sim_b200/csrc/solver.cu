@@ -1253,8 +1253,9 @@ dev::ModeCoefs<T> marchCoefs(const double Kb[576], bool& ok) {
 // The tiles of a marched level: columns of 30 x ny nodes cut into chunks of planes, trimmed to the planes with an
 // active node. A CTA of n planes takes about n + 4 steps (one plane of halo below and above, two to fill and
 // drain), so the chunk length is the one with the least waves x steps on `slots` resident CTAs: long chunks where
-// the level has many columns, short ones where it would leave SMs idle.
-std::vector<dev::MarchTile> marchTiles(const HostLevel& h, int ny, int slots) {
+// the level has many columns, short ones where it would leave SMs idle. whole: every column and plane, untrimmed, the
+// chunks without an active node marked.
+std::vector<dev::MarchTile> marchTiles(const HostLevel& h, int ny, int slots, bool whole = false) {
     const int ntx = (h.NX + dev::MARCH_NX - 1) / dev::MARCH_NX, nty = (h.NY + ny - 1) / ny;
     const size_t cols = size_t(ntx) * nty;
     std::vector<uint8_t> act(cols * h.NZ, 0);  // [k][ty][tx]
@@ -1290,7 +1291,8 @@ std::vector<dev::MarchTile> marchTiles(const HostLevel& h, int ny, int slots) {
                     if (lo < 0) lo = k;
                     hi = k + 1;
                 }
-            if (lo >= 0) out.push_back({uint16_t(c % ntx), uint16_t(c / ntx), uint16_t(lo), uint16_t(hi)});
+            if (whole) out.push_back({uint16_t(size_t(c % ntx) | (lo < 0 ? dev::MARCH_EMPTY : 0)), uint16_t(c / ntx), uint16_t(kz), uint16_t(std::min(h.NZ, kz + best))});
+            else if (lo >= 0) out.push_back({uint16_t(c % ntx), uint16_t(c / ntx), uint16_t(lo), uint16_t(hi)});
         }
     return out;
 }
@@ -1305,6 +1307,8 @@ struct DevLevel {
     DevMem word, nmask, own, own16, invD, dadd, dadd32, bc;
     DevMem tiles32, tiles64;  // marched levels: the 32- and 64-bit tiles with an active node
     int nTiles32 = 0, nTiles64 = 0;
+    DevMem tilesAll;          // the finest level: 64-bit tiles over the whole grid (the allocation-free product)
+    int nTilesAll = 0;
     int nActive = 0;   // active nodes
     // marched levels: the boundary nodes (active, not uniform) and those of them that touch an own
     // matrix (pitched indices, increasing); the marching kernel leaves one of the two lists out
@@ -1333,7 +1337,7 @@ struct DevLevel {
     DevMem stn32, stn16;
     float stnScale = 1.f;
     void release() {
-        for (DevMem* b : {&word, &nmask, &own, &own16, &invD, &dadd, &dadd32, &bc, &tiles32, &tiles64, &blist, &olist, &ebeTiles, &stn32, &stn16}) b->release();
+        for (DevMem* b : {&word, &nmask, &own, &own16, &invD, &dadd, &dadd32, &bc, &tiles32, &tiles64, &tilesAll, &blist, &olist, &ebeTiles, &stn32, &stn16}) b->release();
     }
 };
 
@@ -1474,6 +1478,7 @@ void SharedModel::adopt(Hierarchy&& h) {
         };
         set(dev::k_march<double, dev::TOP_APPLY>, dev::marchSmemBytes<double>());
         set(dev::k_march<double, dev::TOP_DOT>, dev::marchSmemBytes<double>());
+        set(dev::k_march<double, dev::TOP_DOT, true>, dev::marchSmemBytes<double>());
         set(dev::k_march<float, dev::TOP_APPLY>, dev::marchSmemBytes<float>());
         set(dev::k_march<float, dev::TOP_CHEB>, dev::marchSmemBytes<float>());
         set(dev::k_march<float, dev::TOP_RESID>, dev::marchSmemBytes<float>());
@@ -1645,6 +1650,11 @@ void SharedModel::uploadLevel(int l) {
         if (const char* e = std::getenv("PSFEA_TILE_MIN_NODES")) minNodes = std::atoll(e);
         D.m64 = marchCoefs<double>(h.Kb, D.useTiles);
         D.m32 = marchCoefs<float>(h.Kb, D.useTiles);
+        if (l == 0 && D.useTiles) {
+            const std::vector<dev::MarchTile> ta = marchTiles(h, dev::marchNY<double>(), smCount, true);
+            D.nTilesAll = int(ta.size());
+            upload(D.tilesAll, ta, bytes, ms);
+        }
         D.useTiles = D.useTiles && h.nNodes >= minNodes;
         int64_t max8 = 30000;
         if (const char* e = std::getenv("PSFEA_OP8_MAX_NODES")) max8 = std::atoll(e);
@@ -2028,7 +2038,7 @@ void SolverImpl::op64(int l, const double* xin, double* y, bool raw, dev::Ctl ct
     }
     const bool split = !D.inner64;
     launch(dev::k_march<double, dev::TOP_APPLY>, D.nTiles64, dev::marchThreads<double>(), dev::marchSmemBytes<double>(), stream, D.view, D.m64,
-           D.tiles64.as<dev::MarchTile>(), xin, y, nullptr, nullptr, dev::MarchIO{0.f, 0.f, raw ? 1 : 0, 0, D.outBit(split)}, st(), part(), tick(), ctl);
+           D.tiles64.as<dev::MarchTile>(), xin, y, nullptr, nullptr, dev::MarchIO{0.f, 0.f, raw ? 1 : 0, 0, D.outBit(split), 0, nullptr}, st(), part(), tick(), ctl);
     if (const int nl = D.listCount(split))
         launch(dev::k_bnd<double, dev::TOP_APPLY, false, false>, nodeGrid(nl), dev::NODE_THREADS, 0, stream, D.view, D.c64, D.list(split), nl, xin,
                y, nullptr, nullptr, 0.f, 0.f, raw ? 1 : 0, st(), part(), tick(), ctl);
@@ -2109,7 +2119,7 @@ void SolverImpl::op32(int l, const float* xin, float* y, float c1, float c2, dev
     const int* bl = D.list(D.split32);
     const int nl = D.listCount(D.split32);
     launch(dev::k_march<float, SM_>, D.nTiles32, dev::marchThreads<float>(), dev::marchSmemBytes<float>(), stream, D.view, D.m32,
-           D.tiles32.as<dev::MarchTile>(), xin, y, rr, dd, dev::MarchIO{c1, c2, 0, 0, D.outBit(D.split32)}, st(), part(), tick(), ctl);
+           D.tiles32.as<dev::MarchTile>(), xin, y, rr, dd, dev::MarchIO{c1, c2, 0, 0, D.outBit(D.split32), 0, nullptr}, st(), part(), tick(), ctl);
     if (!nl) return;
     if (stn) {
         stencilPass();
@@ -2428,7 +2438,7 @@ void SolverImpl::recordPlainIteration(dev::Ctl ctl, bool own16) {
         const bool split = !D.inner64;
         const int nl = D.listCount(split);
         launch(dev::k_march<double, dev::TOP_DOT>, D.nTiles64, dev::marchThreads<double>(), dev::marchSmemBytes<double>(), stream, D.view, D.m64,
-               D.tiles64.as<dev::MarchTile>(), p.as<double>(), q.as<double>(), nullptr, nullptr, dev::MarchIO{0.f, 0.f, 0, nl ? 1 : 0, D.outBit(split)},
+               D.tiles64.as<dev::MarchTile>(), p.as<double>(), q.as<double>(), nullptr, nullptr, dev::MarchIO{0.f, 0.f, 0, nl ? 1 : 0, D.outBit(split), 0, nullptr},
                st(), part(), tick(), ctl);
         if (nl)
             launch(dev::k_bnd<double, dev::TOP_DOT, false, false>, nodeGrid(nl), dev::NODE_THREADS, 0, stream, D.view, D.c64, D.list(split), nl,
@@ -2463,7 +2473,7 @@ void SolverImpl::recordMixedIteration(dev::Ctl ctl, bool refine, bool half) {
                st(), part(), tick(), dev::Ctl{ctl.skipIf, nullptr});
     } else {
         launch(dev::k_march<float, dev::TOP_DOT>, D.nTiles32, dev::marchThreads<float>(), dev::marchSmemBytes<float>(), stream, D.view, D.m32,
-               D.tiles32.as<dev::MarchTile>(), p32.as<float>(), q32.as<float>(), nullptr, nullptr, dev::MarchIO{0.f, 0.f, 0, 0, NM_PLAIN}, st(), part(),
+               D.tiles32.as<dev::MarchTile>(), p32.as<float>(), q32.as<float>(), nullptr, nullptr, dev::MarchIO{0.f, 0.f, 0, 0, NM_PLAIN, 0, nullptr}, st(), part(),
                tick(), dev::Ctl{ctl.skipIf, nullptr});
     }
     // the fold (u += x32, the FP64 defect as the new r32) is due every few iterations only: it sits
@@ -3687,45 +3697,13 @@ void Solver::reactions(const double* u, const double* f, double R[3]) {
 // cannot afford the implicit device synchronisation a cudaMalloc may cause. y = K x and x.y on the
 // finest level with the reduction's scratch (per-block partial sums and the last-block ticket) in
 // this file-scope device array instead of handle-owned or newly allocated memory. Its size caps the
-// kernel's grid at NOALLOC_BLOCKS blocks (grid-stride, so any model size fits); a device whose
+// kernel's grid at NOALLOC_BLOCKS blocks (they take the tiles in turn, so any model size fits); a device whose
 // launch shape would need more is refused. Every call on a device shares the array: calls that
 // overlap on the GPU race, and each call clears the ticket before use.
 
 constexpr int NOALLOC_BLOCKS = 4096;
 constexpr size_t NOALLOC_BYTES = 256 + size_t(NOALLOC_BLOCKS) * sizeof(double);  // ticket line + partials
 static __device__ __align__(256) unsigned char g_noallocScratch[NOALLOC_BYTES];
-
-namespace dev {
-
-// q = K p (FP64, held DOFs 0) and p.q into *dot, the reduction scratch in g_noallocScratch
-__global__ void __launch_bounds__(NODE_THREADS) k_apply_dot_static(LevelView L, Coefs<double> C, const double* __restrict__ p,
-                                                                   double* __restrict__ q, double* __restrict__ dot,
-                                                                   unsigned char* scratch) {
-    // p and q are the caller's vectors in the reference's dense layout (node nd = i + NX (j + NY k));
-    // masks, words and the diagonal shift are the level's pitched arrays
-    double v[1] = {0.0};
-    const long long nDense = (long long)L.NX * L.NY * L.NZ;
-    for (long long nd = blockIdx.x * (long long)blockDim.x + threadIdx.x; nd < nDense; nd += (long long)gridDim.x * blockDim.x) {
-        const long long row = nd / L.NX;
-        const int i = int(nd - row * L.NX), j = int(row % L.NY), k = int(row / L.NY);
-        const long long n = i + (long long)L.PX * row;
-        const uint8_t mask = __ldg(L.nmask + n);
-        double acc[3];
-        applyAt<double, false>(L, C, p, i, j, k, nd, mask, acc, L.NX, n);
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-            const double y = fixedDof(mask, c) ? 0.0 : acc[c];
-            q[3 * nd + c] = y;
-            v[0] += p[3 * nd + c] * y;
-        }
-    }
-    unsigned* ticket = reinterpret_cast<unsigned*>(scratch);
-    double* partials = reinterpret_cast<double*>(scratch + 256);
-    double tot[1];
-    if (gridReduce<1>(v, 0u, partials, ticket, tot) && threadIdx.x == 0) *dot = tot[0];
-}
-
-}  // namespace dev
 
 namespace {
 
@@ -3749,9 +3727,8 @@ unsigned char* noallocScratch(int devId) {
 
 void Solver::applyDotStatic(const double* xDev, double* yDev, double* dotDev, void* s) {
     SolverImpl& I = *impl_;
-    const HostLevel& h = I.H.levels[0];
     DevLevel& D = I.L[0];
-    const int grid = I.nodeGrid(h.nNodes);
+    const int grid = std::min(D.nTilesAll, I.smCount * 16);
     if (grid > NOALLOC_BLOCKS)
         throw Error(PS_EINVAL, "this device needs " + std::to_string(grid) + " reduction blocks; the static scratch holds " +
                                    std::to_string(NOALLOC_BLOCKS));
@@ -3765,7 +3742,10 @@ void Solver::applyDotStatic(const double* xDev, double* yDev, double* dotDev, vo
     if (st != I.stream) check(cudaStreamWaitEvent(st, I.M->readyEv, 0), "wait for the model");
     unsigned char* scratch = noallocScratch(cur);
     check(cudaMemsetAsync(scratch, 0, 256, st), "ticket clear");
-    I.launch(dev::k_apply_dot_static, grid, dev::NODE_THREADS, 0, st, D.view, D.c64, xDev, yDev, dotDev, scratch);
+    I.launch(dev::k_march<double, dev::TOP_DOT, true>, grid, dev::marchThreads<double>(), dev::marchSmemBytes<double>(), st, D.view, D.m64,
+             D.tilesAll.as<dev::MarchTile>(), xDev, yDev, static_cast<const float*>(nullptr), static_cast<float*>(nullptr), dev::MarchIO{0.f, 0.f, 0, 0, 0u, D.nTilesAll, dotDev},
+             static_cast<dev::SolveState*>(nullptr), reinterpret_cast<double*>(scratch + 256), reinterpret_cast<unsigned*>(scratch),
+             dev::Ctl{nullptr, nullptr});
     check(cudaGetLastError(), "apply_dot_static");
 }
 

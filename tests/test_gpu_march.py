@@ -3,6 +3,7 @@ product and against the one-thread-per-node operator, at the sizes where its til
 end, forced onto every level whatever its size (PSFEA_TILE_MIN_NODES=0)."""
 import numpy as np
 import pytest
+import torch
 
 import oracle
 import psfea
@@ -48,6 +49,14 @@ def test_product_matches_the_oracle(monkeypatch, dims, empty):
         x = rng.standard_normal(bc.size)
         for raw in (False, True):
             assert rel(S.apply(x, raw=raw), P.apply(x, raw=raw)) < 1e-12, (shift is None, raw)
+        # the allocation-free product on the caller's dense vectors: the same y, 0 at held DOFs and off the part, and x . y
+        y0 = P.apply(x)
+        xd, yd, dd = torch.from_numpy(x).cuda(), torch.full((x.size,), float("nan"), dtype=torch.float64, device="cuda"), torch.zeros(1, dtype=torch.float64, device="cuda")
+        for _ in range(2):
+            S.apply_dot_noalloc(xd.data_ptr(), yd.data_ptr(), dd.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert rel(yd.cpu().numpy(), y0) < 1e-12
+        assert np.all(yd.cpu().numpy()[P.fixed(0) != 0] == 0)
+        assert abs(float(dd[0]) - float(x @ y0)) < 1e-12 * float(np.abs(x * y0).sum())
 
 
 def blocky(dims, seed):
