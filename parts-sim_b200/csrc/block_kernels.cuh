@@ -224,7 +224,8 @@ __device__ __forceinline__ void applyNbr(const LevelView& L, const Coefs<T>& C, 
 //   BOP_CHEB   d = c1 d + c2 D^-1 (r - K x); y = x + d        (Chebyshev / Jacobi step, 32-bit)
 //   BOP_RESID  y = r - K x
 //   BOP_DOT    y = K x (held 0) and each right-hand side's CG step alpha = rz / (x . y); x . y <= 0
-//              ends that right-hand side as a breakdown (voxel_fea.cpp:902-905)
+//              ends that right-hand side as a breakdown (voxel_fea.cpp:902-905); finest level only
+// On the finest level block_march.cuh makes these passes; kb_op makes the first three below it.
 // The product is the single-vector one (applyAt, voxel_fea.cpp:422-486) with the block's stride.
 // The block path's assembled stencils are node-major: node t's row at t * STN_ROW holds its 27 3x3
 // blocks with the neighbours taken in pairs (m, m + 1) = (2 P, 2 P + 1), P = 0..13 (m = (ox + 1) +
@@ -278,23 +279,22 @@ __device__ __forceinline__ void stnBlock(const LevelView& L, const T* __restrict
 }
 
 // STN: the product from the level's assembled stencils (stn, over act) instead of the gather.
-template <class T, int MODE, bool OWN16, int RB, bool STN = false>
-__global__ void __launch_bounds__(BLOCK_THREADS, 2) kb_op(LevelView L, Coefs<T> C, const int* __restrict__ act, int nAct,
-                                                       const T* __restrict__ stn, const T* __restrict__ x, T* __restrict__ y,
+template <int MODE, bool OWN16, int RB, bool STN = false>
+__global__ void __launch_bounds__(BLOCK_THREADS, 2) kb_op(LevelView L, Coefs<float> C, const int* __restrict__ act, int nAct,
+                                                       const float* __restrict__ stn, const float* __restrict__ x, float* __restrict__ y,
                                                        const float* __restrict__ r, float* __restrict__ d, float c1, float c2, int raw,
-                                                       BlockState* bs, double* partials, unsigned* ticket, Ctl ctl) {
+                                                       Ctl ctl) {
     if (skipped(ctl)) return;
     constexpr int NPW = 32 / RB;
     const int lane = threadIdx.x & 31, q = lane % RB, sub = lane / RB;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((long long)gridDim.x * blockDim.x) >> 5;
     extern __shared__ __align__(16) unsigned char kbRaw[];
-    T* rows = reinterpret_cast<T*>(kbRaw) + (threadIdx.x >> 5) * NPW * STN_ROW;  // this warp's NPW stencil rows
-    double dot[1] = {0.0};
+    float* rows = reinterpret_cast<float*>(kbRaw) + (threadIdx.x >> 5) * NPW * STN_ROW;  // this warp's NPW stencil rows
     // warp-uniform sweep (the stencil rows are shared within the warp); lanes past the list idle
     for (long long tb = warp * NPW; tb < nAct; tb += nw * NPW) {
         const long long t = tb + sub;
         if constexpr (STN) {
-            constexpr int VP = 16 / int(sizeof(T)), PIECES = STN_ROW / VP;  // 16-byte pieces of a row
+            constexpr int VP = 4, PIECES = STN_ROW / VP;  // 16-byte pieces of a row
             for (int e = lane; e < NPW * PIECES; e += 32) {
                 const int u = e / PIECES, g = e - u * PIECES;
                 if (tb + u < nAct) {
@@ -309,55 +309,30 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 2) kb_op(LevelView L, Coefs<T> 
             const uint8_t mask = __ldg(L.nmask + n);
             int i, j, k;
             nodeCoords(L, n, i, j, k);
-            T acc[3];
-            if constexpr (STN) stnBlock<T, RB>(L, rows + sub * STN_ROW, x + q, n, i, j, k, acc);
-            else applyNbr<T, OWN16, RB>(L, C, x + q, i, j, k, n, mask, acc);
+            float acc[3];
+            if constexpr (STN) stnBlock<float, RB>(L, rows + sub * STN_ROW, x + q, n, i, j, k, acc);
+            else applyNbr<float, OWN16, RB>(L, C, x + q, i, j, k, n, mask, acc);
 #pragma unroll
             for (int c = 0; c < 3; c++) {
                 const long long id = (3 * n + c) * RB + q;
                 const bool fx = fixedDof(mask, c);
                 if constexpr (MODE == BOP_APPLY) {
-                    y[id] = (!raw && fx) ? T(0) : acc[c];
-                } else if constexpr (MODE == BOP_DOT) {
-                    const T yv = fx ? T(0) : acc[c];
-                    y[id] = yv;
-                    dot[0] += double(x[id]) * double(yv);
+                    y[id] = (!raw && fx) ? 0.f : acc[c];
                 } else if constexpr (MODE == BOP_RESID) {
-                    y[id] = fx ? T(0) : T(r[id]) - acc[c];
+                    y[id] = fx ? 0.f : r[id] - acc[c];
                 } else {
                     if (fx) {
                         d[id] = 0.f;
-                        y[id] = T(0);
+                        y[id] = 0.f;
                     } else {
-                        const float dn = c1 * d[id] + c2 * __ldg(L.invD + 3 * n + c) * (r[id] - float(acc[c]));
+                        const float dn = c1 * d[id] + c2 * __ldg(L.invD + 3 * n + c) * (r[id] - acc[c]);
                         d[id] = dn;
-                        y[id] = x[id] + T(dn);
+                        y[id] = x[id] + dn;
                     }
                 }
             }
         }
         if constexpr (STN) __syncwarp();  // the rows are refilled next
-    }
-    if constexpr (MODE == BOP_DOT) {
-        double tot[1];
-        if (laneGridReduce<1, RB>(dot, 0u, partials, ticket, tot)) {
-            const int qq = threadIdx.x;
-            if (qq < RB) {
-                bs->pq[qq] = tot[0];
-                if (!rhsRunning(bs, qq)) {
-                    bs->alpha[qq] = 0;
-                } else if (!(tot[0] > 0)) {
-                    bs->alpha[qq] = 0;
-                    bs->status[qq] = ST_BREAKDOWN;
-                    bs->done[qq] = 1;
-                    bs->it[qq] = bs->iter;
-                } else {
-                    bs->alpha[qq] = bs->rz[qq] / tot[0];
-                }
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) blockAllDone(bs);
-        }
     }
 }
 

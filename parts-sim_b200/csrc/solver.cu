@@ -1038,6 +1038,7 @@ __global__ void k_reactions(long long nNodes, const uint8_t* __restrict__ nmask,
 
 #include "march_kernels.cuh"  // the marched operator of large levels
 #include "block_kernels.cuh"  // the multi-RHS kernels (they use the control helpers above)
+#include "block_march.cuh"    // their finest-level operator
 #include "ebe_kernels.cuh"    // the tensor-core element-block operator
 #include "block_tc.cuh"       // the block operator on the tensor cores
 #include "stencil_kernels.cuh"  // assembled stencils of the Galerkin levels
@@ -1250,13 +1251,13 @@ dev::ModeCoefs<T> marchCoefs(const double Kb[576], bool& ok) {
     return {T(b0), T(a0), T(a1), T(b1), T(c2), T(e2), T(b3), T(a3)};
 }
 
-// The tiles of a marched level: columns of 30 x ny nodes cut into chunks of planes, trimmed to the planes with an
+// The tiles of a marched level: columns of nx x ny nodes (`groups` CTAs each) cut into chunks of planes, trimmed to the planes with an
 // active node. A CTA of n planes takes about n + 4 steps (one plane of halo below and above, two to fill and
 // drain), so the chunk length is the one with the least waves x steps on `slots` resident CTAs: long chunks where
 // the level has many columns, short ones where it would leave SMs idle. whole: every column and plane, untrimmed, the
 // chunks without an active node marked.
-std::vector<dev::MarchTile> marchTiles(const HostLevel& h, int ny, int slots, bool whole = false) {
-    const int ntx = (h.NX + dev::MARCH_NX - 1) / dev::MARCH_NX, nty = (h.NY + ny - 1) / ny;
+std::vector<dev::MarchTile> marchTiles(const HostLevel& h, int nx, int ny, int groups, int slots, bool whole = false) {
+    const int ntx = (h.NX + nx - 1) / nx, nty = (h.NY + ny - 1) / ny;
     const size_t cols = size_t(ntx) * nty;
     std::vector<uint8_t> act(cols * h.NZ, 0);  // [k][ty][tx]
     parallelFor(h.NZ, [&](int64_t ka, int64_t kb) {
@@ -1264,7 +1265,7 @@ std::vector<dev::MarchTile> marchTiles(const HostLevel& h, int ny, int slots, bo
             for (int j = 0; j < h.NY; j++) {
                 const uint8_t* row = h.nmask.data() + h.node(0, j, int(k));
                 uint8_t* a = act.data() + size_t(k) * cols + size_t(j / ny) * ntx;
-                for (int i = 0; i < h.NX; i++) a[i / dev::MARCH_NX] |= (row[i] & NM_ACTIVE) ? 1 : 0;
+                for (int i = 0; i < h.NX; i++) a[i / nx] |= (row[i] & NM_ACTIVE) ? 1 : 0;
             }
     }, 8);
     size_t live = 0;
@@ -1276,7 +1277,7 @@ std::vector<dev::MarchTile> marchTiles(const HostLevel& h, int ny, int slots, bo
     int best = 1;
     int64_t bestCost = INT64_MAX;
     for (int tz = 1; tz <= std::min(h.NZ, 96); tz++) {
-        const int64_t ctas = int64_t(live) * ((h.NZ + tz - 1) / tz), cost = ((ctas + slots - 1) / slots) * (tz + 4);
+        const int64_t ctas = int64_t(live) * groups * ((h.NZ + tz - 1) / tz), cost = ((ctas + slots - 1) / slots) * (tz + 4);
         if (cost < bestCost) {
             bestCost = cost;
             best = tz;
@@ -1651,7 +1652,7 @@ void SharedModel::uploadLevel(int l) {
         D.m64 = marchCoefs<double>(h.Kb, D.useTiles);
         D.m32 = marchCoefs<float>(h.Kb, D.useTiles);
         if (l == 0 && D.useTiles) {
-            const std::vector<dev::MarchTile> ta = marchTiles(h, dev::marchNY<double>(), smCount, true);
+            const std::vector<dev::MarchTile> ta = marchTiles(h, dev::MARCH_NX, dev::marchNY<double>(), 1, smCount, true);
             D.nTilesAll = int(ta.size());
             upload(D.tilesAll, ta, bytes, ms);
         }
@@ -1660,7 +1661,7 @@ void SharedModel::uploadLevel(int l) {
         if (const char* e = std::getenv("PSFEA_OP8_MAX_NODES")) max8 = std::atoll(e);
         D.use8 = !D.useTiles && l > 0 && h.nNodes <= max8;
         if (D.useTiles) {
-            const std::vector<dev::MarchTile> t32 = marchTiles(h, dev::marchNY<float>(), smCount), t64 = marchTiles(h, dev::marchNY<double>(), smCount);
+            const std::vector<dev::MarchTile> t32 = marchTiles(h, dev::MARCH_NX, dev::marchNY<float>(), 1, smCount), t64 = marchTiles(h, dev::MARCH_NX, dev::marchNY<double>(), 1, smCount);
             D.nTiles32 = int(t32.size());
             D.nTiles64 = int(t64.size());
             upload(D.tiles32, t32, bytes, ms);
@@ -2797,6 +2798,8 @@ struct BlockImpl final : BlockBase {
     std::vector<LevelWork> W;     // FP32 V-cycle vectors per level, RB wide
     DevMem f, x, r, p, q, z64;    // FP64 vectors of the finest level, RB wide
     DevMem state, partials, ticket;
+    DevMem tiles32, tiles64;      // the finest level's tiles (block_march.cuh)
+    int nTiles32 = 0, nTiles64 = 0;
     dev::BlockState* hostState = nullptr;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev = nullptr;
@@ -2814,8 +2817,12 @@ struct BlockImpl final : BlockBase {
             auto set = [](auto kernel, size_t b) {
                 check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(b)), "attr");
             };
-            set(dev::kb_op<float, dev::BOP_CHEB, false, RB, true>, dev::stnBlockSmem<float>(32 / RB));
-            set(dev::kb_op<float, dev::BOP_RESID, false, RB, true>, dev::stnBlockSmem<float>(32 / RB));
+            set(dev::kb_op<dev::BOP_CHEB, false, RB, true>, dev::stnBlockSmem<float>(32 / RB));
+            set(dev::kb_op<dev::BOP_RESID, false, RB, true>, dev::stnBlockSmem<float>(32 / RB));
+            set(dev::kb_march<float, dev::BOP_CHEB, RB>, dev::bmSmemBytes<float>());
+            set(dev::kb_march<float, dev::BOP_RESID, RB>, dev::bmSmemBytes<float>());
+            set(dev::kb_march<double, dev::BOP_APPLY, RB>, dev::bmSmemBytes<double>());
+            set(dev::kb_march<double, dev::BOP_DOT, RB>, dev::bmSmemBytes<double>());
         });
         check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "stream");
         check(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
@@ -2832,7 +2839,14 @@ struct BlockImpl final : BlockBase {
         for (DevMem* b : {&f, &x, &r, &p, &q}) b->alloc(n, bytes, stream);
         if (M->exactOneLevel()) z64.alloc(n, bytes, stream);
         state.alloc(sizeof(dev::BlockState), bytes, stream);
-        partials.alloc(size_t(smCount) * 16 * RB * 3 * sizeof(double) + 4096, bytes, stream);
+        const auto t32 = marchTiles(H.levels[0], dev::BM_NX, dev::bmNY<float>(), RB / dev::BM_G, smCount);
+        const auto t64 = marchTiles(H.levels[0], dev::BM_NX, dev::bmNY<double>(), RB / dev::BM_G, smCount);
+        nTiles32 = int(t32.size());
+        nTiles64 = int(t64.size());
+        upload(tiles32, t32, bytes, stream);
+        upload(tiles64, t64, bytes, stream);
+        check(cudaStreamSynchronize(stream), "tile upload");  // (from pageable memory that ends here)
+        partials.alloc((size_t(smCount) * 16 * 3 + size_t(nTiles64)) * RB * sizeof(double) + 4096, bytes, stream);
         ticket.alloc(64, bytes, stream);
         check(cudaStreamWaitEvent(stream, M->readyEv, 0), "wait");
     }
@@ -2841,7 +2855,7 @@ struct BlockImpl final : BlockBase {
         for (auto& g : graph)
             if (g) cudaGraphExecDestroy(g);
         for (auto& w : W) w.release();
-        for (DevMem* b : {&f, &x, &r, &p, &q, &z64, &state, &partials, &ticket}) b->release();
+        for (DevMem* b : {&f, &x, &r, &p, &q, &z64, &state, &partials, &ticket, &tiles32, &tiles64}) b->release();
         if (ev) cudaEventDestroy(ev);
         if (hostState) cudaFreeHost(hostState);
         cudaStreamSynchronize(stream);
@@ -2890,25 +2904,26 @@ struct BlockImpl final : BlockBase {
                 return;
             }
         }
-        const auto& C = [&]() -> const dev::Coefs<T>& {
-            if constexpr (sizeof(T) == 8) return D.c64;
-            else return D.c32;
-        }();
-        // the assembled stencils of the Galerkin levels
-        if constexpr (sizeof(T) == 4) {
+        if constexpr (sizeof(T) == 8) {  // only ever on the finest level
+            launch(dev::kb_march<double, MODE, RB>, nTiles64 * (RB / dev::BM_G), dev::bmThreads<double>(), dev::bmSmemBytes<double>(), D.view, D.m64,
+                   tiles64.template as<dev::MarchTile>(), nTiles64, xin, y, rr, dd, c1, c2, raw ? 1 : 0, bs(), part(), tick(), ctl);
+        } else {
+            const dev::Coefs<float>& C = D.c32;
+            // the assembled stencils of the Galerkin levels
             const float* stn = M->bstn32.empty() ? nullptr : M->bstn32[size_t(l)].template as<float>();
-            if (stn) {
-                launch(dev::kb_op<float, MODE, false, RB, true>, laneGrid(l), dev::BLOCK_THREADS, dev::stnBlockSmem<float>(32 / RB), D.view, C,
-                       act(l), nAct(l), stn, xin, y, rr, dd, c1, c2, raw ? 1 : 0, bs(), part(), tick(), ctl);
-                return;
-            }
+            if (stn)
+                launch(dev::kb_op<MODE, false, RB, true>, laneGrid(l), dev::BLOCK_THREADS, dev::stnBlockSmem<float>(32 / RB), D.view, C, act(l),
+                       nAct(l), stn, xin, y, rr, dd, c1, c2, raw ? 1 : 0, ctl);
+            else if (l == 0)
+                launch(dev::kb_march<float, MODE, RB>, nTiles32 * (RB / dev::BM_G), dev::bmThreads<float>(), dev::bmSmemBytes<float>(), D.view, D.m32,
+                       tiles32.template as<dev::MarchTile>(), nTiles32, xin, y, rr, dd, c1, c2, raw ? 1 : 0, bs(), part(), tick(), ctl);
+            else if (own16 && D.hasOwn)
+                launch(dev::kb_op<MODE, true, RB>, laneGrid(l), dev::BLOCK_THREADS, 0, D.view, C, act(l), nAct(l),
+                       static_cast<const float*>(nullptr), xin, y, rr, dd, c1, c2, raw ? 1 : 0, ctl);
+            else
+                launch(dev::kb_op<MODE, false, RB>, laneGrid(l), dev::BLOCK_THREADS, 0, D.view, C, act(l), nAct(l),
+                       static_cast<const float*>(nullptr), xin, y, rr, dd, c1, c2, raw ? 1 : 0, ctl);
         }
-        if (own16 && D.hasOwn)
-            launch(dev::kb_op<T, MODE, true, RB>, laneGrid(l), dev::BLOCK_THREADS, 0, D.view, C, act(l), nAct(l), static_cast<const T*>(nullptr),
-                   xin, y, rr, dd, c1, c2, raw ? 1 : 0, bs(), part(), tick(), ctl);
-        else
-            launch(dev::kb_op<T, MODE, false, RB>, laneGrid(l), dev::BLOCK_THREADS, 0, D.view, C, act(l), nAct(l), static_cast<const T*>(nullptr),
-                   xin, y, rr, dd, c1, c2, raw ? 1 : 0, bs(), part(), tick(), ctl);
     }
 
     void coarse(const float* rin, float* zout, dev::Ctl ctl) {
