@@ -1337,8 +1337,9 @@ struct DevLevel {
     int nStn = 0;
     DevMem stn32, stn16;
     float stnScale = 1.f;
+    DevMem stn8;  // FP32, the layout of k_stn8: the small levels' instead of stn32 / stn16
     void release() {
-        for (DevMem* b : {&word, &nmask, &own, &own16, &invD, &dadd, &dadd32, &bc, &tiles32, &tiles64, &tilesAll, &blist, &olist, &ebeTiles, &stn32, &stn16}) b->release();
+        for (DevMem* b : {&word, &nmask, &own, &own16, &invD, &dadd, &dadd32, &bc, &tiles32, &tiles64, &tilesAll, &blist, &olist, &ebeTiles, &stn32, &stn16, &stn8}) b->release();
     }
 };
 
@@ -1647,7 +1648,10 @@ void SharedModel::uploadLevel(int l) {
         }
         // small levels have too few tiles to fill the GPU: one thread per node instead, or eight
         // lanes per node on the smallest ones
-        int64_t minNodes = 400000;
+        // (marched levels with own matrices take a second launch for the nodes that touch one: worth it from 400 k nodes;
+        // without, one thread per node is the faster only below some 8 k nodes: 64x16x16 cantilever 1.45 -> 1.26 ms a solve,
+        // SIMP 96x48x48 19.6 -> 16.5 ms, while marching that grid's level 1 of 30 k nodes, 85 % own matrices, costs 1.2 ms)
+        int64_t minNodes = h.nOwn == 0 ? 8000 : 400000;
         if (const char* e = std::getenv("PSFEA_TILE_MIN_NODES")) minNodes = std::atoll(e);
         D.m64 = marchCoefs<double>(h.Kb, D.useTiles);
         D.m32 = marchCoefs<float>(h.Kb, D.useTiles);
@@ -1716,15 +1720,24 @@ void SharedModel::ensureStencils(bool half) {
     for (size_t l = 1; l < L.size() && l < 63; l++) {
         DevLevel& D = L[l];
         const int cnt = D.useTiles ? D.listCount(D.split32) : nAct[l];
-        if (!((stencilLevels >> l) & 1) || cnt <= 0 || cnt < stencilMinNodes) continue;
+        if (!((stencilLevels >> l) & 1) || cnt <= 0 || (D.useTiles && cnt < stencilMinNodes)) continue;
         const int* nodes = D.useTiles ? D.list(D.split32) : act[l].as<int>();
         if (D.stnNodes != nodes) {  // (the autotuner may switch a level's list)
             D.stn32.release();
             D.stn16.release();
+            D.stn8.release();
         }
         D.stnNodes = nodes;
         D.nStn = cnt;
         const int grid = gridFor(int64_t(cnt) * 27, 256, smCount * 32);
+        if (cnt < stencilMinNodes) {
+            if (D.stn8.p) continue;
+            D.stn8.alloc(size_t(cnt) * dev::STN8_ROW * sizeof(float), bytes, ms);
+            dev::k_stn_build<float, float, dev::STN_LANES><<<grid, 256, 0, ms>>>(D.view, D.c32, D.stnNodes, cnt, D.stn8.as<float>(), 1.f);
+            check(cudaGetLastError(), "stencil build");
+            built = true;
+            continue;
+        }
         if (!half && !D.stn32.p) {
             D.stn32.alloc(size_t(cnt) * dev::stnChunks<4>() * 4 * sizeof(float), bytes, ms);
             dev::k_stn_build<float, float><<<grid, 256, 0, ms>>>(D.view, D.c32, D.stnNodes, cnt, D.stn32.as<float>(), 1.f);
@@ -1767,7 +1780,7 @@ void SharedModel::ensureBlockStencils() {
         const int grid = gridFor(int64_t(cnt) * 27, 256, smCount * 32);
         if (l > 0 || blockStencil0) {
             bstn32[l].alloc(size_t(cnt) * dev::STN_ROW * sizeof(float), bytes, ms);
-            dev::k_stn_build<float, float, true><<<grid, 256, 0, ms>>>(D.view, D.c32, act[l].as<int>(), cnt, bstn32[l].as<float>(), 1.f);
+            dev::k_stn_build<float, float, dev::STN_PAIRED><<<grid, 256, 0, ms>>>(D.view, D.c32, act[l].as<int>(), cnt, bstn32[l].as<float>(), 1.f);
             check(cudaGetLastError(), "block stencil build");
         }
     }
@@ -2081,6 +2094,11 @@ void SolverImpl::op32(int l, const float* xin, float* y, float c1, float c2, dev
     };
     const bool stn = l > 0 && !diff && D.nStn > 0 && (s16 ? D.stn16.p != nullptr : D.stn32.p != nullptr) &&
                      (!D.useTiles || D.stnNodes == D.list(D.split32));
+    if (l > 0 && !diff && !D.useTiles && D.stn8.p) {  // a small level
+        launch(dev::k_stn8<SM_>, unsigned((int64_t(D.nStn) * 8 + 255) / 256), 256, 0, stream, D.view, D.stnNodes, D.nStn, D.stn8.as<float4>(), xin, y, rr,
+               dd, c1, c2, 0, ctl);
+        return;
+    }
     if (stn && !D.useTiles) {
         stencilPass();
         return;
@@ -3281,6 +3299,7 @@ int64_t estimateDeviceBytes(const Hierarchy& H) {
              4 * (h.nNodes / 1024 + 1);
         if (l == 0) b += dofs;
         b += 16 * dofs;  // V-cycle vectors r, z, t, d
+        if (l > 0 && nodes < 65536) b += 4 * int64_t(dev::STN8_ROW) * nodes;  // the small levels' stencils
         allocs += 12;
     }
     const int64_t n = 3 * int64_t(pitch4(H.levels[0].NX)) * H.levels[0].NY * H.levels[0].NZ;

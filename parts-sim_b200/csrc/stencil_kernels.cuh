@@ -28,8 +28,15 @@ __device__ __forceinline__ void stStn(__half* p, float v, float inv) { *p = __fl
 // otherwise); the diagonal shift joins the centre block. Sums in CT (FP32, or FP64 for the block
 // path's FP64 product), stored as floats (4-value chunks), doubles (2-value chunks) or halves
 // times inv (8-value chunks).
-// NODE_MAJOR: the block path's paired layout instead (row t at t * STN_ROW, block_kernels.cuh).
-template <class ST, class CT = float, bool NODE_MAJOR = false>
+// LAYOUT: STN_PAIRED the block path's paired layout instead (row t at t * STN_ROW, block_kernels.cuh), STN_LANES that of
+// k_stn8 (its padding is zeroed by the allocation).
+enum { STN_CHUNKS = 0, STN_PAIRED = 1, STN_LANES = 2 };
+constexpr int STN8_ROW = 288;  // floats of a node in the layout of k_stn8
+__host__ __device__ __forceinline__ long long stn8At(int m, int c, long long t) {
+    const int pos = 9 * (m >> 3) + c;
+    return ((t * 9 + pos / 4) * 8 + (m & 7)) * 4 + pos % 4;
+}
+template <class ST, class CT = float, int LAYOUT = STN_CHUNKS>
 __global__ void k_stn_build(LevelView L, Coefs<CT> C, const int* __restrict__ list, int count, ST* __restrict__ stn, float inv) {
     constexpr int CW = 16 / int(sizeof(ST));
     const long long total = (long long)count * 27;
@@ -63,7 +70,10 @@ __global__ void k_stn_build(LevelView L, Coefs<CT> C, const int* __restrict__ li
         if (m == 13 && L.dadd32)
             for (int p = 0; p < 3; p++) blk[4 * p] += sizeof(CT) == 8 ? CT(L.dadd[3 * n + p]) : CT(L.dadd32[3 * n + p]);
         for (int c = 0; c < 9; c++)
-            stStn(stn + (NODE_MAJOR ? (long long)t * STN_ROW + stnPairAt(m, c / 3, c % 3) : stnAt<CW>(9 * m + c, t, count)), blk[c], inv);
+            stStn(stn + (LAYOUT == STN_PAIRED ? (long long)t * STN_ROW + stnPairAt(m, c / 3, c % 3)
+                  : LAYOUT == STN_LANES ? stn8At(m, c, t)
+                                        : stnAt<CW>(9 * m + c, t, count)),
+                  blk[c], inv);
     }
 }
 
@@ -153,6 +163,69 @@ __global__ void __launch_bounds__(256) k_stn(LevelView L, const int* __restrict_
                 }
             }
         }
+    }
+}
+
+// The same passes on the small levels, eight lanes a node: lane l holds the blocks of the neighbours l, l + 8, l + 16
+// and l + 24 (36 floats in nine 16-byte loads, the nine lines of a node contiguous), the eight partial sums meet by shuffles
+// and three lanes run the epilogue. A level of some thousand nodes is a chain of dependent loads, not a stream: here
+// it is list entry, neighbour values, sum, and everything else (coefficients, r, d, 1/diag) is on its way beside it.
+// Out-of-grid neighbours have zero blocks; their addresses are clamped into the vector.
+// Chosen for untiled levels of fewer than stencilMinNodes listed nodes (above, k_stn's 972 bytes a node instead of
+// 1152 count for more than the latency).
+template <int MODE>
+__global__ void __launch_bounds__(256) k_stn8(LevelView L, const int* __restrict__ list, int count, const float4* __restrict__ stn,
+                                              const float* __restrict__ x, float* __restrict__ y, const float* __restrict__ r,
+                                              float* __restrict__ d, float c1, float c2, int raw, Ctl ctl) {
+    if (skipped(ctl)) return;
+    const int lane = threadIdx.x & 7;
+    const long long at = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3;
+    const long long t = at < count ? at : count - 1;  // (a repeat of the last node, not stored)
+    float4 cf[9];
+#pragma unroll
+    for (int s = 0; s < 9; s++) cf[s] = __ldg(stn + (t * 9 + s) * 8 + lane);
+    const long long n = __ldg(list + t), NX = L.PX, NXY = (long long)L.PX * L.NY;
+    float xm[4][3];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+        const int m = lane + 8 * u < 27 ? lane + 8 * u : 13;
+        const long long o = n + (m % 3 - 1) + ((m / 3) % 3 - 1) * NX + (m / 9 - 1) * NXY;
+        const float* xp = x + 3 * (o < 0 ? 0 : o >= L.nNodes ? L.nNodes - 1 : o);
+        xm[u][0] = __ldg(xp);
+        xm[u][1] = __ldg(xp + 1);
+        xm[u][2] = __ldg(xp + 2);
+    }
+    const int q = lane < 3 ? lane : 0;
+    const long long id = 3 * n + q;
+    const uint8_t mask = __ldg(L.nmask + n);
+    float rv = 0.f, dv = 0.f, iv = 0.f, xv = 0.f;
+    if (MODE != TOP_APPLY) rv = __ldg(r + id);
+    if (MODE == TOP_CHEB) {
+        dv = d[id];
+        iv = __ldg(L.invD + id);
+        xv = __ldg(x + id);
+    }
+    float a[3] = {0.f, 0.f, 0.f};
+    const float* cv = reinterpret_cast<const float*>(cf);
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+#pragma unroll
+        for (int e = 0; e < 9; e++) a[e / 3] += cv[9 * u + e] * xm[u][e % 3];
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+        for (int c = 0; c < 3; c++) a[c] += __shfl_xor_sync(0xffffffffu, a[c], o);
+    if (at >= count || lane >= 3) return;
+    const float kx = q == 0 ? a[0] : (q == 1 ? a[1] : a[2]);
+    const bool fx = fixedDof(mask, q);
+    if (MODE == TOP_APPLY) {
+        y[id] = (!raw && fx) ? 0.f : kx;
+    } else if (MODE == TOP_RESID) {
+        y[id] = fx ? 0.f : rv - kx;
+    } else {
+        const float dn = fx ? 0.f : c1 * dv + c2 * iv * (rv - kx);
+        d[id] = dn;
+        y[id] = fx ? 0.f : xv + dn;
     }
 }
 

@@ -132,3 +132,26 @@ def test_empty_voxels_do_not_carry_infinities():
                     touched[k + dk:k + dk + 2, j + dj:j + dj + 2, i + di:i + di + 2] = True
     assert np.array_equal(~np.isfinite(y).all(axis=-1), touched)
     assert np.array_equal(y[~touched], ref[~touched])
+
+
+@pytest.mark.parametrize("dims", [(13, 9, 7), (30, 44, 17), (48, 20, 24)])
+@pytest.mark.parametrize("shift", [False, True])
+def test_small_levels_stencils_match_the_gather(monkeypatch, dims, shift):
+    """The small Galerkin levels' eight-lane stencils (level node counts that leave part of a warp, one and several blocks, with
+    and without a diagonal shift) against the per-voxel gather (PSFEA_STENCIL_LEVELS=0): the V-cycle of a load to a few FP32
+    roundings a pass, and solves in every form."""
+    d, bc = blocky(dims, 4)
+    rng = np.random.default_rng(1)
+    add = rng.uniform(0.0, 0.2, bc.size) if shift else None
+    monkeypatch.setenv("PSFEA_STENCIL_LEVELS", "0")
+    A = psfea.VoxelFEA(dims, d, 0.3, bc, 60, diag_add=add)
+    monkeypatch.delenv("PSFEA_STENCIL_LEVELS")
+    B = psfea.VoxelFEA(dims, d, 0.3, bc, 60, diag_add=add)
+    assert A.n_levels >= 3
+    f = rng.standard_normal(A.n_dof) * (A.fixed(0) == 0)
+    for prec in ("fp64", "mixed", "fp32"):
+        for deg in (0, 3):
+            a = A.solve(f, tol=1e-9, max_iter=3000, precision=prec, smoother_degree=deg)
+            b = B.solve(f, tol=1e-9, max_iter=3000, precision=prec, smoother_degree=deg)
+            assert a.converged and b.converged and rel(b.u, a.u) < 1e-5, (prec, deg)
+    assert rel(B.precondition(f), A.precondition(f)) < 1e-5
