@@ -361,33 +361,13 @@ __global__ void kb_restrict(LevelView F, LevelView C, const int* __restrict__ cA
     constexpr int NPW = 32 / RB;
     const int lane = threadIdx.x & 31, q = lane % RB, sub = lane / RB;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    const long long FPX = F.PX, FPXY = (long long)F.PX * F.NY;
     for (long long t = warp * NPW + sub; t < nCAct; t += nw * NPW) {
         const long long cn = cAct[t];
         const uint8_t mask = C.nmask[cn];
         int I, J, K;
         nodeCoords(C, cn, I, J, K);
-        float s0 = 0, s1 = 0, s2 = 0;
-        for (int dk = -1; dk <= 1; dk++) {
-            const int k = 2 * K + dk;
-            if (k < 0 || k >= F.NZ) continue;
-            const float wk = dk ? 0.5f : 1.f;
-            for (int dj = -1; dj <= 1; dj++) {
-                const int j = 2 * J + dj;
-                if (j < 0 || j >= F.NY) continue;
-                const float wj = (dj ? 0.5f : 1.f) * wk;
-                for (int di = -1; di <= 1; di++) {
-                    const int i = 2 * I + di;
-                    if (i < 0 || i >= F.NX) continue;
-                    const float w = (di ? 0.5f : 1.f) * wj;
-                    const float* p = rf + 3 * RB * (i + j * FPX + k * FPXY) + q;
-                    s0 += w * p[0];
-                    s1 += w * p[RB];
-                    s2 += w * p[2 * RB];
-                }
-            }
-        }
-        const float sv[3] = {s0, s1, s2};
+        float sv[3];
+        restrictAt<RB>(F, rf + q, I, J, K, sv);
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             const long long id = (3 * cn + c) * RB + q;
@@ -417,44 +397,55 @@ __global__ void kb_prolong(LevelView F, int CPX, int CNY, const int* __restrict_
         if ((mask & 7) == 7) continue;
         int i, j, k;
         nodeCoords(F, fn, i, j, k);
-        const int i0 = i >> 1, j0 = j >> 1, k0 = k >> 1;
-        const int ni = (i & 1) ? 2 : 1, nj = (j & 1) ? 2 : 1, nk = (k & 1) ? 2 : 1;
-        const float w = ((i & 1) ? 0.5f : 1.f) * ((j & 1) ? 0.5f : 1.f) * ((k & 1) ? 0.5f : 1.f);
-        float s0 = 0, s1 = 0, s2 = 0;
-        for (int c = 0; c < nk; c++)
-            for (int b = 0; b < nj; b++)
-                for (int a = 0; a < ni; a++) {
-                    const float* p = zc + 3 * RB * ((i0 + a) + (j0 + b) * CNX + (k0 + c) * CNXY) + q;
-                    s0 += w * p[0];
-                    s1 += w * p[RB];
-                    s2 += w * p[2 * RB];
-                }
         float* o = zf + 3 * RB * fn + q;
-        if (!fixedDof(mask, 0)) o[0] += s0;
-        if (!fixedDof(mask, 1)) o[RB] += s1;
-        if (!fixedDof(mask, 2)) o[2 * RB] += s2;
+        const float z0 = o[0], z1 = o[RB], z2 = o[2 * RB];
+        float s[3];
+        prolongAt<RB>(CNX, CNXY, zc + q, i, j, k, s);
+        if (!fixedDof(mask, 0)) o[0] = z0 + s[0];
+        if (!fixedDof(mask, 1)) o[RB] = z1 + s[1];
+        if (!fixedDof(mask, 2)) o[2 * RB] = z2 + s[2];
     }
 }
 
-// coarsest level: z = A^-1 r over the m free DOFs for every right-hand side (FP64 dense inverse,
-// one row per lane group; the row's entries are read once for the group's right-hand sides)
+// coarsest level: z = A^-1 r over the m free DOFs for every right-hand side (FP64 dense inverse). A block takes KBC_ROWS
+// rows, its warps every 8th group of NPW columns each (the lane groups of a warp a column of their own), the partial sums
+// meet in shared memory in a fixed order. (One lane group over a whole row, column after column, was a chain of m / 2
+// dependent loads: 96 us at m = 312.)
+constexpr int KBC_ROWS = 2;
 template <class TI, class TO, int RB>
-__global__ void kb_coarse(int m, const int* __restrict__ dof, const double* __restrict__ Ainv, const TI* __restrict__ r, TO* __restrict__ z,
-                          Ctl ctl) {
+__global__ void __launch_bounds__(BLOCK_THREADS) kb_coarse(int m, const int* __restrict__ dof, const double* __restrict__ Ainv,
+                                                           const TI* __restrict__ r, TO* __restrict__ z, Ctl ctl) {
     if (skipped(ctl)) return;
-    constexpr int NPW = 32 / RB;
-    const int lane = threadIdx.x & 31, q = lane % RB, sub = lane / RB;
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long row = warp * NPW + sub; row < m; row += nw * NPW) {
-        const double* a = Ainv + (size_t)row * m;
-        double s0 = 0, s1 = 0;
-        int c = 0;
-        for (; c + 1 < m; c += 2) {
-            s0 += a[c] * double(r[(long long)dof[c] * RB + q]);
-            s1 += a[c + 1] * double(r[(long long)dof[c + 1] * RB + q]);
+    constexpr int NPW = 32 / RB, NW = BLOCK_THREADS / 32, U = 4;
+    __shared__ double sh[KBC_ROWS][NW][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = lane % RB, sub = lane / RB;
+    const int row = blockIdx.x * KBC_ROWS;
+    double s[KBC_ROWS] = {};
+    for (int c0 = wid * NPW + sub; c0 < m; c0 += NW * NPW * U) {
+        double rv[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int c = c0 + u * NW * NPW;
+            rv[u] = c < m ? double(__ldg(r + (long long)__ldg(dof + c) * RB + q)) : 0.0;
         }
-        if (c < m) s0 += a[c] * double(r[(long long)dof[c] * RB + q]);
-        z[(long long)dof[row] * RB + q] = TO(s0 + s1);
+#pragma unroll
+        for (int e = 0; e < KBC_ROWS; e++)
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int c = c0 + u * NW * NPW;
+                if (c < m && row + e < m) s[e] += __ldg(Ainv + (size_t)(row + e) * m + c) * rv[u];
+            }
+    }
+#pragma unroll
+    for (int e = 0; e < KBC_ROWS; e++) sh[e][wid][lane] = s[e];
+    __syncthreads();
+    if (threadIdx.x < KBC_ROWS * RB) {
+        const int e = threadIdx.x / RB, qq = threadIdx.x % RB;
+        double t = 0;
+        for (int w = 0; w < NW; w++)
+#pragma unroll
+            for (int u = 0; u < NPW; u++) t += sh[e][w][u * RB + qq];
+        if (row + e < m) z[(long long)__ldg(dof + row + e) * RB + qq] = TO(t);
     }
 }
 

@@ -58,12 +58,16 @@ struct SolveState {
 };
 enum { ST_RUNNING = 0, ST_CONVERGED = 1, ST_MAXITER = 2, ST_BREAKDOWN = 3 };
 
-// a kernel runs unless *skipIf != 0 or (runIf and *runIf == 0)
+// A kernel runs unless *skipIf != 0 or (runIf and *runIf == 0). Every kernel of an iteration asks this first; there it also
+// waits for the kernel before it (a programmatic dependent launch may have started it while that one ran; a
+// no-op otherwise) and lets the next one start coming in.
 struct Ctl {
     const int* skipIf;
     const int* runIf;
 };
 __device__ __forceinline__ bool skipped(const Ctl& c) {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     if (c.skipIf && *((volatile const int*)c.skipIf)) return true;
     if (c.runIf && !*((volatile const int*)c.runIf)) return true;
     return false;
@@ -331,6 +335,35 @@ __global__ void k_cheb_first(long long nDof, const V* __restrict__ r, const floa
     }
 }
 
+// Sum over the fine nodes 2I + (-1 .. 1) per axis, weights 1, 1/2 per axis off the centre, of the fine vector's three
+// components (S: the stride of consecutive DOFs, rf at the lane's right-hand side). Written without branches, so that
+// all 81 loads are in flight at once (a loop with bounds tests was a chain of 27 L2 latencies: 7 us on the smallest
+// levels, where a pass is nothing else): a neighbour outside the grid reads the nearest node of the grid with weight 0.
+template <int S, class VF>
+__device__ __forceinline__ void restrictAt(const LevelView& F, const VF* __restrict__ rf, int I, int J, int K, float s[3]) {
+    const long long FPX = F.PX, FPXY = (long long)F.PX * F.NY;
+    s[0] = s[1] = s[2] = 0.f;
+#pragma unroll
+    for (int dk = -1; dk <= 1; dk++) {
+        const int k = 2 * K + dk, kc = min(max(k, 0), F.NZ - 1);
+        const float wk = k == kc ? (dk ? 0.5f : 1.f) : 0.f;
+#pragma unroll
+        for (int dj = -1; dj <= 1; dj++) {
+            const int j = 2 * J + dj, jc = min(max(j, 0), F.NY - 1);
+            const float wj = j == jc ? (dj ? 0.5f : 1.f) * wk : 0.f;
+#pragma unroll
+            for (int di = -1; di <= 1; di++) {
+                const int i = 2 * I + di, ic = min(max(i, 0), F.NX - 1);
+                const float w = i == ic ? (di ? 0.5f : 1.f) * wj : 0.f;
+                const VF* p = rf + 3 * S * (ic + jc * FPX + kc * FPXY);
+                s[0] += w * ldv<float>(p);
+                s[1] += w * ldv<float>(p + S);
+                s[2] += w * ldv<float>(p + 2 * S);
+            }
+        }
+    }
+}
+
 // rc = P^T rf gathered per coarse node: fine 2I (weight 1) and 2I +- 1 (weight 1/2) per axis;
 // held / inactive coarse DOFs 0. VF / VC: the fine / coarse storage (float, or __half for the FP16
 // coarse-level vectors, whose residual scales differ by the power of two sr: rc = sr P^T rf).
@@ -338,42 +371,24 @@ template <class VF = float, class VC = float>
 __global__ void k_restrict(LevelView F, LevelView C, const VF* __restrict__ rf, VC* __restrict__ rc, VC* __restrict__ dc,
                            VC* __restrict__ zc, float c0, float sr, Ctl ctl) {
     if (skipped(ctl)) return;
-    const int FNX = F.NX, FNY = F.NY, FNZ = F.NZ;
-    const long long FPX = F.PX, FPXY = (long long)F.PX * F.NY;
     for (long long cn = blockIdx.x * (long long)blockDim.x + threadIdx.x; cn < C.nNodes; cn += (long long)gridDim.x * blockDim.x) {
-        const uint8_t mask = C.nmask[cn];
-        float s0 = 0, s1 = 0, s2 = 0;
+        const uint8_t mask = __ldg(C.nmask + cn);
+        float sv[3] = {0.f, 0.f, 0.f}, iv[3] = {0.f, 0.f, 0.f};
         if (mask & NM_ACTIVE) {
             int I, J, K;
             nodeCoords(C, cn, I, J, K);
-            for (int dk = -1; dk <= 1; dk++) {
-                const int k = 2 * K + dk;
-                if (k < 0 || k >= FNZ) continue;
-                const float wk = dk ? 0.5f : 1.f;
-                for (int dj = -1; dj <= 1; dj++) {
-                    const int j = 2 * J + dj;
-                    if (j < 0 || j >= FNY) continue;
-                    const float wj = (dj ? 0.5f : 1.f) * wk;
-                    for (int di = -1; di <= 1; di++) {
-                        const int i = 2 * I + di;
-                        if (i < 0 || i >= FNX) continue;
-                        const float w = (di ? 0.5f : 1.f) * wj;
-                        const VF* p = rf + 3 * (i + j * FPX + k * FPXY);
-                        s0 += w * ldf(p);
-                        s1 += w * ldf(p + 1);
-                        s2 += w * ldf(p + 2);
-                    }
-                }
-            }
+            if (dc)
+#pragma unroll
+                for (int q = 0; q < 3; q++) iv[q] = __ldg(C.invD + 3 * cn + q);
+            restrictAt<1>(F, rf, I, J, K, sv);
         }
-        const float sv[3] = {s0, s1, s2};
         constexpr bool SCALED = !std::is_same<VC, float>::value;
 #pragma unroll
         for (int q = 0; q < 3; q++) {
             const float v = fixedDof(mask, q) ? 0.f : (SCALED ? sr * sv[q] : sv[q]);
             stv(rc + 3 * cn + q, v);
             if (dc) {  // the coarse level's first smoothing step, d = z = c0 D^-1 r
-                const float dv = c0 * C.invD[3 * cn + q] * v;
+                const float dv = c0 * iv[q] * v;
                 stv(dc + 3 * cn + q, dv);
                 stv(zc + 3 * cn + q, dv);
             }
@@ -381,65 +396,97 @@ __global__ void k_restrict(LevelView F, LevelView C, const VF* __restrict__ rf, 
     }
 }
 
-// zf += P zc at free fine DOFs (trilinear: coarse i/2 and, when odd, (i+1)/2, weight 1/2 each);
-// VC / VF as in k_restrict, the iterate scales differing by the power of two sp: zf += sp P zc.
-// list: the fine level's active nodes (inactive ones are all held and never written), or null for
-// every node of the level.
+// Trilinear value at fine node (i, j, k) of a coarse vector (coarse i/2 and, when odd, (i + 1)/2, weight 1/2 each); the up to
+// eight corners without branches as in restrictAt (an even axis reads its one node twice, the second time with weight 0)
+template <int S, class VC>
+__device__ __forceinline__ void prolongAt(long long CNX, long long CNXY, const VC* __restrict__ zc, int i, int j, int k, float s[3]) {
+    const int oi = i & 1, oj = j & 1, ok = k & 1;
+    const float w = (oi ? 0.5f : 1.f) * (oj ? 0.5f : 1.f) * (ok ? 0.5f : 1.f);
+    const VC* p0 = zc + 3 * S * ((i >> 1) + (j >> 1) * CNX + (k >> 1) * CNXY);
+    s[0] = s[1] = s[2] = 0.f;
+#pragma unroll
+    for (int c = 0; c < 2; c++)
+#pragma unroll
+        for (int b = 0; b < 2; b++)
+#pragma unroll
+            for (int a = 0; a < 2; a++) {
+                const VC* p = p0 + 3 * S * ((a & oi) + (b & oj) * CNX + (c & ok) * CNXY);
+                const float wt = (a > oi || b > oj || c > ok) ? 0.f : w;
+                s[0] += wt * ldv<float>(p);
+                s[1] += wt * ldv<float>(p + S);
+                s[2] += wt * ldv<float>(p + 2 * S);
+            }
+}
+
+// zf += P zc at free fine DOFs; VC / VF as in k_restrict, the iterate scales differing by the power of two sp: zf +=
+// sp P zc. list: the fine level's active nodes (inactive ones are all held and never written), or null for every node
+// of the level.
 template <class VC = float, class VF = float>
 __global__ void k_prolong(LevelView F, int CPX, int CNY, const int* __restrict__ list, long long count, const VC* __restrict__ zc,
                           VF* __restrict__ zf, float sp, Ctl ctl) {
     if (skipped(ctl)) return;
     const long long CNX = CPX, CNXY = (long long)CPX * CNY;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < count; t += (long long)gridDim.x * blockDim.x) {
-        const long long fn = list ? (long long)list[t] : t;
-        const uint8_t mask = F.nmask[fn];
+        const long long fn = list ? (long long)__ldg(list + t) : t;
+        const uint8_t mask = __ldg(F.nmask + fn);
         if ((mask & 7) == 7) continue;
         int i, j, k;
         nodeCoords(F, fn, i, j, k);
-        const int i0 = i >> 1, j0 = j >> 1, k0 = k >> 1;
-        const int ni = (i & 1) ? 2 : 1, nj = (j & 1) ? 2 : 1, nk = (k & 1) ? 2 : 1;
-        const float w = ((i & 1) ? 0.5f : 1.f) * ((j & 1) ? 0.5f : 1.f) * ((k & 1) ? 0.5f : 1.f);
-        float s0 = 0, s1 = 0, s2 = 0;
-        for (int c = 0; c < nk; c++)
-            for (int b = 0; b < nj; b++)
-                for (int a = 0; a < ni; a++) {
-                    const VC* p = zc + 3 * ((i0 + a) + (j0 + b) * CNX + (k0 + c) * CNXY);
-                    s0 += w * ldf(p);
-                    s1 += w * ldf(p + 1);
-                    s2 += w * ldf(p + 2);
-                }
+        const float z0 = ldf(zf + 3 * fn), z1 = ldf(zf + 3 * fn + 1), z2 = ldf(zf + 3 * fn + 2);
+        float s[3];
+        prolongAt<1>(CNX, CNXY, zc, i, j, k, s);
         constexpr bool SCALED = !std::is_same<VC, float>::value;
         if (SCALED) {
-            s0 *= sp;
-            s1 *= sp;
-            s2 *= sp;
+            s[0] *= sp;
+            s[1] *= sp;
+            s[2] *= sp;
         }
-        if (!fixedDof(mask, 0)) stv(zf + 3 * fn, ldf(zf + 3 * fn) + s0);
-        if (!fixedDof(mask, 1)) stv(zf + 3 * fn + 1, ldf(zf + 3 * fn + 1) + s1);
-        if (!fixedDof(mask, 2)) stv(zf + 3 * fn + 2, ldf(zf + 3 * fn + 2) + s2);
+        if (!fixedDof(mask, 0)) stv(zf + 3 * fn, z0 + s[0]);
+        if (!fixedDof(mask, 1)) stv(zf + 3 * fn + 1, z1 + s[1]);
+        if (!fixedDof(mask, 2)) stv(zf + 3 * fn + 2, z2 + s[2]);
     }
 }
 
 // coarsest level: z = A^-1 r over the m free DOFs (FP64 dense inverse, one warp per row);
 // r, z are the level's vectors (float or double), held DOFs of z are never written (stay 0)
 // (zs: the FP16 coarse-level vectors' iterate-to-residual scale, a power of two; 1 otherwise)
+// A row's first 512 entries are on their way while the block gathers r.
 template <class TI, class TO>
 __global__ void k_coarse(int m, const int* __restrict__ dof, const double* __restrict__ Ainv, const TI* __restrict__ r, TO* __restrict__ z,
                          double zs, Ctl ctl) {
     if (skipped(ctl)) return;
     extern __shared__ double rs[];
-    for (int q = threadIdx.x; q < m; q += blockDim.x) rs[q] = ldv<double>(r + dof[q]);
-    __syncthreads();
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    for (int row = blockIdx.x * warps + (threadIdx.x >> 5); row < m; row += gridDim.x * warps) {
-        const double* a = Ainv + (size_t)row * m;
+    constexpr int U = 16;
+    double a[U];
+    auto entries = [&](int row, int base) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int c = base + lane + 32 * u;
+            a[u] = (row < m && c < m) ? __ldg(Ainv + (size_t)row * m + c) : 0.0;
+        }
+    };
+    const int row0 = blockIdx.x * warps + (threadIdx.x >> 5);
+    entries(row0, 0);
+#pragma unroll 4
+    for (int q = threadIdx.x; q < m; q += blockDim.x) rs[q] = ldv<double>(r + __ldg(dof + q));
+    __syncthreads();
+    for (int row = row0; row < m; row += gridDim.x * warps) {
+        if (row != row0) entries(row, 0);
         double s = 0;
-        for (int c = lane; c < m; c += 32) s += a[c] * rs[c];
+        for (int base = 0; base < m; base += 32 * U) {
+            if (base) entries(row, base);
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int c = base + lane + 32 * u;
+                if (c < m) s += a[u] * rs[c];
+            }
+        }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
         if (lane == 0) {
-            if constexpr (std::is_same<TO, __half>::value) z[dof[row]] = __double2half(s * zs);
-            else z[dof[row]] = TO(s);
+            if constexpr (std::is_same<TO, __half>::value) z[__ldg(dof + row)] = __double2half(s * zs);
+            else z[__ldg(dof + row)] = TO(s);
         }
     }
 }
@@ -1437,6 +1484,7 @@ struct SharedModel {
     bool blockStencil0 = false;
     int64_t stencilLevels = ~int64_t(1);  // PSFEA_STENCIL_LEVELS: bit l = level l (never level 0)
     int64_t stencilMinNodes = 65536;      // PSFEA_STENCIL_MIN_NODES: smaller node lists keep the gather
+    int64_t pdlCtas = 592;                // PSFEA_PDL_CTAS
     bool foldBranch = true;               // PSFEA_FOLD_BRANCH: the FP32-Krylov fold as a conditional graph branch
     bool exactOneLevel() const { return L.size() == 1 && H.hasFactor(); }
 };
@@ -1466,6 +1514,7 @@ void SharedModel::adopt(Hierarchy&& h) {
     if (const char* e = std::getenv("PSFEA_REFINE_ETA")) refineEta = std::atof(e);
     if (const char* e = std::getenv("PSFEA_STENCIL_LEVELS")) stencilLevels = std::atoll(e) & ~int64_t(1);
     if (const char* e = std::getenv("PSFEA_STENCIL_MIN_NODES")) stencilMinNodes = std::atoll(e);
+    if (const char* e = std::getenv("PSFEA_PDL_CTAS")) pdlCtas = std::atoll(e);
     if (const char* e = std::getenv("PSFEA_FOLD_BRANCH")) foldBranch = std::atoi(e) != 0;
     if (const char* e = std::getenv("PSFEA_BLOCK_STENCIL")) blockStencils = std::atoi(e) != 0;
     if (const char* e = std::getenv("PSFEA_BLOCK_STENCIL0")) blockStencil0 = std::atoi(e) != 0;
@@ -1888,10 +1937,30 @@ struct SolverImpl {
         : M(std::move(model)), H(M->H), L(M->L), cDof(M->cDof), cInv(M->cInv), m(M->m), smCount(M->smCount) {}
     void allocate();
 
+    // While an iteration is recorded (pdl), a kernel of few CTAs after another kernel is launched programmatically: its
+    // launch overlaps the kernel before it, for whose completion it waits in skipped(). PDL_ARMED: from the second kernel
+    // on (the first follows something that is not a kernel)
+    enum { PDL_OFF, PDL_ARMED, PDL_ON };
+    int pdl = PDL_OFF;
     template <class... KArgs, class... Args>
     void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
-        kernel<<<grid, block, smem, s>>>(std::forward<Args>(args)...);
         ++launches;
+        if (pdl == PDL_ON && int64_t(grid.x) <= M->pdlCtas) {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = grid;
+            cfg.blockDim = block;
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = s;
+            cudaLaunchAttribute at{};
+            at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at.val.programmaticStreamSerializationAllowed = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            check(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...), "launch");
+            return;
+        }
+        kernel<<<grid, block, smem, s>>>(std::forward<Args>(args)...);
+        if (pdl == PDL_ARMED) pdl = PDL_ON;
     }
 
     int nodeGrid(int64_t nNodes) const { return gridFor(nNodes, dev::NODE_THREADS, smCount * 16); }
@@ -2464,6 +2533,7 @@ void SolverImpl::recordPlainIteration(dev::Ctl ctl, bool own16) {
                    p.as<double>(), q.as<double>(), nullptr, nullptr, 0.f, 0.f, 0, st(), part(), tick(), ctl);
     }
     const bool one = exactOneLevel();
+    pdl = PDL_ON;
     launch(dev::k_cg_update, vecGrid(pn(0)), dev::VEC_THREADS, 0, stream, pn(0), D.view.nmask, x.as<double>(), r.as<double>(), p.as<double>(),
            q.as<double>(), one ? nullptr : W0.r.as<float>(), D.invD.as<float>(), W0.d.as<float>(), W0.z.as<float>(), D.cf0, st(), part(), tick(),
            ctl);
@@ -2479,6 +2549,7 @@ void SolverImpl::recordPlainIteration(dev::Ctl ctl, bool own16) {
     launch(dev::k_cg_dots, vecGrid(pn(0)), dev::VEC_THREADS, 0, stream, pn(0), D.view.nmask, r.as<double>(), z32, z64.as<double>(),
            q.as<double>(), st(), part(), tick(), ctl);
     launch(dev::k_cg_p, vecGrid(pn(0)), dev::VEC_THREADS, 0, stream, pn(0), D.view.nmask, z32, z64.as<double>(), p.as<double>(), st(), ctl);
+    pdl = PDL_OFF;
 }
 
 // one FP32 CG iteration with the FP64 fold (runs only when due)
@@ -2522,10 +2593,12 @@ void SolverImpl::recordMixedIteration(dev::Ctl ctl, bool refine, bool half) {
             launch(dev::k_mx_rescale, vecGrid(pd(0)), dev::VEC_THREADS, 0, stream, pd(0), W0.r.as<float>(), invD0, d0, z0, D.cf0, st(),
                    dev::Ctl{ctl.skipIf, &st()->restart});
         foldKernels = 0;
+        pdl = half ? PDL_OFF : PDL_ON;  // (the FP16 V-cycle clears a vector between its kernels)
         float* z32 = vcycleFor(half, ctl, M->mixedOwn16, true);
         launch(dev::k_mx_dots, vecGrid(pn(0)), dev::VEC_THREADS, 0, stream, pn(0), D.view.nmask, W0.r.as<float>(), z32, q32.as<float>(), st(),
                part(), tick(), ctl);
         launch(dev::k_mx_p, vecGrid(pn(0)), dev::VEC_THREADS, 0, stream, pn(0), D.view.nmask, z32, p32.as<float>(), st(), ctl);
+        pdl = PDL_OFF;
         return;
     }
     const cudaGraphNode_t* deps = nullptr;
@@ -2557,10 +2630,12 @@ void SolverImpl::recordMixedIteration(dev::Ctl ctl, bool refine, bool half) {
     cudaGraph_t body = nullptr;
     check(cudaStreamEndCapture(stream, &body), "capture the fold");
     stream = mainStream;
+    pdl = half ? PDL_OFF : PDL_ARMED;
     float* z32 = vcycleFor(half, ctl, M->mixedOwn16, true);  // the first smoothing step came with the update or the fold
     launch(dev::k_mx_dots, vecGrid(pn(0)), dev::VEC_THREADS, 0, stream, pn(0), D.view.nmask, W0.r.as<float>(), z32, q32.as<float>(), st(), part(),
            tick(), ctl);
     launch(dev::k_mx_p, vecGrid(pn(0)), dev::VEC_THREADS, 0, stream, pn(0), D.view.nmask, z32, p32.as<float>(), st(), ctl);
+    pdl = PDL_OFF;
 }
 
 void SolverImpl::startSolve(const double* fDev, const double* x0Dev, const ps_solve_opts& o, double* uDev, double* uHost) {
@@ -2679,6 +2754,7 @@ void SolverImpl::startIterations() {
         // counted per fold; a graph's node types are not queried, the driver does not report the
         // conditional node's)
         const int64_t l0 = launches;
+        pdl = PDL_OFF;
         check(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "capture");
         if (mixed) recordMixedIteration(ctl, refine, half);
         else recordPlainIteration(ctl, own16);
@@ -2945,8 +3021,7 @@ struct BlockImpl final : BlockBase {
     }
 
     void coarse(const float* rin, float* zout, dev::Ctl ctl) {
-        const int warpsNeeded = (M->m + (32 / RB) - 1) / (32 / RB);
-        const int grid = std::max(1, std::min(smCount * 8, (warpsNeeded + 7) / 8));
+        const int grid = (M->m + dev::KBC_ROWS - 1) / dev::KBC_ROWS;
         launch(dev::kb_coarse<float, float, RB>, grid, dev::BLOCK_THREADS, 0, M->m, M->cDof.template as<int>(), M->cInv.template as<double>(),
                rin, zout, ctl);
     }
@@ -3002,8 +3077,7 @@ struct BlockImpl final : BlockBase {
     // z of the finest level: the V-cycle (from the fused first step) or the direct solve
     const float* precond(dev::Ctl ctl, bool own16) {
         if (M->exactOneLevel()) {
-            const int warpsNeeded = (M->m + (32 / RB) - 1) / (32 / RB);
-            const int grid = std::max(1, std::min(smCount * 8, (warpsNeeded + 7) / 8));
+            const int grid = (M->m + dev::KBC_ROWS - 1) / dev::KBC_ROWS;
             launch(dev::kb_coarse<double, double, RB>, grid, dev::BLOCK_THREADS, 0, M->m, M->cDof.template as<int>(),
                    M->cInv.template as<double>(), r.template as<double>(), z64.template as<double>(), ctl);
             return nullptr;
