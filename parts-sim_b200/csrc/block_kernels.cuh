@@ -278,9 +278,10 @@ __device__ __forceinline__ void stnBlock(const LevelView& L, const T* __restrict
     acc[2] = a2[2].x + a2[2].y;
 }
 
-// STN: the product from the level's assembled stencils (stn, over act) instead of the gather.
+// STN: the product from the level's assembled stencils (stn, over act) instead of the gather; latency-bound on neighbour values
+// from L2, so at four CTAs an SM (load groups SIMP 96x48x48 x 32: 167.6 ms at two, 165.6 at three, 162.0 at four).
 template <int MODE, bool OWN16, int RB, bool STN = false>
-__global__ void __launch_bounds__(BLOCK_THREADS, 2) kb_op(LevelView L, Coefs<float> C, const int* __restrict__ act, int nAct,
+__global__ void __launch_bounds__(BLOCK_THREADS, STN ? 4 : 2) kb_op(LevelView L, Coefs<float> C, const int* __restrict__ act, int nAct,
                                                        const float* __restrict__ stn, const float* __restrict__ x, float* __restrict__ y,
                                                        const float* __restrict__ r, float* __restrict__ d, float c1, float c2, int raw,
                                                        Ctl ctl) {
@@ -716,23 +717,20 @@ __global__ void kb_rmax(const int* __restrict__ act, int nAct, const uint8_t* __
     }
 }
 
-// z = z32 / vscale at active nodes (voxel_fea.cpp:859-860), 0 for finished right-hand sides
-template <int RB>
-__global__ void kb_vc_store(const int* __restrict__ act, int nAct, const float* __restrict__ z32, double* __restrict__ z, const BlockState* bs) {
-    const long long total = (long long)nAct * 3 * RB;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
-        const long long t = e / (3 * RB);
-        const int rem = int(e - t * 3 * RB), c = rem / RB, q = rem - c * RB;
-        const long long id = (3 * (long long)act[t] + c) * RB + q;
-        z[id] = rhsRunning(bs, q) ? double(z32[id]) / bs->vscale[q] : 0.0;
-    }
-}
-
 // ---- the C ABI's dense vectors (nrhs consecutive vectors of 3 NX NY NZ values, node i + NX (j + NY k))
 // <-> the block layout over pitched nodes; 32 consecutive dense DOFs x RB right-hand sides per
 // thread block through shared memory, so both sides are read and written contiguously. Right-hand
 // sides q >= nrhs read as 0 and are not written back. scale (optional, per right-hand side)
 // multiplies the values on the way.
+// (32-bit index arithmetic where the vector allows it: a 64-bit division is a long software sequence)
+__device__ __forceinline__ long long pitchedDof(long long e, int NX, int PX) {
+    if (e <= 0xffffffffLL) {
+        const unsigned u = unsigned(e), nd = u / 3u, row = nd / unsigned(NX);
+        return 3 * ((long long)(nd - row * unsigned(NX)) + (long long)PX * row) + (u - 3u * nd);
+    }
+    const long long nd = e / 3, row = nd / NX;
+    return 3 * ((nd - row * NX) + (long long)PX * row) + (e - 3 * nd);
+}
 template <int RB>
 __global__ void __launch_bounds__(256) kb_pack(double* __restrict__ dense, int nrhs, long long nDense, double* __restrict__ blk, int NX,
                                                int NY, int PX, int toBlock, const double* __restrict__ scale) {
@@ -747,11 +745,7 @@ __global__ void __launch_bounds__(256) kb_pack(double* __restrict__ dense, int n
             for (int w = threadIdx.x; w < 32 * RB; w += 256) {
                 const int de = w / RB, q = w - de * RB;
                 const long long ee = e0 + de;
-                if (ee < nDense) {
-                    const long long nd = ee / 3, row = nd / NX;
-                    const long long pn = (nd - row * NX) + (long long)PX * row;
-                    blk[(3 * pn + (ee - 3 * nd)) * RB + q] = scale ? tile[q][de] * scale[q] : tile[q][de];
-                }
+                if (ee < nDense) blk[pitchedDof(ee, NX, PX) * RB + q] = scale ? tile[q][de] * scale[q] : tile[q][de];
             }
         } else {
             for (int w = threadIdx.x; w < 32 * RB; w += 256) {
@@ -759,9 +753,7 @@ __global__ void __launch_bounds__(256) kb_pack(double* __restrict__ dense, int n
                 const long long ee = e0 + de;
                 double v = 0.0;
                 if (ee < nDense) {
-                    const long long nd = ee / 3, row = nd / NX;
-                    const long long pn = (nd - row * NX) + (long long)PX * row;
-                    v = blk[(3 * pn + (ee - 3 * nd)) * RB + q];
+                    v = blk[pitchedDof(ee, NX, PX) * RB + q];
                     if (scale) v *= scale[q];
                 }
                 tile[q][de] = v;
@@ -773,6 +765,32 @@ __global__ void __launch_bounds__(256) kb_pack(double* __restrict__ dense, int n
         __syncthreads();
     }
     (void)NY;
+}
+
+// the block preconditioner's result to the caller's dense vectors: z = z32 / vscale at active nodes (voxel_fea.cpp:859-860),
+// 0 elsewhere and for zero vectors
+template <int RB>
+__global__ void __launch_bounds__(256) kb_unpack_z(double* __restrict__ dense, int nvec, long long nDense, const float* __restrict__ z32,
+                                                   const uint8_t* __restrict__ nmask, int NX, int PX, const BlockState* bs) {
+    __shared__ float tile[RB][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
+    for (long long e0 = (long long)blockIdx.x * 32; e0 < nDense; e0 += (long long)gridDim.x * 32) {
+        const long long e = e0 + tx;
+        for (int w = threadIdx.x; w < 32 * RB; w += 256) {
+            const int de = w / RB, q = w - de * RB;
+            const long long ee = e0 + de;
+            float v = 0.f;
+            if (ee < nDense) {
+                const long long pe = pitchedDof(ee, NX, PX);
+                if (nmask[pe / 3] & NM_ACTIVE) v = z32[pe * RB + q];
+            }
+            tile[q][de] = v;
+        }
+        __syncthreads();
+        for (int q = ty; q < nvec && q < RB; q += 8)
+            if (e < nDense) dense[(long long)q * nDense + e] = rhsRunning(bs, q) ? double(tile[q][tx]) / bs->vscale[q] : 0.0;
+        __syncthreads();
+    }
 }
 
 // held DOFs of every right-hand side set to 0 over all pitched nodes (a warm start's held values)

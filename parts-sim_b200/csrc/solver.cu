@@ -1664,17 +1664,23 @@ void SharedModel::uploadLevel(int l) {
     {
         // (the largest grids the 64-bit tile indices of the element-block lists hold)
         if ((h.NX + 31) / 32 > 2047 || (h.NY + 7) / 8 > 2047 || (h.NZ + 3) / 4 > 1023) throw Error(PS_EINVAL, "grid too large for the tile index");
-        std::vector<int64_t> planeActive(size_t(h.NZ), 0);
+        // active nodes, and those of them that touch an own matrix
+        std::vector<int64_t> planeActive(size_t(h.NZ), 0), planeOwn(size_t(h.NZ), 0);
         parallelFor(h.NZ, [&](int64_t k0, int64_t k1) {
             for (int64_t k = k0; k < k1; k++) {
                 const uint8_t* mk = h.nmask.data() + h.node(0, 0, int(k));
-                int64_t n = 0;
-                for (int64_t q = 0; q < int64_t(h.NX) * h.NY; q++) n += (mk[q] & NM_ACTIVE) ? 1 : 0;
+                int64_t n = 0, o = 0;
+                for (int64_t q = 0; q < int64_t(h.NX) * h.NY; q++) {
+                    n += (mk[q] & NM_ACTIVE) ? 1 : 0;
+                    o += (mk[q] & (NM_ACTIVE | NM_PLAIN)) == NM_ACTIVE ? 1 : 0;
+                }
                 planeActive[size_t(k)] = n;
+                planeOwn[size_t(k)] = o;
             }
         }, 8);
-        int64_t active = 0;
+        int64_t active = 0, ownNodes = 0;
         for (int64_t n : planeActive) active += n;
+        for (int64_t n : planeOwn) ownNodes += n;
         D.nActive = int(active);
         if (h.nOwn == 0 && l < 63 && ((ebeLevels >> l) & 1)) {
             // the element-block tiles (8 x 8 x 4 nodes) with an active node
@@ -1700,7 +1706,10 @@ void SharedModel::uploadLevel(int l) {
         // (marched levels with own matrices take a second launch for the nodes that touch one: worth it from 400 k nodes;
         // without, one thread per node is the faster only below some 8 k nodes: 64x16x16 cantilever 1.45 -> 1.26 ms a solve,
         // SIMP 96x48x48 19.6 -> 16.5 ms, while marching that grid's level 1 of 30 k nodes, 85 % own matrices, costs 1.2 ms)
+        // (and where more than half of the active nodes touch an own matrix the march has little to do: the stencils then
+        // take the whole level. Gyroid 256x256x128, level 1 with 97 % such nodes: 31 us a pass saved beside the 122 of the stencils)
         int64_t minNodes = h.nOwn == 0 ? 8000 : 400000;
+        if (2 * ownNodes > active) minNodes = INT64_MAX;
         if (const char* e = std::getenv("PSFEA_TILE_MIN_NODES")) minNodes = std::atoll(e);
         D.m64 = marchCoefs<double>(h.Kb, D.useTiles);
         D.m32 = marchCoefs<float>(h.Kb, D.useTiles);
@@ -3262,10 +3271,8 @@ struct BlockImpl final : BlockBase {
         s.nrhs = nvec;
         *hostState = s;
         check(cudaMemcpyAsync(state.p, hostState, sizeof s, cudaMemcpyHostToDevice, stream), "state");
-        check(cudaMemsetAsync(r.p, 0, r.bytes, stream), "memset");
         pack(rDev, nvec, r.template as<double>(), true);
         launch(dev::kb_rmax<RB>, laneGrid(0), dev::BLOCK_THREADS, 0, act(0), nAct(0), D.view.nmask, r.template as<double>(), bs(), part(), tick());
-        check(cudaMemsetAsync(q.p, 0, q.bytes, stream), "memset");
         if (z64.p) check(cudaMemsetAsync(z64.p, 0, z64.bytes, stream), "memset");
         if (M->exactOneLevel()) {
             // the whole model is the coarsest level: its direct FP64 solve (voxel_fea.cpp:838-842)
@@ -3276,8 +3283,9 @@ struct BlockImpl final : BlockBase {
                    W0.r.template as<float>(), D.invD.template as<float>(), W0.d.template as<float>(), W0.z.template as<float>(), D.cf0, bs(),
                    none);
             const float* z32 = vcycle(0, none, false, true);
-            launch(dev::kb_vc_store<RB>, elemGrid(0), dev::BLOCK_THREADS, 0, act(0), nAct(0), z32, q.template as<double>(), bs());
-            pack(zDev, nvec, q.template as<double>(), false);
+            const dev::LevelView& v = D.view;
+            const int64_t nDense = int64_t(3) * v.NX * v.NY * v.NZ;
+            launch(dev::kb_unpack_z<RB>, gridFor(nDense, 32, smCount * 16), 256, 0, zDev, nvec, (long long)nDense, z32, v.nmask, v.NX, v.PX, bs());
         }
         check(cudaGetLastError(), "block precondition");
         if (caller && caller != stream) {
@@ -3760,11 +3768,10 @@ void Solver::stresses(const double* u, double E, double h, bool principals, floa
     dev::StressCoefs sc;
     for (int a = 0; a < 8; a++)
         for (int i = 0; i < 144; i++) sc.S[a][i] = I.H.el.cornerStress[a][i] * E / h;
-    int64_t scratch = 0;
-    DevMem out;
-    out.alloc(size_t(nn) * 4 * 6, scratch);  // three pitched fields and three dense ones
     I.uploadPitched(u, I.p.as<double>(), 0, I.q.as<double>());
-    float* o = out.as<float>();
+    // three pitched fields and three dense ones, 24 bytes a node: in the residual's vector, which every solve and
+    // preconditioning makes anew (allocating and freeing them on each call waited for the whole device)
+    float* o = I.r.as<float>();
     I.launch(dev::k_stresses, I.nodeGrid(nn), dev::NODE_THREADS, 0, I.stream, v, sc, I.p.as<double>(), principals ? 1 : 0, o, o + nn,
              o + 2 * nn);
     const int64_t nd = L0.nNodes;
