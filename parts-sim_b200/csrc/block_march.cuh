@@ -129,56 +129,47 @@ __global__ void __launch_bounds__(bmThreads<T>(), 1)
     }
 #pragma unroll
     for (int m = 0; m < MINE; m++) mkNext[m] = maskAt(pIn[m], pNode[m], k0 - 1 + BM_PREFETCH);
-    FaceModes<T> P, Q;  // the modes of planes k - 1 and k
+    FaceModes<T> P{}, Q;  // the modes of planes k - 1 and k
+    // (the turns at both ends run the whole body too, as in k_march: hold is 0 outside [k0, k1))
     for (int k = k0 - 1; k <= k1; k++) {
         cpAsyncWait<BM_PREFETCH - 1>();
         __syncthreads();
-        if (k > k0 + 1) finish(k - 2);
-        if (k + BM_PREFETCH <= k1) {  // into a slot whose plane's last readers were done before the barrier
-            stage(k + BM_PREFETCH, mkNext);
+        finish(k - 2);
+        stage(k + BM_PREFETCH, mkNext);  // into a slot whose plane's last readers were done before the barrier
 #pragma unroll
-            for (int m = 0; m < MINE; m++) mkNext[m] = maskAt(pIn[m], pNode[m], k + BM_PREFETCH + 1);
-        } else {
-            cpAsyncCommit();
-        }
-        if (k > k0) {
-            hold = holdNext;  // of plane k - 1
-            if (MODE == BOP_CHEB || MODE == BOP_RESID) {
-                if (own && (hold & NM_ACTIVE)) {
-                    const long long n = (k - 1) * PXY + nodeAt, id = 3 * n * RB + rhs + q;
+        for (int m = 0; m < MINE; m++) mkNext[m] = maskAt(pIn[m] && k + BM_PREFETCH < k1, pNode[m], k + BM_PREFETCH + 1);
+        hold = holdNext;  // of plane k - 1
+        if (MODE == BOP_CHEB || MODE == BOP_RESID) {
+            if (own && (hold & NM_ACTIVE)) {
+                const long long n = (k - 1) * PXY + nodeAt, id = 3 * n * RB + rhs + q;
 #pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        er[c] = __ldg(r + id + c * RB);
-                        if (MODE == BOP_CHEB) {
-                            ed[c] = d[id + c * RB];
-                            ei[c] = __ldg(L.invD + 3 * n + c);
-                        }
+                for (int c = 0; c < 3; c++) {
+                    er[c] = __ldg(r + id + c * RB);
+                    if (MODE == BOP_CHEB) {
+                        ed[c] = d[id + c * RB];
+                        ei[c] = __ldg(L.invD + 3 * n + c);
                     }
                 }
             }
         }
-        holdNext = maskAt(own, nodeAt, k < k1 ? k : -1);
+        holdNext = maskAt(own && k >= k0 && k < k1, nodeAt, k);
         const T s = T(fmaxf(__uint_as_float(wNext), 0.f));  // of the layer below
-        if (k < k1) wNext = (voxIn && unsigned(k) < unsigned(L.nz)) ? __ldg(L.word + k * WXY + wordAt) : 0u;
+        wNext = (voxIn && unsigned(k) < unsigned(L.nz)) ? __ldg(L.word + k * WXY + wordAt) : 0u;
         const T* pl = ring + ((k + 1) & (BM_STAGES - 1)) * PLANE + (vy * (BM_VX + 1) + vx) * BM_NODE + q;
 #pragma unroll
         for (int c = 0; c < 3; c++)
             Q.make(c, pl[c * BM_G], pl[BM_NODE + c * BM_G], pl[(BM_VX + 1) * BM_NODE + c * BM_G], pl[(BM_VX + 2) * BM_NODE + c * BM_G]);
-        if (k >= k0) {
-            T H[3][4];
-            marchLayer<T>(K, s, P, Q, F, H);
-            if (k > k0) {
-                // plane k - 1: the share of the thread's own node stays, those of its face's other corners go to their owners
-                T* sh = shares + ((k - 1) & 1) * 3 * SHARES + col * BM_NODE + q;
+        T H[3][4];
+        marchLayer<T>(K, s, P, Q, F, H);
+        // plane k - 1: the share of the thread's own node stays, those of its face's other corners go to their owners
+        T* sh = shares + ((k - 1) & 1) * 3 * SHARES + col * BM_NODE + q;
 #pragma unroll
-                for (int c = 0; c < 3; c++) {
-                    const T s0 = H[c][0] - H[c][2], s1 = H[c][0] + H[c][2], t0 = H[c][1] - H[c][3], t1 = H[c][1] + H[c][3];
-                    mine[c] = s0 - t0;
-                    sh[c * BM_G] = s0 + t0;
-                    sh[SHARES + c * BM_G] = s1 - t1;
-                    sh[2 * SHARES + c * BM_G] = s1 + t1;
-                }
-            }
+        for (int c = 0; c < 3; c++) {
+            const T s0 = H[c][0] - H[c][2], s1 = H[c][0] + H[c][2], t0 = H[c][1] - H[c][3], t1 = H[c][1] + H[c][3];
+            mine[c] = s0 - t0;
+            sh[c * BM_G] = s0 + t0;
+            sh[SHARES + c * BM_G] = s1 - t1;
+            sh[2 * SHARES + c * BM_G] = s1 + t1;
         }
         P = Q;
     }

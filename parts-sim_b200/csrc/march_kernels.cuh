@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(marchThreads<T>(), 1)
         };
 
         T F[3][4] = {};
-        float er[3], ed[3], ei[3];  // epilogue operands of the plane being completed, loaded a step ahead
+        float er[3] = {}, ed[3] = {}, ei[3] = {};  // epilogue operands of the plane being completed, loaded a step ahead
         unsigned eb = 0, mkNext;
         uint32_t wNext = 0;  // the voxel word above the plane, a step ahead; used as loaded only then
 
@@ -268,72 +268,67 @@ __global__ void __launch_bounds__(marchThreads<T>(), 1)
 #pragma unroll
         for (int p = 0; p < MARCH_PREFETCH; p++) stage(k0 - 1 + p, maskAt(nodeIn, nodeAt, k0 - 1 + p));
         mkNext = maskAt(nodeIn, nodeAt, k0 - 1 + MARCH_PREFETCH);
-        FaceModes<T> P, Q;  // the modes of planes k - 1 and k
+        if (lane == 0) bits[((k0 - 1) & (MARCH_BITS - 1)) * ROWS + warp] = 0u;  // plane k0 - 2
+        FaceModes<T> P{}, Q;  // the modes of planes k - 1 and k
+        // The turns at both ends run the whole body too: planes outside [k0, k1) have no output bits, the layer below
+        // plane k0 - 1 has scale 0 and planes past k1 are staged as zeros. Without branches the compiler can spread the loads and
+        // the epilogue over the arithmetic.
+#pragma unroll 2  // (the modes change places without copies)
         for (int k = k0 - 1; k <= k1; k++) {
             cpAsyncWait<MARCH_PREFETCH - 1>();
             __syncthreads();
-            if (k > k0 + 1) finish(k - 2);
+            finish(k - 2);
             __syncwarp();
-            if (k + MARCH_PREFETCH <= k1) {  // into the slot of plane k - 2, whose last reader was this warp, just now
-                stage(k + MARCH_PREFETCH, mkNext);
-                mkNext = maskAt(nodeIn, nodeAt, k + MARCH_PREFETCH + 1);
-            } else {
-                cpAsyncCommit();
+            stage(k + MARCH_PREFETCH, mkNext);  // into the slot of plane k - 2, whose last reader was this warp, just now
+            mkNext = maskAt(nodeIn && k + MARCH_PREFETCH < k1, nodeAt, k + MARCH_PREFETCH + 1);
+            eb = bits[(k & (MARCH_BITS - 1)) * ROWS + warp];
+            const long long at = 3 * (k - 1) * XXY + valueAt;
+            if (CHEB || RESID)
+#pragma unroll
+                for (int q = 0; q < 3; q++)
+                    if (eb & mq[q]) er[q] = __ldg(r + at + 32 * q);
+            if (CHEB) {
+#pragma unroll
+                for (int q = 0; q < 3; q++)
+                    if (eb & mq[q]) ed[q] = d[at + 32 * q];
+#pragma unroll
+                for (int q = 0; q < 3; q++)
+                    if (eb & mq[q]) ei[q] = __ldg(L.invD + at + 32 * q);
             }
             unsigned hold = 0, holdNext = 0;  // the masks of the warp's own row and the next, plane k - 1
-            if (k > k0) {
-                eb = bits[(k & (MARCH_BITS - 1)) * ROWS + warp];
-                const long long at = 3 * (k - 1) * XXY + valueAt;
-                if (CHEB || RESID)
-#pragma unroll
-                    for (int q = 0; q < 3; q++)
-                        if (eb & mq[q]) er[q] = __ldg(r + at + 32 * q);
-                if (CHEB) {
-#pragma unroll
-                    for (int q = 0; q < 3; q++)
-                        if (eb & mq[q]) ed[q] = d[at + 32 * q];
-#pragma unroll
-                    for (int q = 0; q < 3; q++)
-                        if (eb & mq[q]) ei[q] = __ldg(L.invD + at + 32 * q);
-                }
-                if (MASKED && !io.raw) {
-                    hold = maskAt(nodeIn, nodeAt, k - 1);
-                    holdNext = maskAt(nextIn, nodeAt + L.PX, k - 1);
-                }
+            if (MASKED && !io.raw) {
+                hold = maskAt(nodeIn, nodeAt, k - 1);
+                holdNext = maskAt(nextIn, nodeAt + L.PX, k - 1);
             }
             const T s = T(fmaxf(__uint_as_float(wNext), 0.f));  // of the layer below (an own matrix's word is a negative float or NaN: 0)
-            if (k < k1) wNext = (voxIn && unsigned(k) < unsigned(L.nz)) ? __ldg(L.word + k * WXY + wordAt) : 0u;
+            wNext = (voxIn && unsigned(k) < unsigned(L.nz)) ? __ldg(L.word + k * WXY + wordAt) : 0u;
             const T* pl = ring + ((k + 1) & (MARCH_STAGES - 1)) * PLANE + warp * MARCH_ROW + 3 * lane;
             const int right = lane < 31 ? 3 : 0, up = warp < ROWS - 1 ? MARCH_ROW : 0;
 #pragma unroll
             for (int c = 0; c < 3; c++) Q.make(c, pl[c], pl[c + right], pl[up + c], pl[up + c + right]);
-            if (k >= k0) {
-                T G[3][4];
-                if (sizeof(T) == 4 || s != T(0)) {
-                    marchLayer<T>(K, s, P, Q, F, G);
-                } else {  // an empty voxel (64-bit: whatever x holds at its corners, infinities too, stays out)
+            T G[3][4];
+            if (sizeof(T) == 4 || s != T(0)) {
+                marchLayer<T>(K, s, P, Q, F, G);
+            } else {  // an empty voxel (64-bit: whatever x holds at its corners, infinities too, stays out)
 #pragma unroll
-                    for (int c = 0; c < 3; c++)
+                for (int c = 0; c < 3; c++)
 #pragma unroll
-                        for (int m = 0; m < 4; m++) {
-                            G[c][m] = F[c][m];
-                            F[c][m] = T(0);
-                        }
-                }
-                if (k > k0) {
-                    // plane k - 1 back to its nodes: x neighbours by shuffles, the next row's share to its warp
-                    T* sm = sums + (k & 1) * 2 * PLANE + warp * MARCH_ROW + 3 * lane;
-#pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        const T s0 = G[c][0] - G[c][2], s1 = G[c][0] + G[c][2], t0 = G[c][1] - G[c][3], t1 = G[c][1] + G[c][3];
-                        T own = s0 - t0 + __shfl_up_sync(0xffffffffu, s0 + t0, 1);
-                        T next = s1 - t1 + __shfl_up_sync(0xffffffffu, s1 + t1, 1);
-                        if (MASKED && !io.raw && ((hold >> c) & 1u)) own = T(0);
-                        if (MASKED && !io.raw && ((holdNext >> c) & 1u)) next = T(0);
-                        sm[c] = own;
-                        sm[PLANE + c] = next;
+                    for (int m = 0; m < 4; m++) {
+                        G[c][m] = F[c][m];
+                        F[c][m] = T(0);
                     }
-                }
+            }
+            // plane k - 1 back to its nodes: x neighbours by shuffles, the next row's share to its warp
+            T* sm = sums + (k & 1) * 2 * PLANE + warp * MARCH_ROW + 3 * lane;
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const T s0 = G[c][0] - G[c][2], s1 = G[c][0] + G[c][2], t0 = G[c][1] - G[c][3], t1 = G[c][1] + G[c][3];
+                T own = s0 - t0 + __shfl_up_sync(0xffffffffu, s0 + t0, 1);
+                T next = s1 - t1 + __shfl_up_sync(0xffffffffu, s1 + t1, 1);
+                if (MASKED && !io.raw && ((hold >> c) & 1u)) own = T(0);
+                if (MASKED && !io.raw && ((holdNext >> c) & 1u)) next = T(0);
+                sm[c] = own;
+                sm[PLANE + c] = next;
             }
             P = Q;
         }
