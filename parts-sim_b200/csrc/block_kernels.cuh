@@ -367,8 +367,7 @@ __global__ void kb_restrict(LevelView F, LevelView C, const int* __restrict__ cA
         const uint8_t mask = C.nmask[cn];
         int I, J, K;
         nodeCoords(C, cn, I, J, K);
-        float sv[3];
-        restrictAt<RB>(F, rf + q, I, J, K, sv);
+        Values<3> sv = restrictAt<RB, 3>(F, rf + q, I, J, K);
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             const long long id = (3 * cn + c) * RB + q;
@@ -718,10 +717,9 @@ __global__ void kb_rmax(const int* __restrict__ act, int nAct, const uint8_t* __
 }
 
 // ---- the C ABI's dense vectors (nrhs consecutive vectors of 3 NX NY NZ values, node i + NX (j + NY k))
-// <-> the block layout over pitched nodes; 32 consecutive dense DOFs x RB right-hand sides per
-// thread block through shared memory, so both sides are read and written contiguously. Right-hand
-// sides q >= nrhs read as 0 and are not written back. scale (optional, per right-hand side)
-// multiplies the values on the way.
+// <-> the block layout over pitched nodes; 2048 values at a time (PACK_DOFS consecutive dense DOFs x RB right-hand sides)
+// through shared memory, so both sides are read and written contiguously, eight independent values a thread, and a
+// DOF's place is computed once for its right-hand sides. Right-hand sides q >= nrhs read as 0 and are not written back.
 // (32-bit index arithmetic where the vector allows it: a 64-bit division is a long software sequence)
 __device__ __forceinline__ long long pitchedDof(long long e, int NX, int PX) {
     if (e <= 0xffffffffLL) {
@@ -731,40 +729,43 @@ __device__ __forceinline__ long long pitchedDof(long long e, int NX, int PX) {
     const long long nd = e / 3, row = nd / NX;
     return 3 * ((nd - row * NX) + (long long)PX * row) + (e - 3 * nd);
 }
+template <int RB> __host__ __device__ constexpr int packDofs() { return 2048 / RB; }
 template <int RB>
 __global__ void __launch_bounds__(256) kb_pack(double* __restrict__ dense, int nrhs, long long nDense, double* __restrict__ blk, int NX,
-                                               int NY, int PX, int toBlock, const double* __restrict__ scale) {
-    __shared__ double tile[RB][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
-    for (long long e0 = (long long)blockIdx.x * 32; e0 < nDense; e0 += (long long)gridDim.x * 32) {
-        const long long e = e0 + tx;
+                                               int PX, int toBlock) {
+    constexpr int PK = packDofs<RB>();
+    __shared__ double tile[RB][PK + 1];
+    __shared__ long long pos[PK];
+    for (long long e0 = (long long)blockIdx.x * PK; e0 < nDense; e0 += (long long)gridDim.x * PK) {
+        if (threadIdx.x < PK) pos[threadIdx.x] = e0 + threadIdx.x < nDense ? pitchedDof(e0 + threadIdx.x, NX, PX) : -1;
         if (toBlock) {
-            for (int q = ty; q < RB; q += 8) tile[q][tx] = (q < nrhs && e < nDense) ? dense[(long long)q * nDense + e] : 0.0;
+#pragma unroll
+            for (int w = threadIdx.x; w < 2048; w += 256) {
+                const int q = w / PK, de = w % PK;
+                tile[q][de] = (q < nrhs && e0 + de < nDense) ? dense[(long long)q * nDense + e0 + de] : 0.0;
+            }
             __syncthreads();
-            // write: for each of the 32 DOFs, the RB values of its right-hand sides
-            for (int w = threadIdx.x; w < 32 * RB; w += 256) {
-                const int de = w / RB, q = w - de * RB;
-                const long long ee = e0 + de;
-                if (ee < nDense) blk[pitchedDof(ee, NX, PX) * RB + q] = scale ? tile[q][de] * scale[q] : tile[q][de];
+#pragma unroll
+            for (int w = threadIdx.x; w < 2048; w += 256) {
+                const int de = w / RB, q = w % RB;
+                if (pos[de] >= 0) blk[pos[de] * RB + q] = tile[q][de];
             }
         } else {
-            for (int w = threadIdx.x; w < 32 * RB; w += 256) {
-                const int de = w / RB, q = w - de * RB;
-                const long long ee = e0 + de;
-                double v = 0.0;
-                if (ee < nDense) {
-                    v = blk[pitchedDof(ee, NX, PX) * RB + q];
-                    if (scale) v *= scale[q];
-                }
-                tile[q][de] = v;
+            __syncthreads();
+#pragma unroll
+            for (int w = threadIdx.x; w < 2048; w += 256) {
+                const int de = w / RB, q = w % RB;
+                tile[q][de] = pos[de] >= 0 ? blk[pos[de] * RB + q] : 0.0;
             }
             __syncthreads();
-            for (int q = ty; q < nrhs && q < RB; q += 8)
-                if (e < nDense) dense[(long long)q * nDense + e] = tile[q][tx];
+#pragma unroll
+            for (int w = threadIdx.x; w < 2048; w += 256) {
+                const int q = w / PK, de = w % PK;
+                if (q < nrhs && e0 + de < nDense) dense[(long long)q * nDense + e0 + de] = tile[q][de];
+            }
         }
         __syncthreads();
     }
-    (void)NY;
 }
 
 // the block preconditioner's result to the caller's dense vectors: z = z32 / vscale at active nodes (voxel_fea.cpp:859-860),
@@ -772,23 +773,29 @@ __global__ void __launch_bounds__(256) kb_pack(double* __restrict__ dense, int n
 template <int RB>
 __global__ void __launch_bounds__(256) kb_unpack_z(double* __restrict__ dense, int nvec, long long nDense, const float* __restrict__ z32,
                                                    const uint8_t* __restrict__ nmask, int NX, int PX, const BlockState* bs) {
-    __shared__ float tile[RB][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads
-    for (long long e0 = (long long)blockIdx.x * 32; e0 < nDense; e0 += (long long)gridDim.x * 32) {
-        const long long e = e0 + tx;
-        for (int w = threadIdx.x; w < 32 * RB; w += 256) {
-            const int de = w / RB, q = w - de * RB;
-            const long long ee = e0 + de;
-            float v = 0.f;
-            if (ee < nDense) {
-                const long long pe = pitchedDof(ee, NX, PX);
-                if (nmask[pe / 3] & NM_ACTIVE) v = z32[pe * RB + q];
-            }
-            tile[q][de] = v;
+    constexpr int PK = packDofs<RB>();
+    __shared__ float tile[RB][PK + 1];
+    __shared__ long long pos[PK];
+    __shared__ double scale[RB];  // vscale, or 0 for a zero vector
+    if (threadIdx.x < RB) scale[threadIdx.x] = rhsRunning(bs, threadIdx.x) ? bs->vscale[threadIdx.x] : 0.0;
+    for (long long e0 = (long long)blockIdx.x * PK; e0 < nDense; e0 += (long long)gridDim.x * PK) {
+        if (threadIdx.x < PK) {
+            long long p = e0 + threadIdx.x < nDense ? pitchedDof(e0 + threadIdx.x, NX, PX) : -1;
+            if (p >= 0 && !(nmask[p / 3] & NM_ACTIVE)) p = -1;
+            pos[threadIdx.x] = p;
         }
         __syncthreads();
-        for (int q = ty; q < nvec && q < RB; q += 8)
-            if (e < nDense) dense[(long long)q * nDense + e] = rhsRunning(bs, q) ? double(tile[q][tx]) / bs->vscale[q] : 0.0;
+#pragma unroll
+        for (int w = threadIdx.x; w < 2048; w += 256) {
+            const int de = w / RB, q = w % RB;
+            tile[q][de] = pos[de] >= 0 ? z32[pos[de] * RB + q] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int w = threadIdx.x; w < 2048; w += 256) {
+            const int q = w / PK, de = w % PK;
+            if (q < nvec && e0 + de < nDense) dense[(long long)q * nDense + e0 + de] = scale[q] != 0.0 ? double(tile[q][de]) / scale[q] : 0.0;
+        }
         __syncthreads();
     }
 }

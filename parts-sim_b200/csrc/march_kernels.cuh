@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(marchThreads<T>(), 1)
         T F[3][4] = {};
         float er[3] = {}, ed[3] = {}, ei[3] = {};  // epilogue operands of the plane being completed, loaded a step ahead
         unsigned eb = 0, mkNext;
+        unsigned holdAhead = 0, holdNextAhead = 0;  // the masks of the warp's own row and the next, a step ahead
         uint32_t wNext = 0;  // the voxel word above the plane, a step ahead; used as loaded only then
 
         // the finished sums of plane k (in shared memory) through the epilogue
@@ -295,10 +296,10 @@ __global__ void __launch_bounds__(marchThreads<T>(), 1)
                 for (int q = 0; q < 3; q++)
                     if (eb & mq[q]) ei[q] = __ldg(L.invD + at + 32 * q);
             }
-            unsigned hold = 0, holdNext = 0;  // the masks of the warp's own row and the next, plane k - 1
+            const unsigned hold = holdAhead, holdNext = holdNextAhead;  // plane k - 1
             if (MASKED && !io.raw) {
-                hold = maskAt(nodeIn, nodeAt, k - 1);
-                holdNext = maskAt(nextIn, nodeAt + L.PX, k - 1);
+                holdAhead = maskAt(nodeIn, nodeAt, k);
+                holdNextAhead = maskAt(nextIn, nodeAt + L.PX, k);
             }
             const T s = T(fmaxf(__uint_as_float(wNext), 0.f));  // of the layer below (an own matrix's word is a negative float or NaN: 0)
             wNext = (voxIn && unsigned(k) < unsigned(L.nz)) ? __ldg(L.word + k * WXY + wordAt) : 0u;

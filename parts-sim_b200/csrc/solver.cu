@@ -335,14 +335,18 @@ __global__ void k_cheb_first(long long nDof, const V* __restrict__ r, const floa
     }
 }
 
-// Sum over the fine nodes 2I + (-1 .. 1) per axis, weights 1, 1/2 per axis off the centre, of the fine vector's three
-// components (S: the stride of consecutive DOFs, rf at the lane's right-hand side). Written without branches, so that
+// Sum over the fine nodes 2I + (-1 .. 1) per axis, weights 1, 1/2 per axis off the centre, of COMPS components of the fine
+// vector (S: the stride of consecutive DOFs, rf at the lane's right-hand side and first component). Written without branches, so that
 // all 81 loads are in flight at once (a loop with bounds tests was a chain of 27 L2 latencies: 7 us on the smallest
 // levels, where a pass is nothing else): a neighbour outside the grid reads the nearest node of the grid with weight 0.
-template <int S, class VF>
-__device__ __forceinline__ void restrictAt(const LevelView& F, const VF* __restrict__ rf, int I, int J, int K, float s[3]) {
+template <int N> struct Values {
+    float v[N];
+    __device__ __forceinline__ float& operator[](int c) { return v[c]; }
+};
+template <int S, int COMPS, class VF>
+__device__ __forceinline__ Values<COMPS> restrictAt(const LevelView& F, const VF* __restrict__ rf, int I, int J, int K) {
+    Values<COMPS> s{};
     const long long FPX = F.PX, FPXY = (long long)F.PX * F.NY;
-    s[0] = s[1] = s[2] = 0.f;
 #pragma unroll
     for (int dk = -1; dk <= 1; dk++) {
         const int k = 2 * K + dk, kc = min(max(k, 0), F.NZ - 1);
@@ -356,42 +360,40 @@ __device__ __forceinline__ void restrictAt(const LevelView& F, const VF* __restr
                 const int i = 2 * I + di, ic = min(max(i, 0), F.NX - 1);
                 const float w = i == ic ? (di ? 0.5f : 1.f) * wj : 0.f;
                 const VF* p = rf + 3 * S * (ic + jc * FPX + kc * FPXY);
-                s[0] += w * ldv<float>(p);
-                s[1] += w * ldv<float>(p + S);
-                s[2] += w * ldv<float>(p + 2 * S);
+#pragma unroll
+                for (int c = 0; c < COMPS; c++) s[c] += w * ldv<float>(p + c * S);
             }
         }
     }
+    return s;
 }
 
 // rc = P^T rf gathered per coarse node: fine 2I (weight 1) and 2I +- 1 (weight 1/2) per axis;
 // held / inactive coarse DOFs 0. VF / VC: the fine / coarse storage (float, or __half for the FP16
 // coarse-level vectors, whose residual scales differ by the power of two sr: rc = sr P^T rf).
+// One thread a coarse DOF: its 27 loads fit in registers at once (81 of a whole node did not: 5.1 us on a level of some
+// hundred nodes).
 template <class VF = float, class VC = float>
 __global__ void k_restrict(LevelView F, LevelView C, const VF* __restrict__ rf, VC* __restrict__ rc, VC* __restrict__ dc,
                            VC* __restrict__ zc, float c0, float sr, Ctl ctl) {
     if (skipped(ctl)) return;
-    for (long long cn = blockIdx.x * (long long)blockDim.x + threadIdx.x; cn < C.nNodes; cn += (long long)gridDim.x * blockDim.x) {
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < 3 * C.nNodes; e += (long long)gridDim.x * blockDim.x) {
+        const long long cn = e <= 0xffffffffLL ? (long long)(unsigned(e) / 3u) : e / 3;
+        const int q = int(e - 3 * cn);
         const uint8_t mask = __ldg(C.nmask + cn);
-        float sv[3] = {0.f, 0.f, 0.f}, iv[3] = {0.f, 0.f, 0.f};
-        if (mask & NM_ACTIVE) {
+        float v = 0.f, iv = 0.f;
+        if (!fixedDof(mask, q)) {
             int I, J, K;
             nodeCoords(C, cn, I, J, K);
-            if (dc)
-#pragma unroll
-                for (int q = 0; q < 3; q++) iv[q] = __ldg(C.invD + 3 * cn + q);
-            restrictAt<1>(F, rf, I, J, K, sv);
+            if (dc) iv = __ldg(C.invD + e);
+            v = restrictAt<1, 1>(F, rf + q, I, J, K)[0];
+            if (!std::is_same<VC, float>::value) v *= sr;
         }
-        constexpr bool SCALED = !std::is_same<VC, float>::value;
-#pragma unroll
-        for (int q = 0; q < 3; q++) {
-            const float v = fixedDof(mask, q) ? 0.f : (SCALED ? sr * sv[q] : sv[q]);
-            stv(rc + 3 * cn + q, v);
-            if (dc) {  // the coarse level's first smoothing step, d = z = c0 D^-1 r
-                const float dv = c0 * iv[q] * v;
-                stv(dc + 3 * cn + q, dv);
-                stv(zc + 3 * cn + q, dv);
-            }
+        stv(rc + e, v);
+        if (dc) {  // the coarse level's first smoothing step, d = z = c0 D^-1 r
+            const float dv = c0 * iv * v;
+            stv(dc + e, dv);
+            stv(zc + e, dv);
         }
     }
 }
@@ -2336,7 +2338,7 @@ float* SolverImpl::vcycle(int l, dev::Ctl ctl, bool own16, bool firstDone) {
     // restriction, with the coarse level's first smoothing step fused in (unless it is the dense solve)
     const bool fuse = !(l + 1 == last && H.hasFactor());
     const float c0c = (l + 1 == last) ? C.omega : C.cf0;
-    launch(dev::k_restrict<float, float>, gridFor(pn(l + 1), 256, smCount * 16), 256, 0, stream, D.view, C.view, b, Wc.r.as<float>(),
+    launch(dev::k_restrict<float, float>, gridFor(pd(l + 1), 256, smCount * 16), 256, 0, stream, D.view, C.view, b, Wc.r.as<float>(),
            fuse ? Wc.d.as<float>() : nullptr, fuse ? Wc.z.as<float>() : nullptr, c0c, 1.f, ctl);
     float* zc = vcycle(l + 1, ctl, own16, fuse);
     {
@@ -2400,7 +2402,7 @@ float* SolverImpl::vcycleHalf(dev::Ctl ctl, bool own16, bool firstDone) {
     op32<dev::OP_RESID>(0, a, b, 0.f, 0.f, ctl, own16);
     const bool fuse = !(1 == last && H.hasFactor());
     const float c0c = (1 == last) ? C.omega : C.cf0;
-    launch(dev::k_restrict<float, __half>, gridFor(pn(1), 256, smCount * 16), 256, 0, stream, D.view, C.view, b, Wc.r.as<__half>(),
+    launch(dev::k_restrict<float, __half>, gridFor(pd(1), 256, smCount * 16), 256, 0, stream, D.view, C.view, b, Wc.r.as<__half>(),
            fuse ? Wc.d.as<__half>() : nullptr, fuse ? Wc.z.as<__half>() : nullptr, c0c * dc, 0.125f, ctl);
     const __half* zc = vcycle16(1, ctl, own16, fuse);
     {
@@ -2461,7 +2463,7 @@ __half* SolverImpl::vcycle16(int l, dev::Ctl ctl, bool own16, bool firstDone) {
     op16<dev::OP_RESID>(l, a, b, 0.f, 0.f, ctl, own16);
     const bool fuse = !(l + 1 == last && H.hasFactor());
     const float c0c = (l + 1 == last) ? C.omega : C.cf0;
-    launch(dev::k_restrict<__half, __half>, gridFor(pn(l + 1), 256, smCount * 16), 256, 0, stream, D.view, C.view, b, Wc.r.as<__half>(),
+    launch(dev::k_restrict<__half, __half>, gridFor(pd(l + 1), 256, smCount * 16), 256, 0, stream, D.view, C.view, b, Wc.r.as<__half>(),
            fuse ? Wc.d.as<__half>() : nullptr, fuse ? Wc.z.as<__half>() : nullptr, c0c * dc, 0.125f, ctl);
     const __half* zc = vcycle16(l + 1, ctl, own16, fuse);
     {
@@ -3165,12 +3167,12 @@ struct BlockImpl final : BlockBase {
                p.template as<double>(), bs(), ctl);
     }
 
-    // dense <-> block (device to device); scale per right-hand side or null
-    void pack(const double* dense, int nrhs, double* blk, bool toBlock, const double* scale = nullptr) {
+    // dense <-> block (device to device)
+    void pack(const double* dense, int nrhs, double* blk, bool toBlock) {
         const dev::LevelView& v = L[0].view;
         const int64_t nDense = int64_t(3) * v.NX * v.NY * v.NZ;
-        launch(dev::kb_pack<RB>, gridFor(nDense, 32, smCount * 16), 256, 0, const_cast<double*>(dense), nrhs, (long long)nDense, blk, v.NX,
-               v.NY, v.PX, toBlock ? 1 : 0, scale);
+        launch(dev::kb_pack<RB>, gridFor(nDense, dev::packDofs<RB>(), smCount * 16), 256, 0, const_cast<double*>(dense), nrhs, (long long)nDense, blk,
+               v.NX, v.PX, toBlock ? 1 : 0);
     }
 
     void readState() {
@@ -3341,7 +3343,7 @@ struct BlockImpl final : BlockBase {
             const float* z32 = vcycle(0, none, false, true);
             const dev::LevelView& v = D.view;
             const int64_t nDense = int64_t(3) * v.NX * v.NY * v.NZ;
-            launch(dev::kb_unpack_z<RB>, gridFor(nDense, 32, smCount * 16), 256, 0, zDev, nvec, (long long)nDense, z32, v.nmask, v.NX, v.PX, bs());
+            launch(dev::kb_unpack_z<RB>, gridFor(nDense, dev::packDofs<RB>(), smCount * 16), 256, 0, zDev, nvec, (long long)nDense, z32, v.nmask, v.NX, v.PX, bs());
         }
         check(cudaGetLastError(), "block precondition");
         if (caller && caller != stream) {
