@@ -73,6 +73,39 @@ __device__ __forceinline__ bool skipped(const Ctl& c) {
     return false;
 }
 
+// Loads of the model's own data (written before the first iteration), placed before skipped(): under a programmatic
+// launch they are on their way while the kernel before still runs. (volatile: to stay where they are)
+__device__ __forceinline__ int ldModel(const int* p) {
+    int v;
+    asm volatile("ld.global.nc.s32 %0, [%1];\n" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ unsigned ldModel(const uint8_t* p) {
+    unsigned v;
+    asm volatile("ld.global.nc.u8 %0, [%1];\n" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float ldModel(const float* p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];\n" : "=f"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ double ldModel(const double* p) {
+    double v;
+    asm volatile("ld.global.nc.f64 %0, [%1];\n" : "=d"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ldModel(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint64_t ldModel(const uint64_t* p) {
+    uint64_t v;
+    asm volatile("ld.global.nc.u64 %0, [%1];\n" : "=l"(v) : "l"(p));
+    return v;
+}
+
 __device__ __forceinline__ bool fixedDof(uint8_t mask, int d) { return (mask >> d) & 1; }
 
 constexpr int NODE_THREADS = 128;
@@ -376,9 +409,15 @@ __device__ __forceinline__ Values<COMPS> restrictAt(const LevelView& F, const VF
 template <class VF = float, class VC = float>
 __global__ void k_restrict(LevelView F, LevelView C, const VF* __restrict__ rf, VC* __restrict__ rc, VC* __restrict__ dc,
                            VC* __restrict__ zc, float c0, float sr, Ctl ctl) {
+    const long long e0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    auto nodeOf = [](long long e) { return e <= 0xffffffffLL ? (long long)(unsigned(e) / 3u) : e / 3; };
+    if (e0 < 3 * C.nNodes) {  // into L1, for the first turn below
+        ldModel(C.nmask + nodeOf(e0));
+        ldModel(C.invD + e0);
+    }
     if (skipped(ctl)) return;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < 3 * C.nNodes; e += (long long)gridDim.x * blockDim.x) {
-        const long long cn = e <= 0xffffffffLL ? (long long)(unsigned(e) / 3u) : e / 3;
+    for (long long e = e0; e < 3 * C.nNodes; e += (long long)gridDim.x * blockDim.x) {
+        const long long cn = nodeOf(e);
         const int q = int(e - 3 * cn);
         const uint8_t mask = __ldg(C.nmask + cn);
         float v = 0.f, iv = 0.f;
@@ -426,9 +465,11 @@ __device__ __forceinline__ void prolongAt(long long CNX, long long CNXY, const V
 template <class VC = float, class VF = float>
 __global__ void k_prolong(LevelView F, int CPX, int CNY, const int* __restrict__ list, long long count, const VC* __restrict__ zc,
                           VF* __restrict__ zf, float sp, Ctl ctl) {
-    if (skipped(ctl)) return;
     const long long CNX = CPX, CNXY = (long long)CPX * CNY;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < count; t += (long long)gridDim.x * blockDim.x) {
+    const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (t0 < count) ldModel(F.nmask + (list ? (long long)ldModel(list + t0) : t0));  // into L1, for the first turn below
+    if (skipped(ctl)) return;
+    for (long long t = t0; t < count; t += (long long)gridDim.x * blockDim.x) {
         const long long fn = list ? (long long)__ldg(list + t) : t;
         const uint8_t mask = __ldg(F.nmask + fn);
         if ((mask & 7) == 7) continue;
@@ -452,11 +493,10 @@ __global__ void k_prolong(LevelView F, int CPX, int CNY, const int* __restrict__
 // coarsest level: z = A^-1 r over the m free DOFs (FP64 dense inverse, one warp per row);
 // r, z are the level's vectors (float or double), held DOFs of z are never written (stay 0)
 // (zs: the FP16 coarse-level vectors' iterate-to-residual scale, a power of two; 1 otherwise)
-// A row's first 512 entries are on their way while the block gathers r.
+// A row's first 512 entries are on their way before the kernel before is done and while the block gathers r.
 template <class TI, class TO>
 __global__ void k_coarse(int m, const int* __restrict__ dof, const double* __restrict__ Ainv, const TI* __restrict__ r, TO* __restrict__ z,
                          double zs, Ctl ctl) {
-    if (skipped(ctl)) return;
     extern __shared__ double rs[];
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     constexpr int U = 16;
@@ -465,11 +505,12 @@ __global__ void k_coarse(int m, const int* __restrict__ dof, const double* __res
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int c = base + lane + 32 * u;
-            a[u] = (row < m && c < m) ? __ldg(Ainv + (size_t)row * m + c) : 0.0;
+            a[u] = (row < m && c < m) ? ldModel(Ainv + (size_t)row * m + c) : 0.0;
         }
     };
     const int row0 = blockIdx.x * warps + (threadIdx.x >> 5);
     entries(row0, 0);
+    if (skipped(ctl)) return;
 #pragma unroll 4
     for (int q = threadIdx.x; q < m; q += blockDim.x) rs[q] = ldv<double>(r + __ldg(dof + q));
     __syncthreads();
@@ -1542,7 +1583,6 @@ struct SharedModel {
     bool blockStencil0 = false;
     int64_t stencilLevels = ~int64_t(1);  // PSFEA_STENCIL_LEVELS: bit l = level l (never level 0)
     int64_t stencilMinNodes = 65536;      // PSFEA_STENCIL_MIN_NODES: smaller node lists keep the gather
-    int64_t pdlCtas = 592;                // PSFEA_PDL_CTAS
     bool foldBranch = true;               // PSFEA_FOLD_BRANCH: the FP32-Krylov fold as a conditional graph branch
     bool exactOneLevel() const { return L.size() == 1 && H.hasFactor(); }
 };
@@ -1572,7 +1612,6 @@ void SharedModel::adopt(Hierarchy&& h) {
     if (const char* e = std::getenv("PSFEA_REFINE_ETA")) refineEta = std::atof(e);
     if (const char* e = std::getenv("PSFEA_STENCIL_LEVELS")) stencilLevels = std::atoll(e) & ~int64_t(1);
     if (const char* e = std::getenv("PSFEA_STENCIL_MIN_NODES")) stencilMinNodes = std::atoll(e);
-    if (const char* e = std::getenv("PSFEA_PDL_CTAS")) pdlCtas = std::atoll(e);
     if (const char* e = std::getenv("PSFEA_FOLD_BRANCH")) foldBranch = std::atoi(e) != 0;
     if (const char* e = std::getenv("PSFEA_BLOCK_STENCIL")) blockStencils = std::atoi(e) != 0;
     if (const char* e = std::getenv("PSFEA_BLOCK_STENCIL0")) blockStencil0 = std::atoi(e) != 0;
@@ -2004,15 +2043,16 @@ struct SolverImpl {
         : M(std::move(model)), H(M->H), L(M->L), cDof(M->cDof), cInv(M->cInv), m(M->m), smCount(M->smCount) {}
     void allocate();
 
-    // While an iteration is recorded (pdl), a kernel of few CTAs after another kernel is launched programmatically: its
-    // launch overlaps the kernel before it, for whose completion it waits in skipped(). PDL_ARMED: from the second kernel
-    // on (the first follows something that is not a kernel)
+    // While an iteration is recorded (pdl), a kernel after another kernel is launched programmatically: its launch and its
+    // loads of the model's data overlap the kernel before it, for whose completion it waits in skipped() (box 57x41x33 7.95
+    // -> 7.38 ms a solve, SIMP 96x48x48 10.46 -> 9.73, SIMP 192x96x96 40.4 -> 39.2; restricted to launches of at most 592
+    // CTAs 7.41, 9.85, 39.6). PDL_ARMED: from the second kernel on (the first follows something that is not a kernel)
     enum { PDL_OFF, PDL_ARMED, PDL_ON };
     int pdl = PDL_OFF;
     template <class... KArgs, class... Args>
     void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
         ++launches;
-        if (pdl == PDL_ON && int64_t(grid.x) <= M->pdlCtas) {
+        if (pdl == PDL_ON) {
             cudaLaunchConfig_t cfg{};
             cfg.gridDim = grid;
             cfg.blockDim = block;

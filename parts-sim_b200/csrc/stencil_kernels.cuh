@@ -177,14 +177,18 @@ template <int MODE>
 __global__ void __launch_bounds__(256) k_stn8(LevelView L, const int* __restrict__ list, int count, const float4* __restrict__ stn,
                                               const float* __restrict__ x, float* __restrict__ y, const float* __restrict__ r,
                                               float* __restrict__ d, float c1, float c2, int raw, Ctl ctl) {
-    if (skipped(ctl)) return;
     const int lane = threadIdx.x & 7;
     const long long at = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3;
     const long long t = at < count ? at : count - 1;  // (a repeat of the last node, not stored)
+    const long long n = ldModel(list + t), NX = L.PX, NXY = (long long)L.PX * L.NY;
     float4 cf[9];
 #pragma unroll
-    for (int s = 0; s < 9; s++) cf[s] = __ldg(stn + (t * 9 + s) * 8 + lane);
-    const long long n = __ldg(list + t), NX = L.PX, NXY = (long long)L.PX * L.NY;
+    for (int s = 0; s < 9; s++) cf[s] = ldModel(stn + (t * 9 + s) * 8 + lane);
+    const int q = lane < 3 ? lane : 0;
+    const long long id = 3 * n + q;
+    const uint8_t mask = uint8_t(ldModel(L.nmask + n));
+    const float iv = MODE == TOP_CHEB ? ldModel(L.invD + id) : 0.f;
+    if (skipped(ctl)) return;
     float xm[4][3];
 #pragma unroll
     for (int u = 0; u < 4; u++) {
@@ -195,14 +199,10 @@ __global__ void __launch_bounds__(256) k_stn8(LevelView L, const int* __restrict
         xm[u][1] = __ldg(xp + 1);
         xm[u][2] = __ldg(xp + 2);
     }
-    const int q = lane < 3 ? lane : 0;
-    const long long id = 3 * n + q;
-    const uint8_t mask = __ldg(L.nmask + n);
-    float rv = 0.f, dv = 0.f, iv = 0.f, xv = 0.f;
+    float rv = 0.f, dv = 0.f, xv = 0.f;
     if (MODE != TOP_APPLY) rv = __ldg(r + id);
     if (MODE == TOP_CHEB) {
         dv = d[id];
-        iv = __ldg(L.invD + id);
         xv = __ldg(x + id);
     }
     float a[3] = {0.f, 0.f, 0.f};
