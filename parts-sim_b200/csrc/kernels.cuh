@@ -360,9 +360,6 @@ __device__ __forceinline__ void mbarInit(uint64_t* bar, unsigned count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smemAddr(bar)), "r"(count) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
 }
-__device__ __forceinline__ void mbarExpectTx(uint64_t* bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smemAddr(bar)), "r"(bytes) : "memory");
-}
 __device__ __forceinline__ bool mbarTryWait(uint64_t* bar, unsigned parity) {
     unsigned ok;
     asm volatile(
@@ -380,8 +377,6 @@ __device__ __forceinline__ bool mbarWaitParity(uint64_t* bar, unsigned parity, u
     return false;
 }
 __device__ __forceinline__ bool mbarWait(uint64_t* bar, unsigned limit) { return mbarWaitParity(bar, 0, limit); }
-// makes this thread's shared-memory writes visible to later TMA (async proxy) reads
-__device__ __forceinline__ void fenceAsyncShared() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
 }  // namespace dev
 }  // namespace psfea
