@@ -25,13 +25,15 @@
 // move in fully coalesced accesses, at output nodes only, so that the empty space of a lattice costs no memory
 // traffic beyond whole 32-byte sectors. Sums run in a fixed order: bitwise reproducible.
 //
-// What bounds it: latency and issue at one CTA (16 or 12 warps) an SM, not DRAM (SIMP 192x96x96: 110 MB in 48 us).
-// The modes of two planes, the sums and the epilogue operands take 110 (64-bit: 154) registers; any spill costs
+// What bounds it: latency and issue at one CTA (16 or 12 warps) an SM, not DRAM (SIMP 192x96x96: 111 MB in 43 us; warps
+// issue in 68 % of the cycles, the rest goes to the turn's barrier and to the latency of the staged planes).
+// The modes of two planes, the sums and the epilogue operands take 96-109 (64-bit: 143-156) registers; any spill costs
 // more than the warps it buys (64 registers and 32 warps: 117 us; 64-bit at 16 rows and 128 registers:
 // 92-110 us against 68 us). Two rows a thread in paired 32-bit instructions, which on this GPU run at half the rate of
 // single ones, measured 83 us, 8 rows at two CTAs an SM 64 us, 10 rows 56 us, two planes a turn without register
 // copies 64 us. Smoothing step, SIMP 192x96x96 / gyroid 256x256x128 / the same FP64 products: 97 / 254 / 184 / 522 us
-// for 32 x 8 x 4 tiles with the 27-point stencil and per-voxel gathers before, 48 / 207 / 68 / 285 us here.
+// for 32 x 8 x 4 tiles with the 27-point stencil and per-voxel gathers before, 43 / 190 / 63 / 252 us here (48 / 207 / 68 /
+// 285 us with turns that branch on their position and masks loaded where they are used).
 #pragma once
 
 #include "kernels.cuh"
@@ -41,15 +43,16 @@ namespace dev {
 
 constexpr int MARCH_NX = 30;  // output nodes of a tile along x
 template <class T> __host__ __device__ constexpr int marchRows() { return sizeof(T) == 4 ? 16 : 12; }  // node rows of a tile, a warp each
-template <class T> __host__ __device__ constexpr int marchNY() { return marchRows<T>() - 2; }           // output rows
+constexpr int MARCH_ROWS_TALL = 20;                                                                    // the same of a tall tile (32-bit only)
+constexpr double MARCH_TALL_STEP = 1.15;                                                               // a tall tile's time for a plane, of a low one's
 template <class T> __host__ __device__ constexpr int marchThreads() { return 32 * marchRows<T>(); }
 constexpr int MARCH_PREFETCH = 2, MARCH_STAGES = MARCH_PREFETCH + 2;  // planes of x in flight; ring slots (a power of two)
 constexpr int MARCH_ROW = 96;                                         // values of a staged row: 32 nodes
 constexpr int MARCH_BITS = 8;                                         // ring of output-node bits (a power of two > STAGES)
 // shared memory: the ring of x planes, the finished sums of two planes (a warp's own row and its share of the next
 // one), the output bits
-template <class T> __host__ __device__ constexpr size_t marchSmemBytes() {
-    return (sizeof(T) * MARCH_ROW * (MARCH_STAGES + 4) + 4 * MARCH_BITS) * marchRows<T>();
+template <class T> __host__ __device__ constexpr size_t marchSmemBytes(int rows = marchRows<T>()) {
+    return (sizeof(T) * MARCH_ROW * (MARCH_STAGES + 4) + 4 * MARCH_BITS) * rows;
 }
 
 // the level's element in the reflection basis (see above), made from Kb on the host (marchCoefs)
@@ -162,12 +165,12 @@ __device__ __forceinline__ void marchLayer(const ModeCoefs<T>& K, T s, const Fac
 // DENSE (TOP_DOT, 64-bit): the caller's vectors instead, in the reference's layout (rows of NX nodes): y is written at
 // every node of the grid (0 at held DOFs and inactive nodes; a tile of the list with MARCH_EMPTY set has only those),
 // x . y goes to io.dotOut, and the CTAs take the tiles in turn.
-template <class T, int MODE, bool DENSE = false>
-__global__ void __launch_bounds__(marchThreads<T>(), 1)
+template <class T, int MODE, bool DENSE = false, int ROWS = marchRows<T>()>
+__global__ void __launch_bounds__(32 * ROWS, 1)
     k_march(LevelView L, ModeCoefs<T> K, const MarchTile* __restrict__ tiles, const T* __restrict__ x, T* __restrict__ y,
             const float* __restrict__ r, float* __restrict__ d, MarchIO io, SolveState* st, double* partials, unsigned* ticket, Ctl ctl) {
     if (skipped(ctl)) return;
-    constexpr int ROWS = marchRows<T>(), PLANE = ROWS * MARCH_ROW;
+    constexpr int PLANE = ROWS * MARCH_ROW;
     constexpr bool CHEB = MODE == TOP_CHEB, RESID = MODE == TOP_RESID, DOT = MODE == TOP_DOT, APPLY = MODE == TOP_APPLY;
     constexpr bool MASKED = RESID || APPLY || DENSE;  // held DOFs of the result set to 0 by the masks
     extern __shared__ __align__(16) unsigned char marchSmem[];
@@ -182,7 +185,7 @@ __global__ void __launch_bounds__(marchThreads<T>(), 1)
         const MarchTile tile = tiles[tileAt];
         const int k0 = tile.k0, k1 = tile.k1;
         const int i = MARCH_NX * int(tile.tx & ~MARCH_EMPTY) - 1 + lane;      // the lane's node and voxel along x
-        const int j = marchNY<T>() * int(tile.ty) - 1 + warp;  // the warp's node row
+        const int j = (ROWS - 2) * int(tile.ty) - 1 + warp;  // the warp's node row
         const int XROW = DENSE ? L.NX : L.PX;  // the vectors' row pitch
         const long long PXY = (long long)L.PX * L.NY, XXY = (long long)XROW * L.NY, WXY = (long long)L.px * L.ny;  // mask, vector and word planes
         const bool nodeIn = i >= 0 && i < L.NX && j >= 0 && j < L.NY, nextIn = i >= 0 && i < L.NX && j + 1 >= 0 && j + 1 < L.NY;

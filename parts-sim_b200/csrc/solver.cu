@@ -1397,23 +1397,36 @@ dev::ModeCoefs<T> marchCoefs(const double Kb[576], bool& ok) {
     return {T(b0), T(a0), T(a1), T(b1), T(c2), T(e2), T(b3), T(a3)};
 }
 
-// The tiles of a marched level: columns of nx x ny nodes (`groups` CTAs each) cut into chunks of planes, trimmed to the planes with an
-// active node. A CTA of n planes takes about n + 4 steps (one plane of halo below and above, two to fill and
-// drain), so the chunk length is the one with the least waves x steps on `slots` resident CTAs: long chunks where
-// the level has many columns, short ones where it would leave SMs idle. whole: every column and plane, untrimmed, the
-// chunks without an active node marked.
-std::vector<dev::MarchTile> marchTiles(const HostLevel& h, int nx, int ny, int groups, int slots, bool whole = false) {
+// which planes of which columns of nx x ny nodes hold an active node: [k][ty][tx]
+std::vector<uint8_t> marchActivity(const HostLevel& h, int nx, int ny) {
     const int ntx = (h.NX + nx - 1) / nx, nty = (h.NY + ny - 1) / ny;
     const size_t cols = size_t(ntx) * nty;
-    std::vector<uint8_t> act(cols * h.NZ, 0);  // [k][ty][tx]
+    std::vector<uint8_t> act(cols * h.NZ, 0);
     parallelFor(h.NZ, [&](int64_t ka, int64_t kb) {
         for (int64_t k = ka; k < kb; k++)
             for (int j = 0; j < h.NY; j++) {
                 const uint8_t* row = h.nmask.data() + h.node(0, j, int(k));
                 uint8_t* a = act.data() + size_t(k) * cols + size_t(j / ny) * ntx;
-                for (int i = 0; i < h.NX; i++) a[i / nx] |= (row[i] & NM_ACTIVE) ? 1 : 0;
+                for (int t = 0; t < ntx; t++) {
+                    uint8_t any = 0;
+                    for (int i = t * nx, e = std::min(h.NX, i + nx); i < e; i++) any |= row[i];
+                    a[t] |= (any & NM_ACTIVE) ? 1 : 0;
+                }
             }
     }, 8);
+    return act;
+}
+
+// The tiles of a marched level: columns of nx x ny nodes (`groups` CTAs each) cut into chunks of planes, trimmed to the planes with an
+// active node. A CTA of n planes takes about n + 4 steps (one plane of halo below and above, two to fill and
+// drain), so the chunk length is the one with the least waves x steps on `slots` resident CTAs: long chunks where
+// the level has many columns, short ones where it would leave SMs idle. whole: every column and plane, untrimmed, the
+// chunks without an active node marked.
+// act: marchActivity's of the same nx x ny. steps: the waves x steps of the choice.
+std::vector<dev::MarchTile> marchTiles(const HostLevel& h, const std::vector<uint8_t>& act, int nx, int ny, int groups, int slots, bool whole = false,
+                                       int64_t* steps = nullptr) {
+    const int ntx = (h.NX + nx - 1) / nx;
+    const size_t cols = act.size() / size_t(h.NZ);
     size_t live = 0;
     for (size_t c = 0; c < cols; c++) {
         bool any = false;
@@ -1429,6 +1442,7 @@ std::vector<dev::MarchTile> marchTiles(const HostLevel& h, int nx, int ny, int g
             best = tz;
         }
     }
+    if (steps) *steps = bestCost;
     std::vector<dev::MarchTile> out;
     for (int kz = 0; kz < h.NZ; kz += best)
         for (size_t c = 0; c < cols; c++) {
@@ -1454,6 +1468,7 @@ struct DevLevel {
     DevMem word, nmask, own, own16, invD, dadd, dadd32, bc;
     DevMem tiles32, tiles64;  // marched levels: the 32- and 64-bit tiles with an active node
     int nTiles32 = 0, nTiles64 = 0;
+    bool tall32 = false;  // the 32-bit tiles are tall ones
     DevMem tilesAll;          // the finest level: 64-bit tiles over the whole grid (the allocation-free product)
     int nTilesAll = 0;
     int nActive = 0;   // active nodes
@@ -1582,7 +1597,7 @@ struct SharedModel {
     // or not) than the constant-operand gather
     bool blockStencil0 = false;
     int64_t stencilLevels = ~int64_t(1);  // PSFEA_STENCIL_LEVELS: bit l = level l (never level 0)
-    int64_t stencilMinNodes = 65536;      // PSFEA_STENCIL_MIN_NODES: smaller node lists keep the gather
+    int64_t stencilMinNodes = 65536;      // PSFEA_STENCIL_MIN_NODES: shorter node lists give eight lanes to a node
     bool foldBranch = true;               // PSFEA_FOLD_BRANCH: the FP32-Krylov fold as a conditional graph branch
     bool exactOneLevel() const { return L.size() == 1 && H.hasFactor(); }
 };
@@ -1631,6 +1646,10 @@ void SharedModel::adopt(Hierarchy&& h) {
         set(dev::k_march<float, dev::TOP_CHEB>, dev::marchSmemBytes<float>());
         set(dev::k_march<float, dev::TOP_RESID>, dev::marchSmemBytes<float>());
         set(dev::k_march<float, dev::TOP_DOT>, dev::marchSmemBytes<float>());
+        set(dev::k_march<float, dev::TOP_APPLY, false, dev::MARCH_ROWS_TALL>, dev::marchSmemBytes<float>(dev::MARCH_ROWS_TALL));
+        set(dev::k_march<float, dev::TOP_CHEB, false, dev::MARCH_ROWS_TALL>, dev::marchSmemBytes<float>(dev::MARCH_ROWS_TALL));
+        set(dev::k_march<float, dev::TOP_RESID, false, dev::MARCH_ROWS_TALL>, dev::marchSmemBytes<float>(dev::MARCH_ROWS_TALL));
+        set(dev::k_march<float, dev::TOP_DOT, false, dev::MARCH_ROWS_TALL>, dev::marchSmemBytes<float>(dev::MARCH_ROWS_TALL));
         set(dev::k_ebe<dev::TOP_APPLY, 1>, dev::ebeSmemBytes<1>());
         set(dev::k_ebe<dev::TOP_CHEB, 1>, dev::ebeSmemBytes<1>());
         set(dev::k_ebe<dev::TOP_RESID, 1>, dev::ebeSmemBytes<1>());
@@ -1810,8 +1829,10 @@ void SharedModel::uploadLevel(int l) {
         if (const char* e = std::getenv("PSFEA_TILE_MIN_NODES")) minNodes = std::atoll(e);
         D.m64 = marchCoefs<double>(h.Kb, D.useTiles);
         D.m32 = marchCoefs<float>(h.Kb, D.useTiles);
+        std::vector<uint8_t> act64;
+        if (D.useTiles && (l == 0 || h.nNodes >= minNodes)) act64 = marchActivity(h, dev::MARCH_NX, dev::marchRows<double>() - 2);
         if (l == 0 && D.useTiles) {
-            const std::vector<dev::MarchTile> ta = marchTiles(h, dev::MARCH_NX, dev::marchNY<double>(), 1, smCount, true);
+            const std::vector<dev::MarchTile> ta = marchTiles(h, act64, dev::MARCH_NX, dev::marchRows<double>() - 2, 1, smCount, true);
             D.nTilesAll = int(ta.size());
             upload(D.tilesAll, ta, bytes, ms);
         }
@@ -1820,17 +1841,31 @@ void SharedModel::uploadLevel(int l) {
         if (const char* e = std::getenv("PSFEA_OP8_MAX_NODES")) max8 = std::atoll(e);
         D.use8 = !D.useTiles && l > 0 && h.nNodes <= max8;
         if (D.useTiles) {
-            const std::vector<dev::MarchTile> t32 = marchTiles(h, dev::MARCH_NX, dev::marchNY<float>(), 1, smCount), t64 = marchTiles(h, dev::MARCH_NX, dev::marchNY<double>(), 1, smCount);
+            // 32-bit: tiles of 14 or of 18 output rows, whichever is estimated the faster (waves x planes of the longest tile). The
+            // halo of a tall one is a smaller share, but its planes take 1.1-1.2 times as long, so that it pays where there are several waves:
+            // smoothing step at 14 / 18 rows, gyroid 256x256x128 190 / 169 us, 384x384x192 563 / 508, against SIMP 192x96x96
+            // (one wave) 43.1 / 47.3, SIMP 96x48x48 12.4 / 13.3, cantilever 64x16x16 7.5 / 8.3
+            int64_t costLow = 0, costTall = 0;
+            std::vector<dev::MarchTile> t32 = marchTiles(h, marchActivity(h, dev::MARCH_NX, dev::marchRows<float>() - 2), dev::MARCH_NX, dev::marchRows<float>() - 2, 1, smCount, false, &costLow);
+            std::vector<dev::MarchTile> tall = marchTiles(h, marchActivity(h, dev::MARCH_NX, dev::MARCH_ROWS_TALL - 2), dev::MARCH_NX, dev::MARCH_ROWS_TALL - 2, 1, smCount, false, &costTall);
+            D.tall32 = dev::MARCH_TALL_STEP * double(costTall) < double(costLow);
+            if (const char* e = std::getenv("PSFEA_MARCH_TALL")) D.tall32 = std::atoi(e) != 0;
+            if (D.tall32) t32.swap(tall);
+            const std::vector<dev::MarchTile> t64 = marchTiles(h, act64, dev::MARCH_NX, dev::marchRows<double>() - 2, 1, smCount);
             D.nTiles32 = int(t32.size());
             D.nTiles64 = int(t64.size());
             upload(D.tiles32, t32, bytes, ms);
             upload(D.tiles64, t64, bytes, ms);
             std::vector<int32_t> bl(h.boundary.size()), ol;
-            for (size_t q = 0; q < bl.size(); q++) {
-                const int64_t nd = h.boundary[q], row = nd / h.NX;
-                bl[q] = int32_t((nd - row * h.NX) + int64_t(PX) * row);
-                if (!(h.nmask[size_t(nd)] & NM_PLAIN)) ol.push_back(bl[q]);
-            }
+            parallelFor(int64_t(bl.size()), [&](int64_t lo, int64_t hi) {
+                for (int64_t q = lo; q < hi; q++) {
+                    const int64_t nd = h.boundary[size_t(q)], row = nd / h.NX;
+                    bl[size_t(q)] = int32_t((nd - row * h.NX) + int64_t(PX) * row);
+                }
+            });
+            if (ownNodes > 0)
+                for (size_t q = 0; q < bl.size(); q++)
+                    if (!(h.nmask[size_t(h.boundary[q])] & NM_PLAIN)) ol.push_back(bl[q]);
             D.nBnd = int(bl.size());
             D.nOwnNodes = int(ol.size());
             upload(D.blist, bl, bytes, ms);
@@ -2313,7 +2348,8 @@ void SolverImpl::op32(int l, const float* xin, float* y, float c1, float c2, dev
     // marched: the nodes of one scale per voxel; then the list kernels' nodes (those that touch an own matrix)
     const int* bl = D.list(D.split32);
     const int nl = D.listCount(D.split32);
-    launch(dev::k_march<float, SM_>, D.nTiles32, dev::marchThreads<float>(), dev::marchSmemBytes<float>(), stream, D.view, D.m32,
+    const int rows = D.tall32 ? dev::MARCH_ROWS_TALL : dev::marchRows<float>();
+    launch(D.tall32 ? dev::k_march<float, SM_, false, dev::MARCH_ROWS_TALL> : dev::k_march<float, SM_>, D.nTiles32, 32 * rows, dev::marchSmemBytes<float>(rows), stream, D.view, D.m32,
            D.tiles32.as<dev::MarchTile>(), xin, y, rr, dd, dev::MarchIO{c1, c2, 0, 0, D.outBit(D.split32), 0, nullptr}, st(), part(), tick(), ctl);
     if (!nl) return;
     if (stn) {
@@ -2669,7 +2705,8 @@ void SolverImpl::recordMixedIteration(dev::Ctl ctl, bool refine, bool half) {
         launch(dev::k_apply_alpha<float, true>, nodeGrid(pn(0)), dev::NODE_THREADS, 0, stream, D.view, D.c32, p32.as<float>(), q32.as<float>(),
                st(), part(), tick(), dev::Ctl{ctl.skipIf, nullptr});
     } else {
-        launch(dev::k_march<float, dev::TOP_DOT>, D.nTiles32, dev::marchThreads<float>(), dev::marchSmemBytes<float>(), stream, D.view, D.m32,
+        const int rows = D.tall32 ? dev::MARCH_ROWS_TALL : dev::marchRows<float>();
+        launch(D.tall32 ? dev::k_march<float, dev::TOP_DOT, false, dev::MARCH_ROWS_TALL> : dev::k_march<float, dev::TOP_DOT>, D.nTiles32, 32 * rows, dev::marchSmemBytes<float>(rows), stream, D.view, D.m32,
                D.tiles32.as<dev::MarchTile>(), p32.as<float>(), q32.as<float>(), nullptr, nullptr, dev::MarchIO{0.f, 0.f, 0, 0, NM_PLAIN, 0, nullptr}, st(), part(),
                tick(), dev::Ctl{ctl.skipIf, nullptr});
     }
@@ -3040,8 +3077,8 @@ struct BlockImpl final : BlockBase {
         for (DevMem* b : {&f, &x, &r, &p, &q}) b->alloc(n, bytes, stream);
         if (M->exactOneLevel()) z64.alloc(n, bytes, stream);
         state.alloc(sizeof(dev::BlockState), bytes, stream);
-        const auto t32 = marchTiles(H.levels[0], dev::BM_NX, dev::bmNY<float>(), RB / dev::BM_G, smCount);
-        const auto t64 = marchTiles(H.levels[0], dev::BM_NX, dev::bmNY<double>(), RB / dev::BM_G, smCount);
+        const auto t32 = marchTiles(H.levels[0], marchActivity(H.levels[0], dev::BM_NX, dev::bmNY<float>()), dev::BM_NX, dev::bmNY<float>(), RB / dev::BM_G, smCount);
+        const auto t64 = marchTiles(H.levels[0], marchActivity(H.levels[0], dev::BM_NX, dev::bmNY<double>()), dev::BM_NX, dev::bmNY<double>(), RB / dev::BM_G, smCount);
         nTiles32 = int(t32.size());
         nTiles64 = int(t64.size());
         upload(tiles32, t32, bytes, stream);

@@ -155,3 +155,23 @@ def test_small_levels_stencils_match_the_gather(monkeypatch, dims, shift):
             b = B.solve(f, tol=1e-9, max_iter=3000, precision=prec, smoother_degree=deg)
             assert a.converged and b.converged and rel(b.u, a.u) < 1e-5, (prec, deg)
     assert rel(B.precondition(f), A.precondition(f)) < 1e-5
+
+
+@pytest.mark.parametrize("dims", [(29, 17, 13), (30, 18, 9), (61, 35, 8), (31, 36, 20)])
+def test_tall_tiles_match_the_low_ones(monkeypatch, dims):
+    """32-bit tiles of 18 output rows against those of 14, at node rows of one tile, one more, two tiles and one more: the
+    same sums per node (1e-5 for a V-cycle as above), and solves that agree to their tolerance."""
+    d, bc = blocky(dims, 5)
+    monkeypatch.setenv("PSFEA_TILE_MIN_NODES", "0")
+    monkeypatch.setenv("PSFEA_MARCH_TALL", "0")
+    A = psfea.VoxelFEA(dims, d, 0.3, bc, 300)
+    monkeypatch.setenv("PSFEA_MARCH_TALL", "1")
+    B = psfea.VoxelFEA(dims, d, 0.3, bc, 300)
+    r = np.random.default_rng(9).standard_normal(A.n_dof) * (A.fixed(0) == 0)
+    assert rel(B.precondition(r), A.precondition(r)) < 1e-5
+    f = W._face_load(dims, d, 0, 1, (1.0, -2.0, 0.5))[0]
+    for prec in ("half", "mixed", "fp32"):
+        a = A.solve(f, tol=1e-9, max_iter=3000, precision=prec)
+        b = B.solve(f, tol=1e-9, max_iter=3000, precision=prec)
+        assert a.converged and b.converged, prec
+        assert rel(b.u, a.u) < 1e-5, (prec, rel(b.u, a.u))
