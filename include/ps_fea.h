@@ -182,8 +182,8 @@ ps_status ps_fea_apply_dot_noalloc(ps_fea_t* h, const double* x_dev, double* y_d
  * voxel_fea.cpp:692-725, and the coarsest size, voxel_fea.cpp:174-180) */
 typedef struct ps_tune_result {
     int32_t smoother_degree;   /* chosen Chebyshev degree per V-cycle half (1-4) */
-    int32_t inner64;           /* the finest level's FP64 tiles compute their boundary nodes in the tile */
-    int64_t split_levels;      /* bit l: level l's FP32 tiles leave boundary nodes to the list kernel */
+    int32_t inner64;           /* the finest level's FP64 march computes its boundary nodes itself */
+    int64_t split_levels;      /* bit l: level l's FP32 march leaves boundary nodes to the list kernel */
     int64_t coarsest_max_dof;  /* ps_fea_create_tuned: the chosen coarsening depth (else 0) */
     int32_t trials;            /* solves timed (0: taken from the process's cache of tuned models) */
     int32_t cached;
@@ -194,7 +194,7 @@ typedef struct ps_tune_result {
 #define PS_TUNE_FORCE 1        /* ignore the cache of tuned models */
 
 /* Times complete solves of f (host, nDof values) to opts->tol over smoother degrees 1-4 and the
- * tile-path choices of the tiled levels, keeps the fastest configuration on the handle (solves whose
+ * boundary-node choices of the marched levels, keeps the fastest configuration on the handle (solves whose
  * smoother_degree is 0 use the tuned degree) and caches it for models with the same voxel words,
  * masks and depth. opts->precision and max_iter apply to the trials. */
 ps_status ps_fea_autotune(ps_fea_t* h, const double* f, const ps_solve_opts* opts, int32_t flags, ps_tune_result* out);

@@ -10,7 +10,7 @@
 // product is the three-term split hi*hi + hi*lo + lo*hi (hi = the TF32 truncation, lo = the rest),
 // close to FP32 accuracy. The rows come back with tcgen05.ld, scaled by s_v, into shared memory,
 // and every owned node sums its up-to-8 voxel rows in a fixed order (deterministic), then runs the
-// tile kernel's epilogue (APPLY / CHEB / RESID).
+// marched kernel's epilogue (APPLY / CHEB / RESID).
 //
 // Shared-memory operands use the canonical K-major layout without swizzle: element (row, k) of an
 // R-row operand at byte (k / 8) (R / 8) 256 + ((k % 8) / 4) 128 + (row / 8) 256 + (row % 8) 16 +

@@ -16,8 +16,8 @@ struct BlockBase;
 // the configuration an autotune run chose for a model (and what it measured)
 struct TuneResult {
     int degree = 2;           // Chebyshev smoother degree per V-cycle half
-    int64_t splitLevels = 0;  // bit l: level l's 32-bit tiles leave boundary nodes to the list kernel
-    int inner64 = 0;          // the finest level's 64-bit tiles compute boundary nodes in the tile
+    int64_t splitLevels = 0;  // bit l: level l's 32-bit march leaves boundary nodes to the list kernel
+    int inner64 = 0;          // the finest level's 64-bit march computes boundary nodes itself
     int trials = 0;           // solves timed (0: taken from the cache)
     double bestSeconds = 0;   // the chosen configuration's solve time
     double defaultSeconds = 0;  // the configuration before tuning
@@ -63,8 +63,8 @@ public:
     // Chebyshev step of the V-cycle, 1 = the FP64 product of the CG
     double timeKernel(int which, int reps);
     int64_t launches() const;
-    // times solves of f (host) to o.tol over smoother degrees 1-4 and the tile-path choices of the
-    // tiled levels (coordinate descent: degree first, then each tile flag), keeps the fastest
+    // times solves of f (host) to o.tol over smoother degrees 1-4 and the boundary-node choices of the
+    // marched levels (coordinate descent: degree first, then each flag), keeps the fastest
     // configuration on this handle (solves that leave the degree open use it) and caches it by the
     // model's signature; force: ignore the cache
     TuneResult autotune(const double* f, const ps_solve_opts& o, bool force);

@@ -364,7 +364,7 @@ class VoxelFEA:
         return z
 
     def autotune(self, f, tol=1e-8, max_iter=5000, precision="fp64", force=False):
-        """Times solves of f over smoother degrees and tile paths, keeps the fastest on this handle
+        """Times solves of f over smoother degrees and boundary-node paths, keeps the fastest on this handle
         (see ps_fea_autotune); returns the choice as a dict."""
         f = self._check_vec(f, "f")
         o = make_opts(tol, max_iter, precision)
