@@ -16,24 +16,24 @@
 // as 4 x one corner + differences), so the rounding error scales with the field's local variation and a
 // rigid translation gives exact zeros: what keeps the FP32 CG accurate on smooth search directions.
 //
-// One CTA computes a tile of 30 x 14 nodes (64-bit: 30 x 10) over a range of z planes. Lane l of a warp holds the
+// One CTA computes a tile of 30 x 14 nodes (30 x 18 where a level has several waves of them; 64-bit: 30 x 10) over a range of z planes. Lane l of a warp holds the
 // nodes i = 30 tx - 1 + l and the voxels right of them (lanes 0 and 31 are halo), warp w the node row
-// j = 14 ty - 1 + w and the voxels above it (the first and last warp are halo). Planes of x are staged into a ring
+// j = (ROWS - 2) ty - 1 + w and the voxels above it (the first and last warp are halo). Planes of x are staged into a ring
 // in shared memory by asynchronous copies of one value each (zeros at inactive nodes, which are not read), two planes
 // ahead; a plane's in-plane modes stay in registers until the next plane has come. Finished sums go to shared
 // memory once (node order in, DOF order out), from where the epilogue runs in DOF order: r, d, 1/diag and the results
 // move in fully coalesced accesses, at output nodes only, so that the empty space of a lattice costs no memory
 // traffic beyond whole 32-byte sectors. Sums run in a fixed order: bitwise reproducible.
 //
-// What bounds it: latency and issue at one CTA (16 or 12 warps) an SM, not DRAM (SIMP 192x96x96: 111 MB in 43 us; warps
+// What bounds it: latency and issue at one CTA (16, 20 or 12 warps) an SM, not DRAM (SIMP 192x96x96: 111 MB in 43 us; warps
 // issue in 68 % of the cycles, the rest goes to the turn's barrier and to the latency of the staged planes).
 // The modes of two planes, the sums and the epilogue operands take 96-109 (64-bit: 143-156) registers; any spill costs
 // more than the warps it buys (64 registers and 32 warps: 117 us; 64-bit at 16 rows and 128 registers:
 // 92-110 us against 68 us). Two rows a thread in paired 32-bit instructions, which on this GPU run at half the rate of
 // single ones, measured 83 us, 8 rows at two CTAs an SM 64 us, 10 rows 56 us, two planes a turn without register
 // copies 64 us. Smoothing step, SIMP 192x96x96 / gyroid 256x256x128 / the same FP64 products: 97 / 254 / 184 / 522 us
-// for 32 x 8 x 4 tiles with the 27-point stencil and per-voxel gathers before, 43 / 190 / 63 / 252 us here (48 / 207 / 68 /
-// 285 us with turns that branch on their position and masks loaded where they are used).
+// for 32 x 8 x 4 tiles with the 27-point stencil and per-voxel gathers before, 43 / 170 / 63 / 252 us here (43 / 190 with 14 output
+// rows on both grids; 48 / 207 / 68 / 285 us with turns that branch on their position and masks loaded where they are used).
 #pragma once
 
 #include "kernels.cuh"
