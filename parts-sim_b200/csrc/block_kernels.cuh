@@ -690,10 +690,11 @@ __global__ void kb_final(const int* __restrict__ act, int nAct, const uint8_t* _
     }
 }
 
-// max |r_free| per right-hand side into rmax / scale (the block preconditioner's entry)
+// max |r_free| per right-hand side into rmax / scale (the block preconditioner's entry). nvec comes as an argument: the call returns
+// before the GPU has run it, so a state copied from a host buffer could be the next call's.
 template <int RB>
-__global__ void kb_rmax(const int* __restrict__ act, int nAct, const uint8_t* __restrict__ nmask, const double* __restrict__ r, BlockState* bs,
-                        double* partials, unsigned* ticket) {
+__global__ void kb_rmax(const int* __restrict__ act, int nAct, const uint8_t* __restrict__ nmask, const double* __restrict__ r, int nvec,
+                        BlockState* bs, double* partials, unsigned* ticket) {
     constexpr int NPW = 32 / RB;
     const int lane = threadIdx.x & 31, q = lane % RB, sub = lane / RB;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -711,8 +712,9 @@ __global__ void kb_rmax(const int* __restrict__ act, int nAct, const uint8_t* __
         if (qq < RB) {
             bs->rmax[qq] = tot[0];
             bs->scale[qq] = tot[0] > 0 ? 1.0 / tot[0] : 1.0;
-            bs->done[qq] = (qq < bs->nrhs && tot[0] > 0) ? 0 : 1;  // a zero vector gives z = 0
+            bs->done[qq] = (qq < nvec && tot[0] > 0) ? 0 : 1;  // a zero vector gives z = 0
         }
+        if (qq == 0) bs->nrhs = nvec;
     }
 }
 

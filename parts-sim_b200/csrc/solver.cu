@@ -3402,12 +3402,9 @@ struct BlockImpl final : BlockBase {
             check(cudaEventRecord(ev, caller), "event");
             check(cudaStreamWaitEvent(stream, ev, 0), "wait");
         }
-        dev::BlockState s{};
-        s.nrhs = nvec;
-        *hostState = s;
-        check(cudaMemcpyAsync(state.p, hostState, sizeof s, cudaMemcpyHostToDevice, stream), "state");
         pack(rDev, nvec, r.template as<double>(), true);
-        launch(dev::kb_rmax<RB>, laneGrid(0), dev::BLOCK_THREADS, 0, act(0), nAct(0), D.view.nmask, r.template as<double>(), bs(), part(), tick());
+        launch(dev::kb_rmax<RB>, laneGrid(0), dev::BLOCK_THREADS, 0, act(0), nAct(0), D.view.nmask, r.template as<double>(), nvec, bs(), part(),
+               tick());
         if (z64.p) check(cudaMemsetAsync(z64.p, 0, z64.bytes, stream), "memset");
         if (M->exactOneLevel()) {
             // the whole model is the coarsest level: its direct FP64 solve (voxel_fea.cpp:838-842)
