@@ -120,7 +120,7 @@ enum { BOP_APPLY = 0, BOP_CHEB = 1, BOP_RESID = 2, BOP_DOT = 3 };
 // gather. Neighbours outside the grid read 0; they only ever meet empty voxels.
 // V: the storage type of x (T, or __half for the FP16 coarse-level vectors; converted on load).
 template <class T, bool OWN16, int S, bool SMEM = false, class V = T>
-__device__ __forceinline__ void applyNbr(const LevelView& L, const Coefs<T>& C, const V* __restrict__ x, int i, int j, int k, long long n,
+__device__ __forceinline__ void applyNbr(const LevelView& L, const Coefs<T>& C, const V* x, int i, int j, int k, long long n,
                                          uint8_t mask, T acc[3]) {
     acc[0] = acc[1] = acc[2] = T(0);
     if (!(mask & NM_ACTIVE)) return;

@@ -68,8 +68,8 @@ __device__ __forceinline__ float tf32Hi(float v) { return __uint_as_float(__floa
 
 template <int MODE, int SPLIT>
 __global__ void __launch_bounds__(EBE_THREADS, SPLIT == 3 ? 1 : 3)
-    k_ebe(LevelView L, Coefs<float> C, const uint32_t* __restrict__ tiles, const float* __restrict__ x, float* __restrict__ y,
-          const float* __restrict__ r, float* __restrict__ d, float c1, float c2, int raw, SolveState* st, Ctl ctl) {
+    k_ebe(LevelView L, Coefs<float> C, const uint32_t* __restrict__ tiles, const float* x, float* __restrict__ y,
+          const float* r, float* __restrict__ d, float c1, float c2, int raw, SolveState* st, Ctl ctl) {
     if (skipped(ctl)) return;
     extern __shared__ __align__(1024) unsigned char ebeRaw[];
     unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ebeRaw) + 1023) & ~uintptr_t(1023));
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(EBE_THREADS, SPLIT == 3 ? 1 : 3)
         const int hy = row % EHY, hz = row / EHY;
         const int gi = i0 - 1 + hx, gj = j0 - 1 + hy, gk = k0 - 1 + hz;
         float v = 0.f;
-        if (gi >= 0 && gj >= 0 && gk >= 0 && gi < L.NX && gj < L.NY && gk < L.NZ) v = __ldg(x + 3 * (gi + (long long)L.PX * (gj + (long long)L.NY * gk)) + c);
+        if (gi >= 0 && gj >= 0 && gk >= 0 && gi < L.NX && gj < L.NY && gk < L.NZ) v = x[3 * (gi + (long long)L.PX * (gj + (long long)L.NY * gk)) + c];
         xs[e] = v;
     }
     for (int e = tid; e < EBE_VOX; e += EBE_THREADS) {

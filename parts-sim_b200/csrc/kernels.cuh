@@ -114,16 +114,16 @@ __device__ __forceinline__ void own16Rows(const __half* M, const T xe[24], T t[3
 // vector; the block width for the RHS-minor layout of a multi-RHS block, x then pointing at the
 // lane's right-hand side). SMEM: L.own / L.own16 point at a copy in shared memory.
 template <class T, bool OWN16, bool DIFF = false, int S = 1, bool SMEM = false>
-__device__ __forceinline__ void applyAt(const LevelView& L, const Coefs<T>& C, const T* __restrict__ x, int i, int j, int k,
+__device__ __forceinline__ void applyAt(const LevelView& L, const Coefs<T>& C, const T* x, int i, int j, int k,
                                         long long n, uint8_t mask, T acc[3], long long XP, long long nm) {
     acc[0] = acc[1] = acc[2] = T(0);
     if (!(mask & NM_ACTIVE)) return;
     const long long NX = XP, NXY = XP * L.NY;
     T own0 = 0, own1 = 0, own2 = 0;
     if (DIFF) {
-        own0 = __ldg(x + 3 * S * n);
-        own1 = __ldg(x + 3 * S * n + S);
-        own2 = __ldg(x + 3 * S * n + 2 * S);
+        own0 = x[3 * S * n];
+        own1 = x[3 * S * n + S];
+        own2 = x[3 * S * n + 2 * S];
     }
     if (mask & NM_UNIFORM) {
         const float s = __uint_as_float(__ldg(L.word + L.wi(i - 1, j - 1, k - 1)));
@@ -133,7 +133,7 @@ __device__ __forceinline__ void applyAt(const LevelView& L, const Coefs<T>& C, c
             const int ox = m % 3 - 1, oy = (m / 3) % 3 - 1, oz = m / 9 - 1;
             if (DIFF && m == 13) continue;  // the node itself: a zero difference
             const T* xp = x + 3 * S * (n + ox + oy * NX + oz * NXY);
-            const T x0 = __ldg(xp) - own0, x1 = __ldg(xp + S) - own1, x2 = __ldg(xp + 2 * S) - own2;
+            const T x0 = xp[0] - own0, x1 = xp[S] - own1, x2 = xp[2 * S] - own2;
             a0 += C.S[m * 9 + 0] * x0;
             a1 += C.S[m * 9 + 4] * x1;
             a2 += C.S[m * 9 + 8] * x2;
@@ -159,9 +159,9 @@ __device__ __forceinline__ void applyAt(const LevelView& L, const Coefs<T>& C, c
             for (int b = 0; b < 8; b++) {
                 const int bx = (b == 1 || b == 2 || b == 5 || b == 6), by = (b == 2 || b == 3 || b == 6 || b == 7), bz = b >> 2;
                 const T* xp = x + 3 * S * (n + (di + bx - 1) + (dj + by - 1) * NX + (dk + bz - 1) * NXY);
-                xe[3 * b] = __ldg(xp) - own0;
-                xe[3 * b + 1] = __ldg(xp + S) - own1;
-                xe[3 * b + 2] = __ldg(xp + 2 * S) - own2;
+                xe[3 * b] = xp[0] - own0;
+                xe[3 * b + 1] = xp[S] - own1;
+                xe[3 * b + 2] = xp[2 * S] - own2;
             }
             if (!(w & OWN_BIT)) {
                 T t[3];
@@ -194,17 +194,18 @@ __device__ __forceinline__ void applyAt(const LevelView& L, const Coefs<T>& C, c
     }
 }
 
-// a read-only vector entry as T: FP32 / FP64 storage as is, FP16 storage converted
+// An entry of a solve's vector as T: FP32 / FP64 storage as is, FP16 storage converted. Plain loads, and no const __restrict__ on the
+// vectors the kernels of an iteration read: the read-only path (__ldg, and what the compiler makes of const
+// __restrict__) asks for data that nothing writes while the kernel is resident, and a programmatically launched kernel is
+// resident while the one before it still writes them. Masks, words, lists, matrices, stencils and 1/diag keep that path.
 template <class T>
-__device__ __forceinline__ T ldv(const float* p) { return T(__ldg(p)); }
+__device__ __forceinline__ T ldv(const float* p) { return T(*p); }
 template <class T>
-__device__ __forceinline__ T ldv(const double* p) { return T(__ldg(p)); }
+__device__ __forceinline__ T ldv(const double* p) { return T(*p); }
 template <class T>
-__device__ __forceinline__ T ldv(const __half* p) { return T(__half2float(__ldg(p))); }
+__device__ __forceinline__ T ldv(const __half* p) { return T(__half2float(*p)); }
 __device__ __forceinline__ void stv(float* p, float v) { *p = v; }
 __device__ __forceinline__ void stv(__half* p, float v) { *p = __float2half_rn(v); }
-__device__ __forceinline__ float ldf(const float* p) { return *p; }
-__device__ __forceinline__ float ldf(const __half* p) { return __half2float(*p); }
 
 // Layout: coefficient c = 9 m + 3 p + q (m the neighbour (ox + 1) + 3 (oy + 1) + 9 (oz + 1), p the
 // row and q the column component) of listed node t sits in chunk c / CW of CW consecutive values

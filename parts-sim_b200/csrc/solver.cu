@@ -120,8 +120,8 @@ enum { OP_APPLY = 0, OP_CHEB = 1, OP_RESID = 2 };
 //   OP_CHEB   d = c1 d + c2 D^-1 (r - K x); y = x + d      (Chebyshev / Jacobi step, 32-bit)
 //   OP_RESID  y = r - K x
 template <class T, int MODE, bool OWN16, bool DIFF = false>
-__global__ void __launch_bounds__(NODE_THREADS) k_op(LevelView L, Coefs<T> C, const T* __restrict__ x, T* __restrict__ y,
-                                                      const float* __restrict__ r, float* __restrict__ d, float c1, float c2, int raw,
+__global__ void __launch_bounds__(NODE_THREADS) k_op(LevelView L, Coefs<T> C, const T* x, T* __restrict__ y,
+                                                      const float* r, float* __restrict__ d, float c1, float c2, int raw,
                                                       Ctl ctl) {
     if (skipped(ctl)) return;
     for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < L.nNodes; n += (long long)gridDim.x * blockDim.x) {
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(NODE_THREADS) k_op(LevelView L, Coefs<T> C, co
 // q = K p on the finest level with the CG step length: alpha = rz / (p . q) (FP64 accumulation);
 // p.q <= 0 ends the solve as a breakdown (voxel_fea.cpp:902-905)
 template <class T, bool OWN16>
-__global__ void __launch_bounds__(NODE_THREADS) k_apply_alpha(LevelView L, Coefs<T> C, const T* __restrict__ p, T* __restrict__ q,
+__global__ void __launch_bounds__(NODE_THREADS) k_apply_alpha(LevelView L, Coefs<T> C, const T* p, T* __restrict__ q,
                                                               SolveState* st, double* partials, unsigned* ticket, Ctl ctl) {
     if (skipped(ctl)) return;
     double v[1] = {0.0};
@@ -194,8 +194,8 @@ __global__ void __launch_bounds__(NODE_THREADS) k_apply_alpha(LevelView L, Coefs
 // by shuffles. Coarse levels have few nodes and many own matrices; spreading a node over eight
 // lanes turns one thread's chain of eight dependent matrix reads into eight parallel ones.
 template <class T, int MODE, bool OWN16, bool DIFF>
-__global__ void __launch_bounds__(256) k_op8(LevelView L, Coefs<T> C, const T* __restrict__ x, T* __restrict__ y,
-                                             const float* __restrict__ r, float* __restrict__ d, float c1, float c2, int raw, Ctl ctl) {
+__global__ void __launch_bounds__(256) k_op8(LevelView L, Coefs<T> C, const T* x, T* __restrict__ y,
+                                             const float* r, float* __restrict__ d, float c1, float c2, int raw, Ctl ctl) {
     if (skipped(ctl)) return;
     __shared__ T kb[576];
     for (int e = threadIdx.x; e < 576; e += blockDim.x) kb[e] = C.Kb[e];
@@ -219,18 +219,18 @@ __global__ void __launch_bounds__(256) k_op8(LevelView L, Coefs<T> C, const T* _
             if (w) {
                 T own[3] = {T(0), T(0), T(0)};
                 if (DIFF) {
-                    own[0] = __ldg(x + 3 * n);
-                    own[1] = __ldg(x + 3 * n + 1);
-                    own[2] = __ldg(x + 3 * n + 2);
+                    own[0] = x[3 * n];
+                    own[1] = x[3 * n + 1];
+                    own[2] = x[3 * n + 2];
                 }
                 T xe[24];
 #pragma unroll
                 for (int b = 0; b < 8; b++) {
                     const int bx = (b == 1 || b == 2 || b == 5 || b == 6), by = (b == 2 || b == 3 || b == 6 || b == 7), bz = b >> 2;
                     const T* xp = x + 3 * (n + (di + bx - 1) + (dj + by - 1) * NX + (dk + bz - 1) * NXY);
-                    xe[3 * b] = __ldg(xp) - own[0];
-                    xe[3 * b + 1] = __ldg(xp + 1) - own[1];
-                    xe[3 * b + 2] = __ldg(xp + 2) - own[2];
+                    xe[3 * b] = xp[0] - own[0];
+                    xe[3 * b + 1] = xp[1] - own[1];
+                    xe[3 * b + 2] = xp[2] - own[2];
                 }
                 if (!(w & OWN_BIT)) {
                     const T* k0 = kb + (3 * a) * 24;
@@ -301,8 +301,8 @@ __global__ void __launch_bounds__(256) k_op8(LevelView L, Coefs<T> C, const T* _
 // epilogues (TOP_*); runs after the marching kernel, which leaves these nodes out, on the same vectors.
 // TOP_DOT adds its p.q share to the marched one (fixed order) and takes the CG step.
 template <class T, int MODE, bool OWN16, bool DIFF>
-__global__ void __launch_bounds__(NODE_THREADS) k_bnd(LevelView L, Coefs<T> C, const int* __restrict__ list, int count, const T* __restrict__ x,
-                                                      T* __restrict__ y, const float* __restrict__ r, float* __restrict__ d, float c1, float c2,
+__global__ void __launch_bounds__(NODE_THREADS) k_bnd(LevelView L, Coefs<T> C, const int* __restrict__ list, int count, const T* x,
+                                                      T* __restrict__ y, const float* r, float* __restrict__ d, float c1, float c2,
                                                       int raw, SolveState* st, double* partials, unsigned* ticket, Ctl ctl) {
     if (skipped(ctl)) return;
     double v[1] = {0.0};
@@ -358,11 +358,11 @@ __global__ void __launch_bounds__(NODE_THREADS) k_bnd(LevelView L, Coefs<T> C, c
 // z = d = c0 D^-1 r (the first Chebyshev step from zero); V = __half: the FP16 coarse-level
 // vectors, c0 carrying the level's iterate-to-residual scale
 template <class V = float>
-__global__ void k_cheb_first(long long nDof, const V* __restrict__ r, const float* __restrict__ invD, V* __restrict__ d, V* __restrict__ z,
+__global__ void k_cheb_first(long long nDof, const V* r, const float* __restrict__ invD, V* __restrict__ d, V* __restrict__ z,
                              float c0, Ctl ctl) {
     if (skipped(ctl)) return;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nDof; i += (long long)gridDim.x * blockDim.x) {
-        const float v = c0 * invD[i] * ldf(r + i);
+        const float v = c0 * invD[i] * ldv<float>(r + i);
         stv(d + i, v);
         stv(z + i, v);
     }
@@ -377,7 +377,7 @@ template <int N> struct Values {
     __device__ __forceinline__ float& operator[](int c) { return v[c]; }
 };
 template <int S, int COMPS, class VF>
-__device__ __forceinline__ Values<COMPS> restrictAt(const LevelView& F, const VF* __restrict__ rf, int I, int J, int K) {
+__device__ __forceinline__ Values<COMPS> restrictAt(const LevelView& F, const VF* rf, int I, int J, int K) {
     Values<COMPS> s{};
     const long long FPX = F.PX, FPXY = (long long)F.PX * F.NY;
 #pragma unroll
@@ -407,7 +407,7 @@ __device__ __forceinline__ Values<COMPS> restrictAt(const LevelView& F, const VF
 // One thread a coarse DOF: its 27 loads fit in registers at once (81 of a whole node did not: 5.1 us on a level of some
 // hundred nodes).
 template <class VF = float, class VC = float>
-__global__ void k_restrict(LevelView F, LevelView C, const VF* __restrict__ rf, VC* __restrict__ rc, VC* __restrict__ dc,
+__global__ void k_restrict(LevelView F, LevelView C, const VF* rf, VC* __restrict__ rc, VC* __restrict__ dc,
                            VC* __restrict__ zc, float c0, float sr, Ctl ctl) {
     const long long e0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     auto nodeOf = [](long long e) { return e <= 0xffffffffLL ? (long long)(unsigned(e) / 3u) : e / 3; };
@@ -440,7 +440,7 @@ __global__ void k_restrict(LevelView F, LevelView C, const VF* __restrict__ rf, 
 // Trilinear value at fine node (i, j, k) of a coarse vector (coarse i/2 and, when odd, (i + 1)/2, weight 1/2 each); the up to
 // eight corners without branches as in restrictAt (an even axis reads its one node twice, the second time with weight 0)
 template <int S, class VC>
-__device__ __forceinline__ void prolongAt(long long CNX, long long CNXY, const VC* __restrict__ zc, int i, int j, int k, float s[3]) {
+__device__ __forceinline__ void prolongAt(long long CNX, long long CNXY, const VC* zc, int i, int j, int k, float s[3]) {
     const int oi = i & 1, oj = j & 1, ok = k & 1;
     const float w = (oi ? 0.5f : 1.f) * (oj ? 0.5f : 1.f) * (ok ? 0.5f : 1.f);
     const VC* p0 = zc + 3 * S * ((i >> 1) + (j >> 1) * CNX + (k >> 1) * CNXY);
@@ -463,7 +463,7 @@ __device__ __forceinline__ void prolongAt(long long CNX, long long CNXY, const V
 // sp P zc. list: the fine level's active nodes (inactive ones are all held and never written), or null for every node
 // of the level.
 template <class VC = float, class VF = float>
-__global__ void k_prolong(LevelView F, int CPX, int CNY, const int* __restrict__ list, long long count, const VC* __restrict__ zc,
+__global__ void k_prolong(LevelView F, int CPX, int CNY, const int* __restrict__ list, long long count, const VC* zc,
                           VF* __restrict__ zf, float sp, Ctl ctl) {
     const long long CNX = CPX, CNXY = (long long)CPX * CNY;
     const long long t0 = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -475,7 +475,7 @@ __global__ void k_prolong(LevelView F, int CPX, int CNY, const int* __restrict__
         if ((mask & 7) == 7) continue;
         int i, j, k;
         nodeCoords(F, fn, i, j, k);
-        const float z0 = ldf(zf + 3 * fn), z1 = ldf(zf + 3 * fn + 1), z2 = ldf(zf + 3 * fn + 2);
+        const float z0 = ldv<float>(zf + 3 * fn), z1 = ldv<float>(zf + 3 * fn + 1), z2 = ldv<float>(zf + 3 * fn + 2);
         float s[3];
         prolongAt<1>(CNX, CNXY, zc, i, j, k, s);
         constexpr bool SCALED = !std::is_same<VC, float>::value;
@@ -495,7 +495,7 @@ __global__ void k_prolong(LevelView F, int CPX, int CNY, const int* __restrict__
 // (zs: the FP16 coarse-level vectors' iterate-to-residual scale, a power of two; 1 otherwise)
 // A row's first 512 entries are on their way before the kernel before is done and while the block gathers r.
 template <class TI, class TO>
-__global__ void k_coarse(int m, const int* __restrict__ dof, const double* __restrict__ Ainv, const TI* __restrict__ r, TO* __restrict__ z,
+__global__ void k_coarse(int m, const int* __restrict__ dof, const double* __restrict__ Ainv, const TI* r, TO* __restrict__ z,
                          double zs, Ctl ctl) {
     extern __shared__ double rs[];
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -615,7 +615,7 @@ __global__ void k_cg_init(long long nNodes, const uint8_t* __restrict__ nmask, c
 // the V-cycle is linear, so any order-one scale serves, voxel_fea.cpp:843-857) and the first
 // Chebyshev step of the finest level, d = z = c0 D^-1 r32.
 __global__ void __launch_bounds__(VEC_THREADS, 4) k_cg_update(long long nNodes, const uint8_t* __restrict__ nmask, double* __restrict__ x, double* __restrict__ r,
-                            const double* __restrict__ p, const double* __restrict__ q, float* __restrict__ r32, const float* __restrict__ invD,
+                            const double* p, const double* q, float* __restrict__ r32, const float* __restrict__ invD,
                             float* __restrict__ d, float* __restrict__ z, float c0, SolveState* st, double* partials, unsigned* ticket,
                             Ctl ctl) {
     if (skipped(ctl)) return;
@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(VEC_THREADS, 4) k_cg_update(long long nNodes, 
 
 // the preconditioner's input: r32 = float(r / max|r_free|) at free DOFs (voxel_fea.cpp:856-857),
 // and (d non-null) the first Chebyshev step d = z = c0 D^-1 r32
-__global__ void k_vc_load(long long nNodes, const uint8_t* __restrict__ nmask, const double* __restrict__ r, float* __restrict__ r32,
+__global__ void k_vc_load(long long nNodes, const uint8_t* __restrict__ nmask, const double* r, float* __restrict__ r32,
                           const float* __restrict__ invD, float* __restrict__ d, float* __restrict__ z, float c0, SolveState* st, Ctl ctl) {
     if (skipped(ctl)) return;
     const double s = st->scale;
@@ -700,8 +700,8 @@ __global__ void k_vc_load(long long nNodes, const uint8_t* __restrict__ nmask, c
 
 // z = z32 / vscale (or z64); rzNew = r.z, zq = z.q; beta = max(0, -alpha zq / rz)
 // (voxel_fea.cpp:913-917); on the first pass beta = 0. Held DOFs carry zeros and are skipped.
-__global__ void k_cg_dots(long long nNodes, const uint8_t* __restrict__ nmask, const double* __restrict__ r, const float* __restrict__ z32,
-                          const double* __restrict__ z64, const double* __restrict__ q, SolveState* st, double* partials, unsigned* ticket,
+__global__ void k_cg_dots(long long nNodes, const uint8_t* __restrict__ nmask, const double* r, const float* z32,
+                          const double* z64, const double* q, SolveState* st, double* partials, unsigned* ticket,
                           Ctl ctl) {
     if (skipped(ctl)) return;
     const double inv = 1.0 / st->vscale;
@@ -727,7 +727,7 @@ __global__ void k_cg_dots(long long nNodes, const uint8_t* __restrict__ nmask, c
 }
 
 // p = z + beta p at free DOFs
-__global__ void k_cg_p(long long nNodes, const uint8_t* __restrict__ nmask, const float* __restrict__ z32, const double* __restrict__ z64,
+__global__ void k_cg_p(long long nNodes, const uint8_t* __restrict__ nmask, const float* z32, const double* z64,
                        double* __restrict__ p, SolveState* st, Ctl ctl) {
     if (skipped(ctl)) return;
     const double inv = 1.0 / st->vscale, beta = st->beta;
@@ -771,7 +771,7 @@ __global__ void k_final(long long nNodes, const uint8_t* __restrict__ nmask, con
 // (foldIf: the graph condition of the fold's branch, set to the decision); with the V-cycle's first
 // smoothing step from zero fused in, d = z = c0 D^-1 r32 (a fold redoes it on its new r32)
 __global__ void __launch_bounds__(VEC_THREADS, 4) k_mx_update(long long nNodes, const uint8_t* __restrict__ nmask, float* __restrict__ x, float* __restrict__ r,
-                            const float* __restrict__ p, const float* __restrict__ q, const float* __restrict__ invD, float* __restrict__ d,
+                            const float* p, const float* q, const float* __restrict__ invD, float* __restrict__ d,
                             float* __restrict__ z, float c0, SolveState* st, double* partials, unsigned* ticket,
                             cudaGraphConditionalHandle foldIf, int useIf, Ctl ctl) {
     if (skipped(ctl)) return;
@@ -832,7 +832,7 @@ __global__ void k_mx_fold1(long long nDof, double* __restrict__ u, float* __rest
 
 // fold part 2 (after q = K u in FP64): r64 = f - q, rel = ||r64|| / bnorm, r32 = float(r64 * scale);
 // stop when rel <= tol, at the cap or after a breakdown
-__global__ void k_mx_fold2(long long nNodes, const uint8_t* __restrict__ nmask, const double* __restrict__ f, const double* __restrict__ q,
+__global__ void k_mx_fold2(long long nNodes, const uint8_t* __restrict__ nmask, const double* f, const double* q,
                            float* __restrict__ r32, const float* __restrict__ invD, float* __restrict__ d, float* __restrict__ z, float c0,
                            SolveState* st, double* partials, unsigned* ticket, Ctl ctl) {
     if (skipped(ctl)) return;
@@ -880,8 +880,8 @@ __global__ void k_mx_fold2(long long nNodes, const uint8_t* __restrict__ nmask, 
 // rzNew = r32.z32, zq = z32.q32 (FP64 sums); beta as in the FP64 form
 // r.z and z.q over the free DOFs (node by node: the held DOFs, every DOF of an inactive node
 // included, add nothing and are not read)
-__global__ void k_mx_dots(long long nNodes, const uint8_t* __restrict__ nmask, const float* __restrict__ r, const float* __restrict__ z,
-                          const float* __restrict__ q, SolveState* st, double* partials, unsigned* ticket, Ctl ctl) {
+__global__ void k_mx_dots(long long nNodes, const uint8_t* __restrict__ nmask, const float* r, const float* z,
+                          const float* q, SolveState* st, double* partials, unsigned* ticket, Ctl ctl) {
     if (skipped(ctl)) return;
     const bool first = st->first;
     double v[2] = {0, 0};
@@ -922,7 +922,7 @@ __global__ void k_mx_rescale(long long nDof, float* __restrict__ r32, const floa
 
 // p = z + beta p at the free DOFs; the first direction of a solve also writes 0 at every held DOF,
 // which then stays 0 (the later steps skip held DOFs and inactive nodes)
-__global__ void k_mx_p(long long nNodes, const uint8_t* __restrict__ nmask, const float* __restrict__ z, float* __restrict__ p,
+__global__ void k_mx_p(long long nNodes, const uint8_t* __restrict__ nmask, const float* z, float* __restrict__ p,
                        const SolveState* st, Ctl ctl) {
     if (skipped(ctl)) return;
     const float beta = float(st->beta);
@@ -1204,7 +1204,7 @@ namespace dev {
 // residual's scale and the caller passes c2 / rho (exact: powers of two). V = float: rho = 1.
 template <int MODE, bool OWN16, bool CLS, class V = float>
 __global__ void __launch_bounds__(512) k_list(LevelView L, Coefs<float> C, const int* __restrict__ list, int count, int nClass,
-                                               const V* __restrict__ x, V* __restrict__ y, const V* __restrict__ r, V* __restrict__ d,
+                                               const V* x, V* __restrict__ y, const V* r, V* __restrict__ d,
                                                float c1, float c2, float rho, int raw, Ctl ctl) {
     if (skipped(ctl)) return;
     extern __shared__ __align__(16) unsigned char clsRaw[];
@@ -1234,15 +1234,15 @@ __global__ void __launch_bounds__(512) k_list(LevelView L, Coefs<float> C, const
             if (MODE == TOP_APPLY) {
                 stv(y + id, (!raw && fx) ? 0.f : kx);
             } else if (MODE == TOP_RESID) {
-                stv(y + id, fx ? 0.f : ldf(r + id) - kx);
+                stv(y + id, fx ? 0.f : ldv<float>(r + id) - kx);
             } else {
                 if (fx) {
                     stv(d + id, 0.f);
                     stv(y + id, 0.f);
                 } else {
-                    const float dn = c1 * ldf(d + id) + c2 * L.invD[id] * (ldf(r + id) - kx);
+                    const float dn = c1 * ldv<float>(d + id) + c2 * L.invD[id] * (ldv<float>(r + id) - kx);
                     stv(d + id, dn);
-                    stv(y + id, ldf(x + id) + dn);
+                    stv(y + id, ldv<float>(x + id) + dn);
                 }
             }
         }

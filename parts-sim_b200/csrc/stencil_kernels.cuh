@@ -86,7 +86,7 @@ __global__ void k_stn_build(LevelView L, Coefs<CT> C, const int* __restrict__ li
 // slower than one, which the passes use.
 template <int MODE, class ST, class V = float, int NPT = 1>
 __global__ void __launch_bounds__(256) k_stn(LevelView L, const int* __restrict__ list, int count, const ST* __restrict__ stn, float ss,
-                                             const V* __restrict__ x, V* __restrict__ y, const V* __restrict__ r, V* __restrict__ d, float c1,
+                                             const V* x, V* __restrict__ y, const V* r, V* __restrict__ d, float c1,
                                              float c2, float rho, int raw, Ctl ctl) {
     if (skipped(ctl)) return;
     constexpr bool H = !std::is_same<V, float>::value;
@@ -150,15 +150,15 @@ __global__ void __launch_bounds__(256) k_stn(LevelView L, const int* __restrict_
                 if (MODE == TOP_APPLY) {
                     stv(y + id, (!raw && fx) ? 0.f : acc);
                 } else if (MODE == TOP_RESID) {
-                    stv(y + id, fx ? 0.f : ldf(r + id) - acc);
+                    stv(y + id, fx ? 0.f : ldv<float>(r + id) - acc);
                 } else {
                     if (fx) {
                         stv(d + id, 0.f);
                         stv(y + id, 0.f);
                     } else {
-                        const float dn = c1 * ldf(d + id) + c2 * L.invD[id] * (ldf(r + id) - acc);
+                        const float dn = c1 * ldv<float>(d + id) + c2 * L.invD[id] * (ldv<float>(r + id) - acc);
                         stv(d + id, dn);
-                        stv(y + id, ldf(x + id) + dn);
+                        stv(y + id, ldv<float>(x + id) + dn);
                     }
                 }
             }
@@ -175,7 +175,7 @@ __global__ void __launch_bounds__(256) k_stn(LevelView L, const int* __restrict_
 // 1152 count for more than the latency).
 template <int MODE>
 __global__ void __launch_bounds__(256) k_stn8(LevelView L, const int* __restrict__ list, int count, const float4* __restrict__ stn,
-                                              const float* __restrict__ x, float* __restrict__ y, const float* __restrict__ r,
+                                              const float* x, float* __restrict__ y, const float* r,
                                               float* __restrict__ d, float c1, float c2, int raw, Ctl ctl) {
     const int lane = threadIdx.x & 7;
     const long long at = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3;
@@ -195,15 +195,15 @@ __global__ void __launch_bounds__(256) k_stn8(LevelView L, const int* __restrict
         const int m = lane + 8 * u < 27 ? lane + 8 * u : 13;
         const long long o = n + (m % 3 - 1) + ((m / 3) % 3 - 1) * NX + (m / 9 - 1) * NXY;
         const float* xp = x + 3 * (o < 0 ? 0 : o >= L.nNodes ? L.nNodes - 1 : o);
-        xm[u][0] = __ldg(xp);
-        xm[u][1] = __ldg(xp + 1);
-        xm[u][2] = __ldg(xp + 2);
+        xm[u][0] = xp[0];
+        xm[u][1] = xp[1];
+        xm[u][2] = xp[2];
     }
     float rv = 0.f, dv = 0.f, xv = 0.f;
-    if (MODE != TOP_APPLY) rv = __ldg(r + id);
+    if (MODE != TOP_APPLY) rv = r[id];
     if (MODE == TOP_CHEB) {
         dv = d[id];
-        xv = __ldg(x + id);
+        xv = x[id];
     }
     float a[3] = {0.f, 0.f, 0.f};
     const float* cv = reinterpret_cast<const float*>(cf);
