@@ -3462,6 +3462,7 @@ std::unique_ptr<BlockBase> makeBlock(std::shared_ptr<SharedModel> M, int width) 
 
 BlockBase* Solver::blockFor(int nrhs) {
     SolverHandle& Hd = *handle_;
+    impl_->prepareSmoothers();  // (of the degree just set, also for a block made before)
     const int fits = Hd.block ? Hd.block->width() : 0;
     const int want = nrhs <= 8 ? 8 : (nrhs <= 16 ? 16 : 32);
     if (Hd.block && fits >= std::min(want, 32)) return Hd.block.get();
@@ -3469,7 +3470,6 @@ BlockBase* Solver::blockFor(int nrhs) {
     check(cudaStreamSynchronize(impl_->stream), "sync");
     const int w = chooseBlockWidth(impl_->H, nrhs);
     if (!w) return nullptr;
-    impl_->prepareSmoothers();
     Hd.block = makeBlock(impl_->M, w);
     return Hd.block.get();
 }

@@ -75,3 +75,19 @@ def test_calls_one_behind_the_other():
     for a, b in zip(after, alone):
         assert a.iterations == b.iterations and np.array_equal(a.u, b.u)
     del keep
+
+
+@pytest.mark.parametrize("degree", [1, 4])
+def test_smoother_degree_of_the_call_not_of_the_one_before(degree):
+    """A block made before a solve at another smoother degree: the block preconditioner is the reference's degree 2 again, and a
+    block solve has its own degree, both as on a handle of their own."""
+    m = W.l_bracket(40, 20, 20, holes=4, seed=2)
+    F = np.stack([m.f, -2 * m.f])
+    S, T = (psfea.VoxelFEA(m.dims, m.density, m.nu, m.bc, m.coarsest_max_dof) for _ in range(2))
+    r = vectors(S, 3, 9)
+    want = one_by_one(S, r)
+    S.solve(m.f, tol=1e-6, max_iter=2000, smoother_degree=degree)
+    assert torch.equal(one_by_one(S, r), want)
+    S.solve(m.f, tol=1e-6, max_iter=2000, smoother_degree=degree)
+    for a, b in zip(S.solve_batch(F, tol=1e-8, max_iter=2000), T.solve_batch(F, tol=1e-8, max_iter=2000)):
+        assert a.iterations == b.iterations and np.array_equal(a.u, b.u)
