@@ -1836,7 +1836,7 @@ void SharedModel::uploadLevel(int l) {
             D.nTilesAll = int(ta.size());
             upload(D.tilesAll, ta, bytes, ms);
         }
-        D.useTiles = D.useTiles && h.nNodes >= minNodes;
+        D.useTiles = D.useTiles && active > 0 && h.nNodes >= minNodes;  // (an empty level has no tile to launch)
         int64_t max8 = 30000;
         if (const char* e = std::getenv("PSFEA_OP8_MAX_NODES")) max8 = std::atoll(e);
         D.use8 = !D.useTiles && l > 0 && h.nNodes <= max8;
