@@ -75,11 +75,14 @@ void finishLevel(HostLevel& L) {
     // both written in full below (one pass per z plane), so allocated without a serial zero fill
     L.nmask.resize(size_t(L.nNodes));
     L.invDiag.resize(size_t(L.nDof));
-    std::vector<int64_t> freeCount(size_t(L.NZ), 0);
+    L.bitRow = (L.NX + 63) / 64;
+    L.activeBits.assign(size_t(L.bitRow) * L.NY * L.NZ, 0);
+    std::vector<int64_t> freeCount(size_t(L.NZ), 0), activeCount(size_t(L.NZ), 0), ownCount(size_t(L.NZ), 0);
     parallelFor(L.NZ, [&](int64_t k0, int64_t k1) {
         for (int64_t k = k0; k < k1; k++) {
-            int64_t nfree = 0;
-            for (int j = 0; j < L.NY; j++)
+            int64_t nfree = 0, nActive = 0, nOwnNodes = 0;
+            for (int j = 0; j < L.NY; j++) {
+                uint64_t* bits = L.activeBits.data() + L.bitRow * (j + int64_t(L.NY) * k);
                 for (int i = 0; i < L.NX; i++) {
                     const int64_t n = L.node(i, j, int(k));
                     double diag[3] = {0, 0, 0};
@@ -102,6 +105,9 @@ void finishLevel(HostLevel& L) {
                     uint8_t m = 0;
                     if (active) {
                         m |= NM_ACTIVE;
+                        bits[i >> 6] |= uint64_t(1) << (i & 63);
+                        nActive++;
+                        nOwnNodes += own;
                         if (uniform && w0 && !(w0 & OWN_BIT)) m |= NM_UNIFORM;
                         if (!own) m |= NM_PLAIN;
                     }
@@ -118,11 +124,18 @@ void finishLevel(HostLevel& L) {
                     }
                     L.nmask[n] = m;
                 }
+            }
             freeCount[size_t(k)] = nfree;
+            activeCount[size_t(k)] = nActive;
+            ownCount[size_t(k)] = nOwnNodes;
         }
     }, 1);
-    L.freeDof = 0;
-    for (auto c : freeCount) L.freeDof += c;
+    L.freeDof = L.nActive = L.nOwnNodes = 0;
+    for (int k = 0; k < L.NZ; k++) {
+        L.freeDof += freeCount[size_t(k)];
+        L.nActive += activeCount[size_t(k)];
+        L.nOwnNodes += ownCount[size_t(k)];
+    }
     L.boundary.clear();
     for (int64_t n = 0; n < L.nNodes; n++)
         if ((L.nmask[n] & NM_ACTIVE) && !(L.nmask[n] & NM_UNIFORM)) L.boundary.push_back(int32_t(n));

@@ -56,6 +56,10 @@ struct HostLevel {
     std::vector<double, UninitAlloc<double>> invDiag;  // per DOF, 0 where fixed
     std::vector<uint8_t, UninitAlloc<uint8_t>> nmask;  // per node
     std::vector<int32_t> boundary;  // active nodes without NM_UNIFORM, increasing
+    // what the device's tile lists are made from, gathered where the masks are made (one pass on all threads):
+    int64_t nActive = 0, nOwnNodes = 0;  // active nodes; those of them that touch an own matrix
+    int64_t bitRow = 0;                  // words of a node row in activeBits
+    std::vector<uint64_t> activeBits;    // one bit per node, rows (j, k) in order
     double lmax = 0;              // largest eigenvalue estimate of D^-1 K (smoother), 0 = not yet
 
     int64_t node(int i, int j, int k) const { return i + int64_t(NX) * (j + int64_t(NY) * k); }

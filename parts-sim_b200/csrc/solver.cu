@@ -1350,15 +1350,15 @@ int gridFor(int64_t n, int threads, int cap) {
 // The element in the reflection basis: block entries (1/64) h_a^T K h_b over the modes h_a = product of (2 x - 1)^a,
 // which vanish outside the blocks of march_kernels.cuh for the element of an isotropic cube and its Galerkin sums
 // over uniform children (checked: ok is false if Kb is anything else).
-template <class T>
-dev::ModeCoefs<T> marchCoefs(const double Kb[576], bool& ok) {
+dev::ModeCoefs<double> marchCoefs(const double Kb[576], bool& ok) {
     double B[24][24];  // [3 a + c][3 b + e], a = ax + 2 ay + 4 az
-    auto sign = [](int a, int corner) {
-        double v = 1;
-        for (int d = 0; d < 3; d++)
-            if ((a >> d) & 1) v *= 2.0 * CORNER_XYZ[corner][d] - 1;
-        return v;
-    };
+    double sign[8][8];
+    for (int a = 0; a < 8; a++)
+        for (int corner = 0; corner < 8; corner++) {
+            sign[a][corner] = 1;
+            for (int d = 0; d < 3; d++)
+                if ((a >> d) & 1) sign[a][corner] *= 2.0 * CORNER_XYZ[corner][d] - 1;
+        }
     double big = 0;
     for (int a = 0; a < 8; a++)
         for (int b = 0; b < 8; b++)
@@ -1366,7 +1366,7 @@ dev::ModeCoefs<T> marchCoefs(const double Kb[576], bool& ok) {
                 for (int e = 0; e < 3; e++) {
                     double v = 0;
                     for (int p = 0; p < 8; p++)
-                        for (int q = 0; q < 8; q++) v += sign(a, p) * sign(b, q) * Kb[(3 * p + c) * 24 + 3 * q + e];
+                        for (int q = 0; q < 8; q++) v += sign[a][p] * sign[b][q] * Kb[(3 * p + c) * 24 + 3 * q + e];
                     B[3 * a + c][3 * b + e] = v / 64;
                     big = std::max(big, std::fabs(v / 64));
                 }
@@ -1394,65 +1394,78 @@ dev::ModeCoefs<T> marchCoefs(const double Kb[576], bool& ok) {
     ok = true;
     for (int r = 0; r < 24; r++)
         for (int q = 0; q < 24; q++) ok = ok && std::fabs(M[r][q] - B[r][q]) <= 1e-12 * big;
-    return {T(b0), T(a0), T(a1), T(b1), T(c2), T(e2), T(b3), T(a3)};
+    return {b0, a0, a1, b1, c2, e2, b3, a3};
 }
 
-// which planes of which columns of nx x ny nodes hold an active node: [k][ty][tx]
-std::vector<uint8_t> marchActivity(const HostLevel& h, int nx, int ny) {
-    const int ntx = (h.NX + nx - 1) / nx, nty = (h.NY + ny - 1) / ny;
-    const size_t cols = size_t(ntx) * nty;
-    std::vector<uint8_t> act(cols * h.NZ, 0);
-    parallelFor(h.NZ, [&](int64_t ka, int64_t kb) {
-        for (int64_t k = ka; k < kb; k++)
-            for (int j = 0; j < h.NY; j++) {
-                const uint8_t* row = h.nmask.data() + h.node(0, j, int(k));
-                uint8_t* a = act.data() + size_t(k) * cols + size_t(j / ny) * ntx;
-                for (int t = 0; t < ntx; t++) {
-                    uint8_t any = 0;
-                    for (int i = t * nx, e = std::min(h.NX, i + nx); i < e; i++) any |= row[i];
-                    a[t] |= (any & NM_ACTIVE) ? 1 : 0;
-                }
-            }
-    }, 8);
+// which tiles of nx nodes of each node row (j, k) hold an active node: [k][j][tx]
+std::vector<uint8_t> rowTiles(const HostLevel& h, int nx) {
+    const int ntx = (h.NX + nx - 1) / nx;  // (nx < 64)
+    const int64_t rows = int64_t(h.NY) * h.NZ;
+    std::vector<uint8_t> any(size_t(rows) * ntx);
+    for (int64_t row = 0; row < rows; row++) {
+        const uint64_t* bits = h.activeBits.data() + h.bitRow * row;
+        for (int t = 0, at = 0; t < ntx; t++, at += nx) {
+            uint64_t b = bits[at >> 6] >> (at & 63);
+            if ((at & 63) + nx > 64 && (at >> 6) + 1 < h.bitRow) b |= bits[(at >> 6) + 1] << (64 - (at & 63));
+            any[size_t(row) * ntx + t] = (b & ((uint64_t(1) << nx) - 1)) != 0;
+        }
+    }
+    return any;
+}
+
+// which planes of which columns of ny of those rows hold an active node: [k][ty][tx]
+std::vector<uint8_t> marchActivity(const HostLevel& h, const std::vector<uint8_t>& rows, int ny) {
+    const int nty = (h.NY + ny - 1) / ny;
+    const size_t ntx = rows.size() / (size_t(h.NY) * h.NZ);
+    std::vector<uint8_t> act(ntx * nty * h.NZ, 0);
+    for (int64_t k = 0; k < h.NZ; k++)
+        for (int j = 0; j < h.NY; j++) {
+            const uint8_t* in = rows.data() + (size_t(k) * h.NY + j) * ntx;
+            uint8_t* a = act.data() + (size_t(k) * nty + j / ny) * ntx;
+            for (size_t t = 0; t < ntx; t++) a[t] |= in[t];
+        }
     return act;
 }
 
-// The tiles of a marched level: columns of nx x ny nodes (`groups` CTAs each) cut into chunks of planes, trimmed to the planes with an
-// active node. A CTA of n planes takes about n + 4 steps (one plane of halo below and above, two to fill and
-// drain), so the chunk length is the one with the least waves x steps on `slots` resident CTAs: long chunks where
-// the level has many columns, short ones where it would leave SMs idle. whole: every column and plane, untrimmed, the
-// chunks without an active node marked.
-// act: marchActivity's of the same nx x ny. steps: the waves x steps of the choice.
-std::vector<dev::MarchTile> marchTiles(const HostLevel& h, const std::vector<uint8_t>& act, int nx, int ny, int groups, int slots, bool whole = false,
-                                       int64_t* steps = nullptr) {
+// The planes of a chunk of a marched level's columns (act: marchActivity's; `groups` CTAs each). A CTA of n planes takes about
+// n + 4 steps (one plane of halo below and above, two to fill and drain), so the chunk length is the one with the
+// least waves x steps on `slots` resident CTAs: long chunks where the level has many columns, short ones where it would
+// leave SMs idle.
+struct MarchCut {
+    int planes = 1;
+    int64_t steps = INT64_MAX;  // waves x steps
+};
+MarchCut marchCut(const HostLevel& h, const std::vector<uint8_t>& act, int groups, int slots) {
+    const size_t cols = act.size() / size_t(h.NZ);
+    std::vector<uint8_t> live(cols, 0);
+    for (size_t k = 0; k < size_t(h.NZ); k++)
+        for (size_t c = 0; c < cols; c++) live[c] |= act[k * cols + c];
+    int64_t n = 0;
+    for (uint8_t v : live) n += v;
+    MarchCut best;
+    for (int tz = 1; tz <= std::min(h.NZ, 96); tz++) {
+        const int64_t ctas = n * groups * ((h.NZ + tz - 1) / tz), steps = ((ctas + slots - 1) / slots) * (tz + 4);
+        if (steps < best.steps) best = {tz, steps};
+    }
+    return best;
+}
+
+// The tiles of a marched level: its columns cut into chunks, trimmed to the planes with an active node. whole: every column and
+// plane, untrimmed, the chunks without an active node marked.
+std::vector<dev::MarchTile> marchTiles(const HostLevel& h, const std::vector<uint8_t>& act, int nx, MarchCut cut, bool whole = false) {
     const int ntx = (h.NX + nx - 1) / nx;
     const size_t cols = act.size() / size_t(h.NZ);
-    size_t live = 0;
-    for (size_t c = 0; c < cols; c++) {
-        bool any = false;
-        for (int k = 0; k < h.NZ && !any; k++) any = act[size_t(k) * cols + c] != 0;
-        live += any;
-    }
-    int best = 1;
-    int64_t bestCost = INT64_MAX;
-    for (int tz = 1; tz <= std::min(h.NZ, 96); tz++) {
-        const int64_t ctas = int64_t(live) * groups * ((h.NZ + tz - 1) / tz), cost = ((ctas + slots - 1) / slots) * (tz + 4);
-        if (cost < bestCost) {
-            bestCost = cost;
-            best = tz;
-        }
-    }
-    if (steps) *steps = bestCost;
     std::vector<dev::MarchTile> out;
-    for (int kz = 0; kz < h.NZ; kz += best)
+    for (int kz = 0; kz < h.NZ; kz += cut.planes)
         for (size_t c = 0; c < cols; c++) {
+            const int kEnd = std::min(h.NZ, kz + cut.planes);
             int lo = -1, hi = -1;
-            for (int k = kz; k < std::min(h.NZ, kz + best); k++)
+            for (int k = kz; k < kEnd; k++)
                 if (act[size_t(k) * cols + c]) {
                     if (lo < 0) lo = k;
                     hi = k + 1;
                 }
-            if (whole) out.push_back({uint16_t(size_t(c % ntx) | (lo < 0 ? dev::MARCH_EMPTY : 0)), uint16_t(c / ntx), uint16_t(kz), uint16_t(std::min(h.NZ, kz + best))});
+            if (whole) out.push_back({uint16_t(size_t(c % ntx) | (lo < 0 ? dev::MARCH_EMPTY : 0)), uint16_t(c / ntx), uint16_t(kz), uint16_t(kEnd)});
             else if (lo >= 0) out.push_back({uint16_t(c % ntx), uint16_t(c / ntx), uint16_t(lo), uint16_t(hi)});
         }
     return out;
@@ -1473,7 +1486,8 @@ struct DevLevel {
     int nTilesAll = 0;
     int nActive = 0;   // active nodes
     // marched levels: the boundary nodes (active, not uniform) and those of them that touch an own
-    // matrix (pitched indices, increasing); the marching kernel leaves one of the two lists out
+    // matrix (pitched indices, increasing); the marching kernel leaves one of the two lists out. The
+    // first list is only there once a split asked for it (ensureBoundaryList).
     DevMem blist, olist;
     int nBnd = 0, nOwnNodes = 0;
     bool inner64 = false;  // 64-bit marches compute the boundary nodes without own matrices too (else k_bnd does)
@@ -1583,6 +1597,7 @@ struct SharedModel {
     void build(const int32_t dims[3], const float* density, double nu, const uint8_t* bc, int64_t coarsest, const double* diagAdd);
     void adopt(Hierarchy&& h);  // upload a hierarchy built on the host beforehand
     void uploadLevel(int l);
+    void ensureBoundaryList(int l);
     void ensureActiveLists();
     // the assembled stencils of the levels in stencilLevels (FP16 copies too when half); the
     // callers' streams wait on readyEv
@@ -1780,24 +1795,7 @@ void SharedModel::uploadLevel(int l) {
     {
         // (the largest grids the 64-bit tile indices of the element-block lists hold)
         if ((h.NX + 31) / 32 > 2047 || (h.NY + 7) / 8 > 2047 || (h.NZ + 3) / 4 > 1023) throw Error(PS_EINVAL, "grid too large for the tile index");
-        // active nodes, and those of them that touch an own matrix
-        std::vector<int64_t> planeActive(size_t(h.NZ), 0), planeOwn(size_t(h.NZ), 0);
-        parallelFor(h.NZ, [&](int64_t k0, int64_t k1) {
-            for (int64_t k = k0; k < k1; k++) {
-                const uint8_t* mk = h.nmask.data() + h.node(0, 0, int(k));
-                int64_t n = 0, o = 0;
-                for (int64_t q = 0; q < int64_t(h.NX) * h.NY; q++) {
-                    n += (mk[q] & NM_ACTIVE) ? 1 : 0;
-                    o += (mk[q] & (NM_ACTIVE | NM_PLAIN)) == NM_ACTIVE ? 1 : 0;
-                }
-                planeActive[size_t(k)] = n;
-                planeOwn[size_t(k)] = o;
-            }
-        }, 8);
-        int64_t active = 0, ownNodes = 0;
-        for (int64_t n : planeActive) active += n;
-        for (int64_t n : planeOwn) ownNodes += n;
-        D.nActive = int(active);
+        D.nActive = int(h.nActive);
         if (h.nOwn == 0 && l < 63 && ((ebeLevels >> l) & 1)) {
             // the element-block tiles (8 x 8 x 4 nodes) with an active node
             const int ex = (h.NX + dev::EX - 1) / dev::EX, ey = (h.NY + dev::EY - 1) / dev::EY, ez = (h.NZ + dev::EZ - 1) / dev::EZ;
@@ -1825,18 +1823,27 @@ void SharedModel::uploadLevel(int l) {
         // (and where more than half of the active nodes touch an own matrix the march has little to do: the stencils then
         // take the whole level. Gyroid 256x256x128, level 1 with 97 % such nodes: 31 us a pass saved beside the 122 of the stencils)
         int64_t minNodes = h.nOwn == 0 ? 8000 : 400000;
-        if (2 * ownNodes > active) minNodes = INT64_MAX;
+        if (2 * h.nOwnNodes > h.nActive) minNodes = INT64_MAX;
         if (const char* e = std::getenv("PSFEA_TILE_MIN_NODES")) minNodes = std::atoll(e);
-        D.m64 = marchCoefs<double>(h.Kb, D.useTiles);
-        D.m32 = marchCoefs<float>(h.Kb, D.useTiles);
-        std::vector<uint8_t> act64;
-        if (D.useTiles && (l == 0 || h.nNodes >= minNodes)) act64 = marchActivity(h, dev::MARCH_NX, dev::marchRows<double>() - 2);
+        if (l == 0 || (h.nActive > 0 && h.nNodes >= minNodes)) {
+            const dev::ModeCoefs<double> c = D.m64 = marchCoefs(h.Kb, D.useTiles);
+            D.m32 = {float(c.b0), float(c.a0), float(c.a1), float(c.b1), float(c.c2), float(c.e2), float(c.b3), float(c.a3)};
+        }
+        const bool march = D.useTiles && h.nActive > 0 && h.nNodes >= minNodes;  // (an empty level has no tile to launch)
+        // (host lists on one thread: a few ms at 28 M nodes, and beside other builds a fork and join waits for its last thread)
+        std::vector<uint8_t> rows, act64;
+        MarchCut cut64;
+        if (march || (l == 0 && D.useTiles)) {
+            rows = rowTiles(h, dev::MARCH_NX);
+            act64 = marchActivity(h, rows, dev::marchRows<double>() - 2);
+            cut64 = marchCut(h, act64, 1, smCount);
+        }
         if (l == 0 && D.useTiles) {
-            const std::vector<dev::MarchTile> ta = marchTiles(h, act64, dev::MARCH_NX, dev::marchRows<double>() - 2, 1, smCount, true);
+            const std::vector<dev::MarchTile> ta = marchTiles(h, act64, dev::MARCH_NX, cut64, true);
             D.nTilesAll = int(ta.size());
             upload(D.tilesAll, ta, bytes, ms);
         }
-        D.useTiles = D.useTiles && active > 0 && h.nNodes >= minNodes;  // (an empty level has no tile to launch)
+        D.useTiles = march;
         int64_t max8 = 30000;
         if (const char* e = std::getenv("PSFEA_OP8_MAX_NODES")) max8 = std::atoll(e);
         D.use8 = !D.useTiles && l > 0 && h.nNodes <= max8;
@@ -1845,31 +1852,25 @@ void SharedModel::uploadLevel(int l) {
             // halo of a tall one is a smaller share, but its planes take 1.1-1.2 times as long, so that it pays where there are several waves:
             // smoothing step at 14 / 18 rows, gyroid 256x256x128 190 / 169 us, 384x384x192 563 / 508, against SIMP 192x96x96
             // (one wave) 43.1 / 47.3, SIMP 96x48x48 12.4 / 13.3, cantilever 64x16x16 7.5 / 8.3
-            int64_t costLow = 0, costTall = 0;
-            std::vector<dev::MarchTile> t32 = marchTiles(h, marchActivity(h, dev::MARCH_NX, dev::marchRows<float>() - 2), dev::MARCH_NX, dev::marchRows<float>() - 2, 1, smCount, false, &costLow);
-            std::vector<dev::MarchTile> tall = marchTiles(h, marchActivity(h, dev::MARCH_NX, dev::MARCH_ROWS_TALL - 2), dev::MARCH_NX, dev::MARCH_ROWS_TALL - 2, 1, smCount, false, &costTall);
-            D.tall32 = dev::MARCH_TALL_STEP * double(costTall) < double(costLow);
+            std::vector<uint8_t> act32 = marchActivity(h, rows, dev::marchRows<float>() - 2), actTall = marchActivity(h, rows, dev::MARCH_ROWS_TALL - 2);
+            MarchCut cut32 = marchCut(h, act32, 1, smCount), cutTall = marchCut(h, actTall, 1, smCount);
+            D.tall32 = dev::MARCH_TALL_STEP * double(cutTall.steps) < double(cut32.steps);
             if (const char* e = std::getenv("PSFEA_MARCH_TALL")) D.tall32 = std::atoi(e) != 0;
-            if (D.tall32) t32.swap(tall);
-            const std::vector<dev::MarchTile> t64 = marchTiles(h, act64, dev::MARCH_NX, dev::marchRows<double>() - 2, 1, smCount);
+            const std::vector<dev::MarchTile> t32 = marchTiles(h, D.tall32 ? actTall : act32, dev::MARCH_NX, D.tall32 ? cutTall : cut32);
+            const std::vector<dev::MarchTile> t64 = marchTiles(h, act64, dev::MARCH_NX, cut64);
             D.nTiles32 = int(t32.size());
             D.nTiles64 = int(t64.size());
             upload(D.tiles32, t32, bytes, ms);
             upload(D.tiles64, t64, bytes, ms);
-            std::vector<int32_t> bl(h.boundary.size()), ol;
-            parallelFor(int64_t(bl.size()), [&](int64_t lo, int64_t hi) {
-                for (int64_t q = lo; q < hi; q++) {
-                    const int64_t nd = h.boundary[size_t(q)], row = nd / h.NX;
-                    bl[size_t(q)] = int32_t((nd - row * h.NX) + int64_t(PX) * row);
-                }
-            });
-            if (ownNodes > 0)
-                for (size_t q = 0; q < bl.size(); q++)
-                    if (!(h.nmask[size_t(h.boundary[q])] & NM_PLAIN)) ol.push_back(bl[q]);
-            D.nBnd = int(bl.size());
-            D.nOwnNodes = int(ol.size());
-            upload(D.blist, bl, bytes, ms);
-            upload(D.olist, ol, bytes, ms);
+            D.nBnd = int(h.boundary.size());
+            if (h.nOwnNodes > 0) {
+                std::vector<int32_t> ol;
+                ol.reserve(size_t(h.nOwnNodes));
+                for (int32_t nd : h.boundary)
+                    if (!(h.nmask[size_t(nd)] & NM_PLAIN)) ol.push_back(int32_t(nd + int64_t(PX - h.NX) * (nd / h.NX)));
+                D.nOwnNodes = int(ol.size());
+                upload(D.olist, ol, bytes, ms);
+            }
             // the marches compute every node that touches no own matrix: a boundary node costs them no more
             // than a uniform one. PSFEA_TILE_INNER64=0 and PSFEA_TILE_SPLIT32 (bit l set = level l) leave all
             // boundary nodes to the list kernels instead
@@ -1877,6 +1878,7 @@ void SharedModel::uploadLevel(int l) {
             if (const char* e = std::getenv("PSFEA_TILE_INNER64")) D.inner64 = std::atoi(e) != 0;
             D.split32 = false;
             if (const char* e = std::getenv("PSFEA_TILE_SPLIT32")) D.split32 = l < 63 && ((std::atoll(e) >> l) & 1);
+            if (D.split32 || !D.inner64) ensureBoundaryList(l);
         }
     }
     dev::LevelView& v = D.view;
@@ -1900,6 +1902,19 @@ void SharedModel::uploadLevel(int l) {
             D.c64.S[m * 9 + e] = h.S[m][e];
             D.c32.S[m * 9 + e] = float(h.S[m][e]);
         }
+}
+
+// the boundary nodes of a marched level, for a split; the caller waits on readyEv
+void SharedModel::ensureBoundaryList(int l) {
+    DevLevel& D = L[size_t(l)];
+    if (D.blist.p || !D.nBnd) return;
+    const HostLevel& h = H.levels[size_t(l)];
+    const int pad = pitch4(h.NX) - h.NX;
+    std::vector<int32_t> bl;
+    bl.reserve(h.boundary.size());
+    for (int32_t nd : h.boundary) bl.push_back(int32_t(nd + int64_t(pad) * (nd / h.NX)));
+    upload(D.blist, bl, bytes, ms);
+    check(cudaEventRecord(readyEv, ms), "event");
 }
 
 void SharedModel::ensureStencils(bool half) {
@@ -3077,13 +3092,17 @@ struct BlockImpl final : BlockBase {
         for (DevMem* b : {&f, &x, &r, &p, &q}) b->alloc(n, bytes, stream);
         if (M->exactOneLevel()) z64.alloc(n, bytes, stream);
         state.alloc(sizeof(dev::BlockState), bytes, stream);
-        const auto t32 = marchTiles(H.levels[0], marchActivity(H.levels[0], dev::BM_NX, dev::bmNY<float>()), dev::BM_NX, dev::bmNY<float>(), RB / dev::BM_G, smCount);
-        const auto t64 = marchTiles(H.levels[0], marchActivity(H.levels[0], dev::BM_NX, dev::bmNY<double>()), dev::BM_NX, dev::bmNY<double>(), RB / dev::BM_G, smCount);
+        const HostLevel& h0 = H.levels[0];
+        const std::vector<uint8_t> rows = rowTiles(h0, dev::BM_NX);
+        auto tilesOf = [&](int ny) {
+            const std::vector<uint8_t> a = marchActivity(h0, rows, ny);
+            return marchTiles(h0, a, dev::BM_NX, marchCut(h0, a, RB / dev::BM_G, smCount));
+        };
+        const auto t32 = tilesOf(dev::bmNY<float>()), t64 = tilesOf(dev::bmNY<double>());
         nTiles32 = int(t32.size());
         nTiles64 = int(t64.size());
         upload(tiles32, t32, bytes, stream);
         upload(tiles64, t64, bytes, stream);
-        check(cudaStreamSynchronize(stream), "tile upload");  // (from pageable memory that ends here)
         partials.alloc((size_t(smCount) * 16 * 3 + size_t(nTiles64)) * RB * sizeof(double) + 4096, bytes, stream);
         ticket.alloc(64, bytes, stream);
         check(cudaStreamWaitEvent(stream, M->readyEv, 0), "wait");
@@ -3794,7 +3813,9 @@ TuneResult Solver::autotune(const double* fHost, const ps_solve_opts& base, bool
             if (!D.useTiles) continue;
             D.split32 = (t.splitLevels >> l) & 1;
             if (l == 0) D.inner64 = t.inner64 != 0;
+            if (D.split32 || !D.inner64) M.ensureBoundaryList(int(l));
         }
+        check(cudaEventSynchronize(M.readyEv), "boundary lists");
         M.version++;  // the iteration graphs are recorded again
     };
     if (!force) {
