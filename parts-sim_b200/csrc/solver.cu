@@ -1482,7 +1482,7 @@ struct DevLevel {
     DevMem tiles32, tiles64;  // marched levels: the 32- and 64-bit tiles with an active node
     int nTiles32 = 0, nTiles64 = 0;
     bool tall32 = false;  // the 32-bit tiles are tall ones
-    DevMem tilesAll;          // the finest level: 64-bit tiles over the whole grid (the allocation-free product)
+    DevMem tilesAll;          // the finest level: 64-bit tiles over the whole grid (the allocation-free product), or none: per node
     int nTilesAll = 0;
     int nActive = 0;   // active nodes
     // marched levels: the boundary nodes (active, not uniform) and those of them that touch an own
@@ -1824,21 +1824,33 @@ void SharedModel::uploadLevel(int l) {
         // take the whole level. Gyroid 256x256x128, level 1 with 97 % such nodes: 31 us a pass saved beside the 122 of the stencils)
         int64_t minNodes = h.nOwn == 0 ? 8000 : 400000;
         if (2 * h.nOwnNodes > h.nActive) minNodes = INT64_MAX;
-        if (const char* e = std::getenv("PSFEA_TILE_MIN_NODES")) minNodes = std::atoll(e);
+        const char* forced = std::getenv("PSFEA_TILE_MIN_NODES");
+        if (forced) minNodes = std::atoll(forced);
         if (l == 0 || (h.nActive > 0 && h.nNodes >= minNodes)) {
             const dev::ModeCoefs<double> c = D.m64 = marchCoefs(h.Kb, D.useTiles);
             D.m32 = {float(c.b0), float(c.a0), float(c.a1), float(c.b1), float(c.c2), float(c.e2), float(c.b3), float(c.a3)};
         }
-        const bool march = D.useTiles && h.nActive > 0 && h.nNodes >= minNodes;  // (an empty level has no tile to launch)
+        bool march = D.useTiles && h.nActive > 0 && h.nNodes >= minNodes;  // (an empty level has no tile to launch)
         // (host lists on one thread: a few ms at 28 M nodes, and beside other builds a fork and join waits for its last thread)
-        std::vector<uint8_t> rows, act64;
-        MarchCut cut64;
+        std::vector<uint8_t> rows, act64, act32, actTall;
+        MarchCut cut64, cut32, cutTall;
         if (march || (l == 0 && D.useTiles)) {
             rows = rowTiles(h, dev::MARCH_NX);
             act64 = marchActivity(h, rows, dev::marchRows<double>() - 2);
             cut64 = marchCut(h, act64, 1, smCount);
         }
-        if (l == 0 && D.useTiles) {
+        if (march) {
+            act32 = marchActivity(h, rows, dev::marchRows<float>() - 2);
+            actTall = marchActivity(h, rows, dev::MARCH_ROWS_TALL - 2);
+            cut32 = marchCut(h, act32, 1, smCount);
+            cutTall = marchCut(h, actTall, 1, smCount);
+            // A slender grid has few columns, each a long march with most of its lanes idle: a step takes some 0.95 us, one thread
+            // per node 6-8 us a pass at 8 k to 30 k nodes (smoothing step marched / per node: 1x1x4000 voxels 32 steps, 32.7 / 8.3 us; 1x100x100
+            // 10 steps, 12.4 / 8.3; 4x4x330 7 steps, 8.3 / 8.3; 20x20x20 5 steps, 6.7 / 8.3)
+            if (!forced && std::max(cut32.steps, cut64.steps) > 6 + h.nNodes / 8000) march = false;
+        }
+        // (the allocation-free product: 1x1x4000 35.2 / 13.5 us, 2x2x1000 11 steps, 16.5 / 14.7, 4x4x330 7 steps, 12.4 / 14.5)
+        if (l == 0 && D.useTiles && (forced || cut64.steps <= 8 + h.nNodes / 8000)) {
             const std::vector<dev::MarchTile> ta = marchTiles(h, act64, dev::MARCH_NX, cut64, true);
             D.nTilesAll = int(ta.size());
             upload(D.tilesAll, ta, bytes, ms);
@@ -1852,8 +1864,6 @@ void SharedModel::uploadLevel(int l) {
             // halo of a tall one is a smaller share, but its planes take 1.1-1.2 times as long, so that it pays where there are several waves:
             // smoothing step at 14 / 18 rows, gyroid 256x256x128 190 / 169 us, 384x384x192 563 / 508, against SIMP 192x96x96
             // (one wave) 43.1 / 47.3, SIMP 96x48x48 12.4 / 13.3, cantilever 64x16x16 7.5 / 8.3
-            std::vector<uint8_t> act32 = marchActivity(h, rows, dev::marchRows<float>() - 2), actTall = marchActivity(h, rows, dev::MARCH_ROWS_TALL - 2);
-            MarchCut cut32 = marchCut(h, act32, 1, smCount), cutTall = marchCut(h, actTall, 1, smCount);
             D.tall32 = dev::MARCH_TALL_STEP * double(cutTall.steps) < double(cut32.steps);
             if (const char* e = std::getenv("PSFEA_MARCH_TALL")) D.tall32 = std::atoi(e) != 0;
             const std::vector<dev::MarchTile> t32 = marchTiles(h, D.tall32 ? actTall : act32, dev::MARCH_NX, D.tall32 ? cutTall : cut32);
@@ -3973,6 +3983,36 @@ constexpr int NOALLOC_BLOCKS = 4096;
 constexpr size_t NOALLOC_BYTES = 256 + size_t(NOALLOC_BLOCKS) * sizeof(double);  // ticket line + partials
 static __device__ __align__(256) unsigned char g_noallocScratch[NOALLOC_BYTES];
 
+namespace dev {
+
+// q = K p (FP64, held DOFs 0) and p.q into *dot, a node a thread: the product of slender grids. p and q are the
+// caller's vectors in the reference's dense layout (node nd = i + NX (j + NY k)); masks, words and the diagonal shift
+// are the level's pitched arrays.
+__global__ void __launch_bounds__(NODE_THREADS) k_apply_dot_static(LevelView L, Coefs<double> C, const double* __restrict__ p,
+                                                                   double* __restrict__ q, double* __restrict__ dot, double* partials,
+                                                                   unsigned* ticket) {
+    double v[1] = {0.0};
+    const long long nDense = (long long)L.NX * L.NY * L.NZ;
+    for (long long nd = blockIdx.x * (long long)blockDim.x + threadIdx.x; nd < nDense; nd += (long long)gridDim.x * blockDim.x) {
+        const long long row = nd / L.NX;
+        const int i = int(nd - row * L.NX), j = int(row % L.NY), k = int(row / L.NY);
+        const long long n = i + (long long)L.PX * row;
+        const uint8_t mask = __ldg(L.nmask + n);
+        double acc[3];
+        applyAt<double, false>(L, C, p, i, j, k, nd, mask, acc, L.NX, n);
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+            const double y = fixedDof(mask, c) ? 0.0 : acc[c];
+            q[3 * nd + c] = y;
+            v[0] += p[3 * nd + c] * y;
+        }
+    }
+    double tot[1];
+    if (gridReduce<1>(v, 0u, partials, ticket, tot) && threadIdx.x == 0) *dot = tot[0];
+}
+
+}  // namespace dev
+
 namespace {
 
 // device address of g_noallocScratch on device devId (the current device), looked up once per
@@ -3996,7 +4036,8 @@ unsigned char* noallocScratch(int devId) {
 void Solver::applyDotStatic(const double* xDev, double* yDev, double* dotDev, void* s) {
     SolverImpl& I = *impl_;
     DevLevel& D = I.L[0];
-    const int grid = std::min(D.nTilesAll, I.smCount * 16);
+    const bool march = D.nTilesAll > 0;
+    const int grid = march ? std::min(D.nTilesAll, I.smCount * 16) : I.nodeGrid(I.H.levels[0].nNodes);
     if (grid > NOALLOC_BLOCKS)
         throw Error(PS_EINVAL, "this device needs " + std::to_string(grid) + " reduction blocks; the static scratch holds " +
                                    std::to_string(NOALLOC_BLOCKS));
@@ -4010,10 +4051,14 @@ void Solver::applyDotStatic(const double* xDev, double* yDev, double* dotDev, vo
     if (st != I.stream) check(cudaStreamWaitEvent(st, I.M->readyEv, 0), "wait for the model");
     unsigned char* scratch = noallocScratch(cur);
     check(cudaMemsetAsync(scratch, 0, 256, st), "ticket clear");
-    I.launch(dev::k_march<double, dev::TOP_DOT, true>, grid, dev::marchThreads<double>(), dev::marchSmemBytes<double>(), st, D.view, D.m64,
-             D.tilesAll.as<dev::MarchTile>(), xDev, yDev, static_cast<const float*>(nullptr), static_cast<float*>(nullptr), dev::MarchIO{0.f, 0.f, 0, 0, 0u, D.nTilesAll, dotDev},
-             static_cast<dev::SolveState*>(nullptr), reinterpret_cast<double*>(scratch + 256), reinterpret_cast<unsigned*>(scratch),
-             dev::Ctl{nullptr, nullptr});
+    double* partials = reinterpret_cast<double*>(scratch + 256);
+    unsigned* ticket = reinterpret_cast<unsigned*>(scratch);
+    if (march)
+        I.launch(dev::k_march<double, dev::TOP_DOT, true>, grid, dev::marchThreads<double>(), dev::marchSmemBytes<double>(), st, D.view, D.m64,
+                 D.tilesAll.as<dev::MarchTile>(), xDev, yDev, static_cast<const float*>(nullptr), static_cast<float*>(nullptr), dev::MarchIO{0.f, 0.f, 0, 0, 0u, D.nTilesAll, dotDev},
+                 static_cast<dev::SolveState*>(nullptr), partials, ticket, dev::Ctl{nullptr, nullptr});
+    else
+        I.launch(dev::k_apply_dot_static, grid, dev::NODE_THREADS, 0, st, D.view, D.c64, xDev, yDev, dotDev, partials, ticket);
     check(cudaGetLastError(), "apply_dot_static");
 }
 
