@@ -2197,6 +2197,14 @@ struct SolverImpl {
             for (DevMem* b : {&W[l].r, &W[l].z, &W[l].t, &W[l].d}) check(cudaMemsetAsync(b->p, 0, b->bytes, stream), "memset");
         halfLeft = false;
     }
+    // the model's stencils of a V-cycle, made on first use, and this context's stream behind them
+    void bringStencils(bool half) {
+        if (exactOneLevel()) return;
+        M->ensureStencils(half);
+        const bool ready = M->actReady.load(std::memory_order_acquire);
+        check(cudaStreamWaitEvent(stream, M->readyEv, 0), "wait");
+        listsWaited = listsWaited || ready;
+    }
     float* vcycleFor(bool half, dev::Ctl ctl, bool own16, bool firstDone = false) {
         return half ? vcycleHalf(ctl, own16, firstDone) : vcycle(0, ctl, own16, firstDone);
     }
@@ -2844,12 +2852,7 @@ void SolverImpl::startIterations() {
     pend.mixed = mixed;
     pend.half = half;
     stn16Pass = mixed;
-    if (!exactOneLevel()) {
-        M->ensureStencils(mixed && M->mixedOwn16);
-        const bool ready = M->actReady.load(std::memory_order_acquire);
-        check(cudaStreamWaitEvent(stream, M->readyEv, 0), "wait");
-        listsWaited = listsWaited || ready;
-    }
+    bringStencils(mixed && M->mixedOwn16);
     if (!half) clearHalf();
     if (half) {
         halfLeft = true;
@@ -3704,6 +3707,7 @@ void Solver::precondition(const double* rHost, double* zHost) {
     const int64_t n = I.pd(0), nn = I.pn(0);
     I.setDegree(2);  // the reference's preconditioner
     I.prepareSmoothers();
+    I.bringStencils(false);  // (the FP64 form's V-cycle, whatever ran before on the handle)
     I.clearHalf();
     I.uploadPitched(rHost, I.r.as<double>(), 0, I.q.as<double>());
     const dev::Ctl none{nullptr, nullptr};
