@@ -1471,6 +1471,61 @@ std::vector<dev::MarchTile> marchTiles(const HostLevel& h, const std::vector<uin
     return out;
 }
 
+// Which passes over a level are marched, and its columns' activity and cuts.
+struct MarchPlan {
+    bool march = false;  // the solves' operator passes
+    bool dense = false;  // the allocation-free product (finest level)
+    dev::ModeCoefs<double> coefs{};
+    std::vector<uint8_t> act64, act32, actTall;
+    MarchCut cut64, cut32, cutTall;
+};
+MarchPlan planMarch(const HostLevel& h, int l, int slots) {
+    MarchPlan p;
+    // (marched levels with own matrices take a second launch for the nodes that touch one: worth it from 400 k nodes;
+    // without, one thread per node is the faster only below some 8 k nodes: 64x16x16 cantilever 1.45 -> 1.26 ms a solve,
+    // SIMP 96x48x48 19.6 -> 16.5 ms, while marching that grid's level 1 of 30 k nodes, 85 % own matrices, costs 1.2 ms)
+    // (and where more than half of the active nodes touch an own matrix the march has little to do: the stencils then
+    // take the whole level. Gyroid 256x256x128, level 1 with 97 % such nodes: 31 us a pass saved beside the 122 of the stencils)
+    int64_t minNodes = h.nOwn == 0 ? 8000 : 400000;
+    if (2 * h.nOwnNodes > h.nActive) minNodes = INT64_MAX;
+    const char* forced = std::getenv("PSFEA_TILE_MIN_NODES");
+    if (forced) minNodes = std::atoll(forced);
+    p.march = h.nActive > 0 && h.nNodes >= minNodes;  // (an empty level has no tile to launch)
+    if (!p.march && l > 0) return p;
+    bool ok = false;
+    p.coefs = marchCoefs(h.Kb, ok);
+    p.march = p.march && ok;
+    if (!ok) return p;
+    // (host lists on one thread: a few ms at 28 M nodes, and beside other builds a fork and join waits for its last thread)
+    const std::vector<uint8_t> rows = rowTiles(h, dev::MARCH_NX);
+    p.act64 = marchActivity(h, rows, dev::marchRows<double>() - 2);
+    p.cut64 = marchCut(h, p.act64, 1, slots);
+    if (p.march) {
+        p.act32 = marchActivity(h, rows, dev::marchRows<float>() - 2);
+        p.actTall = marchActivity(h, rows, dev::MARCH_ROWS_TALL - 2);
+        p.cut32 = marchCut(h, p.act32, 1, slots);
+        p.cutTall = marchCut(h, p.actTall, 1, slots);
+        // A slender grid has few columns, each a long march with most of its lanes idle: a step takes some 0.95 us, one thread
+        // per node 6-8 us a pass at 8 k to 30 k nodes (smoothing step marched / per node: 1x1x4000 voxels 32 steps, 32.7 / 8.3 us; 1x100x100
+        // 10 steps, 12.4 / 8.3; 4x4x330 7 steps, 8.3 / 8.3; 20x20x20 5 steps, 6.7 / 8.3)
+        if (!forced && std::max(p.cut32.steps, p.cut64.steps) > 6 + h.nNodes / 8000) p.march = false;
+    }
+    // (the allocation-free product: 1x1x4000 35.2 / 13.5 us, 2x2x1000 11 steps, 16.5 / 14.7, 4x4x330 7 steps, 12.4 / 14.5)
+    p.dense = l == 0 && (forced || p.cut64.steps <= 8 + h.nNodes / 8000);
+    return p;
+}
+
+// levels with assembled stencils (PSFEA_STENCIL_LEVELS: bit l = level l, never level 0), and the list length from which a
+// thread takes a whole node (PSFEA_STENCIL_MIN_NODES: shorter node lists give eight lanes to a node)
+int64_t stencilLevelsKnob() {
+    const char* e = std::getenv("PSFEA_STENCIL_LEVELS");
+    return (e ? std::atoll(e) : ~int64_t(0)) & ~int64_t(1);
+}
+int64_t stencilMinNodesKnob() {
+    const char* e = std::getenv("PSFEA_STENCIL_MIN_NODES");
+    return e ? std::atoll(e) : 65536;
+}
+
 // Read-only device data of one level, shared by every solve context of a handle.
 struct DevLevel {
     dev::LevelView view{};
@@ -1611,8 +1666,7 @@ struct SharedModel {
     // kernel operand, and measured on the SIMP block solve its stencils were 16-20 % slower (paired
     // or not) than the constant-operand gather
     bool blockStencil0 = false;
-    int64_t stencilLevels = ~int64_t(1);  // PSFEA_STENCIL_LEVELS: bit l = level l (never level 0)
-    int64_t stencilMinNodes = 65536;      // PSFEA_STENCIL_MIN_NODES: shorter node lists give eight lanes to a node
+    int64_t stencilLevels = 0, stencilMinNodes = 0;  // stencilLevelsKnob, stencilMinNodesKnob
     bool foldBranch = true;               // PSFEA_FOLD_BRANCH: the FP32-Krylov fold as a conditional graph branch
     bool exactOneLevel() const { return L.size() == 1 && H.hasFactor(); }
 };
@@ -1640,8 +1694,8 @@ void SharedModel::adopt(Hierarchy&& h) {
     if (const char* e = std::getenv("PSFEA_CLS_SMEM")) clsSmemMax = size_t(std::atoll(e));
     if (const char* e = std::getenv("PSFEA_LIST_LEVELS")) listLevels = std::atoll(e);
     if (const char* e = std::getenv("PSFEA_REFINE_ETA")) refineEta = std::atof(e);
-    if (const char* e = std::getenv("PSFEA_STENCIL_LEVELS")) stencilLevels = std::atoll(e) & ~int64_t(1);
-    if (const char* e = std::getenv("PSFEA_STENCIL_MIN_NODES")) stencilMinNodes = std::atoll(e);
+    stencilLevels = stencilLevelsKnob();
+    stencilMinNodes = stencilMinNodesKnob();
     if (const char* e = std::getenv("PSFEA_FOLD_BRANCH")) foldBranch = std::atoi(e) != 0;
     if (const char* e = std::getenv("PSFEA_BLOCK_STENCIL")) blockStencils = std::atoi(e) != 0;
     if (const char* e = std::getenv("PSFEA_BLOCK_STENCIL0")) blockStencil0 = std::atoi(e) != 0;
@@ -1815,47 +1869,16 @@ void SharedModel::uploadLevel(int l) {
             upload(D.ebeTiles, el, bytes, ms);
             D.ebe = D.nEbeTiles > 0;
         }
-        // small levels have too few tiles to fill the GPU: one thread per node instead, or eight
-        // lanes per node on the smallest ones
-        // (marched levels with own matrices take a second launch for the nodes that touch one: worth it from 400 k nodes;
-        // without, one thread per node is the faster only below some 8 k nodes: 64x16x16 cantilever 1.45 -> 1.26 ms a solve,
-        // SIMP 96x48x48 19.6 -> 16.5 ms, while marching that grid's level 1 of 30 k nodes, 85 % own matrices, costs 1.2 ms)
-        // (and where more than half of the active nodes touch an own matrix the march has little to do: the stencils then
-        // take the whole level. Gyroid 256x256x128, level 1 with 97 % such nodes: 31 us a pass saved beside the 122 of the stencils)
-        int64_t minNodes = h.nOwn == 0 ? 8000 : 400000;
-        if (2 * h.nOwnNodes > h.nActive) minNodes = INT64_MAX;
-        const char* forced = std::getenv("PSFEA_TILE_MIN_NODES");
-        if (forced) minNodes = std::atoll(forced);
-        if (l == 0 || (h.nActive > 0 && h.nNodes >= minNodes)) {
-            const dev::ModeCoefs<double> c = D.m64 = marchCoefs(h.Kb, D.useTiles);
-            D.m32 = {float(c.b0), float(c.a0), float(c.a1), float(c.b1), float(c.c2), float(c.e2), float(c.b3), float(c.a3)};
-        }
-        bool march = D.useTiles && h.nActive > 0 && h.nNodes >= minNodes;  // (an empty level has no tile to launch)
-        // (host lists on one thread: a few ms at 28 M nodes, and beside other builds a fork and join waits for its last thread)
-        std::vector<uint8_t> rows, act64, act32, actTall;
-        MarchCut cut64, cut32, cutTall;
-        if (march || (l == 0 && D.useTiles)) {
-            rows = rowTiles(h, dev::MARCH_NX);
-            act64 = marchActivity(h, rows, dev::marchRows<double>() - 2);
-            cut64 = marchCut(h, act64, 1, smCount);
-        }
-        if (march) {
-            act32 = marchActivity(h, rows, dev::marchRows<float>() - 2);
-            actTall = marchActivity(h, rows, dev::MARCH_ROWS_TALL - 2);
-            cut32 = marchCut(h, act32, 1, smCount);
-            cutTall = marchCut(h, actTall, 1, smCount);
-            // A slender grid has few columns, each a long march with most of its lanes idle: a step takes some 0.95 us, one thread
-            // per node 6-8 us a pass at 8 k to 30 k nodes (smoothing step marched / per node: 1x1x4000 voxels 32 steps, 32.7 / 8.3 us; 1x100x100
-            // 10 steps, 12.4 / 8.3; 4x4x330 7 steps, 8.3 / 8.3; 20x20x20 5 steps, 6.7 / 8.3)
-            if (!forced && std::max(cut32.steps, cut64.steps) > 6 + h.nNodes / 8000) march = false;
-        }
-        // (the allocation-free product: 1x1x4000 35.2 / 13.5 us, 2x2x1000 11 steps, 16.5 / 14.7, 4x4x330 7 steps, 12.4 / 14.5)
-        if (l == 0 && D.useTiles && (forced || cut64.steps <= 8 + h.nNodes / 8000)) {
-            const std::vector<dev::MarchTile> ta = marchTiles(h, act64, dev::MARCH_NX, cut64, true);
+        const MarchPlan plan = planMarch(h, l, smCount);
+        D.useTiles = plan.march;
+        D.m64 = plan.coefs;
+        D.m32 = {float(D.m64.b0), float(D.m64.a0), float(D.m64.a1), float(D.m64.b1), float(D.m64.c2), float(D.m64.e2), float(D.m64.b3), float(D.m64.a3)};
+        if (plan.dense) {
+            const std::vector<dev::MarchTile> ta = marchTiles(h, plan.act64, dev::MARCH_NX, plan.cut64, true);
             D.nTilesAll = int(ta.size());
             upload(D.tilesAll, ta, bytes, ms);
         }
-        D.useTiles = march;
+        // small levels have too few tiles to fill the GPU: one thread per node instead, or eight lanes per node on the smallest ones
         int64_t max8 = 30000;
         if (const char* e = std::getenv("PSFEA_OP8_MAX_NODES")) max8 = std::atoll(e);
         D.use8 = !D.useTiles && l > 0 && h.nNodes <= max8;
@@ -1864,10 +1887,10 @@ void SharedModel::uploadLevel(int l) {
             // halo of a tall one is a smaller share, but its planes take 1.1-1.2 times as long, so that it pays where there are several waves:
             // smoothing step at 14 / 18 rows, gyroid 256x256x128 190 / 169 us, 384x384x192 563 / 508, against SIMP 192x96x96
             // (one wave) 43.1 / 47.3, SIMP 96x48x48 12.4 / 13.3, cantilever 64x16x16 7.5 / 8.3
-            D.tall32 = dev::MARCH_TALL_STEP * double(cutTall.steps) < double(cut32.steps);
+            D.tall32 = dev::MARCH_TALL_STEP * double(plan.cutTall.steps) < double(plan.cut32.steps);
             if (const char* e = std::getenv("PSFEA_MARCH_TALL")) D.tall32 = std::atoi(e) != 0;
-            const std::vector<dev::MarchTile> t32 = marchTiles(h, D.tall32 ? actTall : act32, dev::MARCH_NX, D.tall32 ? cutTall : cut32);
-            const std::vector<dev::MarchTile> t64 = marchTiles(h, act64, dev::MARCH_NX, cut64);
+            const std::vector<dev::MarchTile> t32 = marchTiles(h, D.tall32 ? plan.actTall : plan.act32, dev::MARCH_NX, D.tall32 ? plan.cutTall : plan.cut32);
+            const std::vector<dev::MarchTile> t64 = marchTiles(h, plan.act64, dev::MARCH_NX, plan.cut64);
             D.nTiles32 = int(t32.size());
             D.nTiles64 = int(t64.size());
             upload(D.tiles32, t32, bytes, ms);
@@ -3535,7 +3558,10 @@ Solver::Solver(Hierarchy&& hier) {
 }
 
 int64_t estimateDeviceBytes(const Hierarchy& H) {
-    // what SharedModel::adopt and one SolverImpl::allocate take, plus allocation slack
+    // what SharedModel::adopt, one SolverImpl::allocate and the first solve (ensureStencils) take, plus allocation slack
+    int dev = 0, slots = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&slots, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) cudaGetLastError();
+    const int64_t stencils = stencilLevelsKnob(), minNodes = stencilMinNodesKnob();
     int64_t b = 0, allocs = 0;
     for (size_t l = 0; l < H.levels.size(); l++) {
         const HostLevel& h = H.levels[l];
@@ -3545,14 +3571,26 @@ int64_t estimateDeviceBytes(const Hierarchy& H) {
              4 * (h.nNodes / 1024 + 1);
         if (l == 0) b += dofs;
         b += 16 * dofs;  // V-cycle vectors r, z, t, d
-        if (l > 0 && nodes < 65536) b += 4 * int64_t(dev::STN8_ROW) * nodes;  // the small levels' stencils
-        allocs += 12;
+        const MarchPlan plan = planMarch(h, int(l), slots);
+        if (plan.march || plan.dense) {  // tile lists (at most a tile a cut of every column) and the reductions' partial sums
+            auto tiles = [&](const std::vector<uint8_t>& act, MarchCut c) { return int64_t(act.size()) / h.NZ * ((h.NZ + c.planes - 1) / c.planes); };
+            const int64_t t64 = tiles(plan.act64, plan.cut64);
+            const int64_t t32 = plan.march ? std::max(tiles(plan.act32, plan.cut32), tiles(plan.actTall, plan.cutTall)) : 0;
+            b += int64_t(sizeof(dev::MarchTile)) * (2 * t64 + t32) + 32 * std::max(t32, t64);
+        }
+        if (H.levels.size() > 1) b += 4 * h.nActive + (l == 0 ? 4 * (nodes / 64 + 1) : 0);  // active lists, the block tiles made with them
+        if (plan.march) b += 4 * h.nOwnNodes;
+        if (l > 0 && l < 63 && ((stencils >> l) & 1)) {
+            const int64_t n = plan.march ? (h.nOwnNodes >= minNodes ? h.nOwnNodes : 0) : h.nActive;
+            b += 4 * n * (n < minNodes ? int64_t(dev::STN8_ROW) : 4 * int64_t(dev::stnChunks<4>()));  // (the FP16 rows are smaller)
+        }
+        allocs += 17;
     }
     const int64_t n = 3 * int64_t(pitch4(H.levels[0].NX)) * H.levels[0].NY * H.levels[0].NZ;
     b += 40 * n + 12 * n + (H.levels.size() == 1 ? 8 * n : 0);
     b += 4 * H.coarseM + 8 * H.coarseM * H.coarseM;
     b += 4096 * 32 + 64 * 1024;
-    allocs += 16;
+    allocs += 17;
     return b + allocs * (64 << 10);
 }
 
