@@ -1495,7 +1495,12 @@ MarchPlan planMarch(const HostLevel& h, int l, int slots) {
     bool ok = false;
     p.coefs = marchCoefs(h.Kb, ok);
     p.march = p.march && ok;
-    if (!ok) return p;
+    if (!ok) {
+        // The block solve and the allocation-free product have no other finest-level operator. (No element of an isotropic cube
+        // gets here: for nu from -0.9999 to 0.499999 its entries outside the blocks are some 1e-16 of the largest.)
+        if (l == 0) throw Error(PS_EINVAL, "The element matrix does not split into the reflection modes of a cube.");
+        return p;
+    }
     // (host lists on one thread: a few ms at 28 M nodes, and beside other builds a fork and join waits for its last thread)
     const std::vector<uint8_t> rows = rowTiles(h, dev::MARCH_NX);
     p.act64 = marchActivity(h, rows, dev::marchRows<double>() - 2);
