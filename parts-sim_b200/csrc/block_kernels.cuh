@@ -237,18 +237,16 @@ __device__ __forceinline__ void applyNbr(const LevelView& L, const Coefs<T>& C, 
 // once per node for the whole block.
 constexpr int STN_ROW = 252;
 __host__ __device__ constexpr int stnPairAt(int m, int p, int q) { return 18 * (m >> 1) + 2 * (3 * p + q) + (m & 1); }
-template <class T>
-__host__ __device__ constexpr size_t stnBlockSmem(int npw) { return size_t(BLOCK_THREADS / 32) * npw * STN_ROW * sizeof(T); }
+__host__ __device__ constexpr size_t stnBlockSmem(int npw) { return size_t(BLOCK_THREADS / 32) * npw * STN_ROW * sizeof(float); }
 
-template <class T, int S>
-__device__ __forceinline__ void stnBlock(const LevelView& L, const T* __restrict__ row, const T* __restrict__ x, long long n, int i, int j,
-                                         int k, T acc[3]) {
-    static_assert(sizeof(T) == 4, "the paired layout is FP32");
+template <int S>
+__device__ __forceinline__ void stnBlock(const LevelView& L, const float* __restrict__ row, const float* __restrict__ x, long long n, int i,
+                                         int j, int k, float acc[3]) {
     const long long NX = L.PX, NXY = (long long)L.PX * L.NY;
     auto xOf = [&](int m, float (&v)[3]) {
         const int ox = m % 3 - 1, oy = (m / 3) % 3 - 1, oz = m / 9 - 1;
         const bool in = m < 27 && i + ox >= 0 && j + oy >= 0 && k + oz >= 0 && i + ox < L.NX && j + oy < L.NY && k + oz < L.NZ;
-        const T* xp = x + 3 * S * (n + ox + oy * NX + oz * NXY);
+        const float* xp = x + 3 * S * (n + ox + oy * NX + oz * NXY);
         v[0] = in ? __ldg(xp) : 0.f;
         v[1] = in ? __ldg(xp + S) : 0.f;
         v[2] = in ? __ldg(xp + 2 * S) : 0.f;
@@ -311,7 +309,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, STN ? 4 : 2) kb_op(LevelView L,
             int i, j, k;
             nodeCoords(L, n, i, j, k);
             float acc[3];
-            if constexpr (STN) stnBlock<float, RB>(L, rows + sub * STN_ROW, x + q, n, i, j, k, acc);
+            if constexpr (STN) stnBlock<RB>(L, rows + sub * STN_ROW, x + q, n, i, j, k, acc);
             else applyNbr<float, OWN16, RB>(L, C, x + q, i, j, k, n, mask, acc);
 #pragma unroll
             for (int c = 0; c < 3; c++) {

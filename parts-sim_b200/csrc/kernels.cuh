@@ -353,7 +353,7 @@ __host__ __device__ constexpr size_t align128(size_t b) { return (b + 127) & ~si
 // Bound on the polls of a shared-memory barrier. A wait that never completes (it cannot in a correct
 // launch) is given up: the CTA records ST_ERR_STAGING in st->err and ends the solve.
 constexpr unsigned TILE_WAIT_POLLS = 1u << 22;
-constexpr int ST_ERR_STAGING = 1, ST_ERR_ALIGN = 2;
+constexpr int ST_ERR_STAGING = 1;
 
 // ---- shared-memory barrier primitives (PTX, sm_90 and later)
 __device__ __forceinline__ unsigned smemAddr(const void* p) { return unsigned(__cvta_generic_to_shared(p)); }

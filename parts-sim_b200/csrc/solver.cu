@@ -1716,26 +1716,20 @@ void SharedModel::adopt(Hierarchy&& h) {
         set(dev::k_march<double, dev::TOP_APPLY>, dev::marchSmemBytes<double>());
         set(dev::k_march<double, dev::TOP_DOT>, dev::marchSmemBytes<double>());
         set(dev::k_march<double, dev::TOP_DOT, true>, dev::marchSmemBytes<double>());
-        set(dev::k_march<float, dev::TOP_APPLY>, dev::marchSmemBytes<float>());
         set(dev::k_march<float, dev::TOP_CHEB>, dev::marchSmemBytes<float>());
         set(dev::k_march<float, dev::TOP_RESID>, dev::marchSmemBytes<float>());
         set(dev::k_march<float, dev::TOP_DOT>, dev::marchSmemBytes<float>());
-        set(dev::k_march<float, dev::TOP_APPLY, false, dev::MARCH_ROWS_TALL>, dev::marchSmemBytes<float>(dev::MARCH_ROWS_TALL));
         set(dev::k_march<float, dev::TOP_CHEB, false, dev::MARCH_ROWS_TALL>, dev::marchSmemBytes<float>(dev::MARCH_ROWS_TALL));
         set(dev::k_march<float, dev::TOP_RESID, false, dev::MARCH_ROWS_TALL>, dev::marchSmemBytes<float>(dev::MARCH_ROWS_TALL));
         set(dev::k_march<float, dev::TOP_DOT, false, dev::MARCH_ROWS_TALL>, dev::marchSmemBytes<float>(dev::MARCH_ROWS_TALL));
-        set(dev::k_ebe<dev::TOP_APPLY, 1>, dev::ebeSmemBytes<1>());
         set(dev::k_ebe<dev::TOP_CHEB, 1>, dev::ebeSmemBytes<1>());
         set(dev::k_ebe<dev::TOP_RESID, 1>, dev::ebeSmemBytes<1>());
-        set(dev::k_ebe<dev::TOP_APPLY, 3>, dev::ebeSmemBytes<3>());
         set(dev::k_ebe<dev::TOP_CHEB, 3>, dev::ebeSmemBytes<3>());
         set(dev::k_ebe<dev::TOP_RESID, 3>, dev::ebeSmemBytes<3>());
         set(dev::k_list<dev::TOP_CHEB, true, true>, 200 * 1024);
         set(dev::k_list<dev::TOP_CHEB, false, true>, 200 * 1024);
         set(dev::k_list<dev::TOP_RESID, true, true>, 200 * 1024);
         set(dev::k_list<dev::TOP_RESID, false, true>, 200 * 1024);
-        set(dev::k_list<dev::TOP_APPLY, true, true>, 200 * 1024);
-        set(dev::k_list<dev::TOP_APPLY, false, true>, 200 * 1024);
         set(dev::k_list<dev::TOP_CHEB, true, true, __half>, 200 * 1024);
         set(dev::k_list<dev::TOP_CHEB, false, true, __half>, 200 * 1024);
         set(dev::k_list<dev::TOP_RESID, true, true, __half>, 200 * 1024);
@@ -2338,7 +2332,7 @@ void SolverImpl::op32(int l, const float* xin, float* y, float c1, float c2, dev
     float* dd = W[size_t(l)].d.as<float>();
     if (own16 && D.ebe) {
         // the reduced-precision forms: the element-block product on the tensor cores
-        constexpr int EM = MODE == dev::OP_CHEB ? dev::TOP_CHEB : (MODE == dev::OP_RESID ? dev::TOP_RESID : dev::TOP_APPLY);
+        constexpr int EM = MODE == dev::OP_CHEB ? dev::TOP_CHEB : dev::TOP_RESID;
         const uint32_t* et = D.ebeTiles.as<uint32_t>();
         if (M->ebeSplit == 1)
             launch(dev::k_ebe<EM, 1>, D.nEbeTiles, dev::EBE_THREADS, dev::ebeSmemBytes<1>(), stream, D.view, static_cast<const dev::Coefs<float>&>(D.c32),
@@ -2349,7 +2343,7 @@ void SolverImpl::op32(int l, const float* xin, float* y, float c1, float c2, dev
         return;
     }
     const bool o16 = own16 && D.hasOwn, diff = o16 && M->ownDiff;
-    constexpr int SM_ = MODE == dev::OP_CHEB ? dev::TOP_CHEB : (MODE == dev::OP_RESID ? dev::TOP_RESID : dev::TOP_APPLY);
+    constexpr int SM_ = MODE == dev::OP_CHEB ? dev::TOP_CHEB : dev::TOP_RESID;
     // the assembled stencils of the listed nodes: FP16 in the FP32-Krylov forms, FP32 in the
     // FP64-Krylov ones (PS_PREC_MIXED included: FP16 rounding of the assembled sums, the uniformly
     // scaled voxels' exact FP32 part included, moved its iteration count on the ill-conditioned
@@ -2368,7 +2362,7 @@ void SolverImpl::op32(int l, const float* xin, float* y, float c1, float c2, dev
                      (!D.useTiles || D.stnNodes == D.list(D.split32));
     if (l > 0 && !diff && !D.useTiles && D.stn8.p) {  // a small level
         launch(dev::k_stn8<SM_>, unsigned((int64_t(D.nStn) * 8 + 255) / 256), 256, 0, stream, D.view, D.stnNodes, D.nStn, D.stn8.as<float4>(), xin, y, rr,
-               dd, c1, c2, 0, ctl);
+               dd, c1, c2, ctl);
         return;
     }
     if (stn && !D.useTiles) {
@@ -2377,7 +2371,7 @@ void SolverImpl::op32(int l, const float* xin, float* y, float c1, float c2, dev
     }
     if (l < 63 && ((M->listLevels >> l) & 1) && !diff && !M->act.empty()) {
         // the whole level over its active-node list
-        constexpr int LM = MODE == dev::OP_CHEB ? dev::TOP_CHEB : (MODE == dev::OP_RESID ? dev::TOP_RESID : dev::TOP_APPLY);
+        constexpr int LM = MODE == dev::OP_CHEB ? dev::TOP_CHEB : dev::TOP_RESID;
         const int* al = M->act[size_t(l)].as<int>();
         const int na = M->nAct[size_t(l)];
         const size_t cls = D.hasOwn ? size_t(D.nOwnDev) * 576 * (o16 ? 2 : 4) : 0;
@@ -2498,7 +2492,7 @@ void SolverImpl::op16(int l, const __half* xin, __half* y, float c1, float c2, d
     DevLevel& D = L[size_t(l)];
     const int na = M->nAct[size_t(l)];
     if (!na) return;
-    constexpr int LM = MODE == dev::OP_CHEB ? dev::TOP_CHEB : (MODE == dev::OP_RESID ? dev::TOP_RESID : dev::TOP_APPLY);
+    constexpr int LM = MODE == dev::OP_CHEB ? dev::TOP_CHEB : dev::TOP_RESID;
     const float delta = M->halfDelta[size_t(l)], rho = 1.f / delta;
     const __half* rr = W[size_t(l)].r.as<__half>();
     __half* dd = W[size_t(l)].d.as<__half>();
@@ -3043,8 +3037,7 @@ bool SolverImpl::advance(bool block, ps_solve_result& res) {
     const dev::SolveState& hs = *hostState;
     if (hs.err) {
         pend.active = false;
-        throw Error(PS_ECUDA, hs.err == dev::ST_ERR_STAGING ? "a tiled operator kernel gave up waiting for its staged data"
-                                                            : "a tiled operator kernel found its shared memory misaligned");
+        throw Error(PS_ECUDA, "the tensor-core operator gave up waiting for its products");
     }
     ps_status outcome = pend.outcome;
     res.iterations = hs.it;
@@ -3111,8 +3104,8 @@ struct BlockImpl final : BlockBase {
             auto set = [](auto kernel, size_t b) {
                 check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(b)), "attr");
             };
-            set(dev::kb_op<dev::BOP_CHEB, false, RB, true>, dev::stnBlockSmem<float>(32 / RB));
-            set(dev::kb_op<dev::BOP_RESID, false, RB, true>, dev::stnBlockSmem<float>(32 / RB));
+            set(dev::kb_op<dev::BOP_CHEB, false, RB, true>, dev::stnBlockSmem(32 / RB));
+            set(dev::kb_op<dev::BOP_RESID, false, RB, true>, dev::stnBlockSmem(32 / RB));
             set(dev::kb_march<float, dev::BOP_CHEB, RB>, dev::bmSmemBytes<float>());
             set(dev::kb_march<float, dev::BOP_RESID, RB>, dev::bmSmemBytes<float>());
             set(dev::kb_march<double, dev::BOP_APPLY, RB>, dev::bmSmemBytes<double>());
@@ -3210,7 +3203,7 @@ struct BlockImpl final : BlockBase {
             // the assembled stencils of the Galerkin levels
             const float* stn = M->bstn32.empty() ? nullptr : M->bstn32[size_t(l)].template as<float>();
             if (stn)
-                launch(dev::kb_op<MODE, false, RB, true>, laneGrid(l), dev::BLOCK_THREADS, dev::stnBlockSmem<float>(32 / RB), D.view, C, act(l),
+                launch(dev::kb_op<MODE, false, RB, true>, laneGrid(l), dev::BLOCK_THREADS, dev::stnBlockSmem(32 / RB), D.view, C, act(l),
                        nAct(l), stn, xin, y, rr, dd, c1, c2, raw ? 1 : 0, ctl);
             else if (l == 0)
                 launch(dev::kb_march<float, MODE, RB>, nTiles32 * (RB / dev::BM_G), dev::bmThreads<float>(), dev::bmSmemBytes<float>(), D.view, D.m32,

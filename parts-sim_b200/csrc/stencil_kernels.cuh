@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(256) k_stn(LevelView L, const int* __restrict_
     }
 }
 
-// The same passes on the small levels, eight lanes a node: lane l holds the blocks of the neighbours l, l + 8, l + 16
+// The smoothing and residual passes on the small levels, eight lanes a node: lane l holds the blocks of the neighbours l, l + 8, l + 16
 // and l + 24 (36 floats in nine 16-byte loads, the nine lines of a node contiguous), the eight partial sums meet by shuffles
 // and three lanes run the epilogue. A level of some thousand nodes is a chain of dependent loads, not a stream: here
 // it is list entry, neighbour values, sum, and everything else (coefficients, r, d, 1/diag) is on its way beside it.
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(256) k_stn(LevelView L, const int* __restrict_
 template <int MODE>
 __global__ void __launch_bounds__(256) k_stn8(LevelView L, const int* __restrict__ list, int count, const float4* __restrict__ stn,
                                               const float* x, float* __restrict__ y, const float* r,
-                                              float* __restrict__ d, float c1, float c2, int raw, Ctl ctl) {
+                                              float* __restrict__ d, float c1, float c2, Ctl ctl) {
     const int lane = threadIdx.x & 7;
     const long long at = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3;
     const long long t = at < count ? at : count - 1;  // (a repeat of the last node, not stored)
@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(256) k_stn8(LevelView L, const int* __restrict
         xm[u][1] = xp[1];
         xm[u][2] = xp[2];
     }
-    float rv = 0.f, dv = 0.f, xv = 0.f;
-    if (MODE != TOP_APPLY) rv = r[id];
+    const float rv = r[id];
+    float dv = 0.f, xv = 0.f;
     if (MODE == TOP_CHEB) {
         dv = d[id];
         xv = x[id];
@@ -218,9 +218,7 @@ __global__ void __launch_bounds__(256) k_stn8(LevelView L, const int* __restrict
     if (at >= count || lane >= 3) return;
     const float kx = q == 0 ? a[0] : (q == 1 ? a[1] : a[2]);
     const bool fx = fixedDof(mask, q);
-    if (MODE == TOP_APPLY) {
-        y[id] = (!raw && fx) ? 0.f : kx;
-    } else if (MODE == TOP_RESID) {
+    if (MODE == TOP_RESID) {
         y[id] = fx ? 0.f : rv - kx;
     } else {
         const float dn = fx ? 0.f : c1 * dv + c2 * iv * (rv - kx);
