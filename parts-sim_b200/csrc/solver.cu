@@ -1502,6 +1502,18 @@ MarchPlan planMarch(const HostLevel& h, int l, int slots) {
         return p;
     }
     // (host lists on one thread: a few ms at 28 M nodes, and beside other builds a fork and join waits for its last thread)
+    // Slender and thin grids: most lanes of a tile are idle (few columns, few rows in a column) or most of its steps are its
+    // ends (few planes). A step takes some 0.9 us whatever it does, one thread per node 6-8 us a pass on small levels and some 65 ps
+    // (FP64 product 130 ps) a voxel on large ones: marched where a third of the lanes work or where the steps are fewer than that. Smoothing step
+    // marched / per node, us: 1x1x4000 voxels 32.7 / 8.3, 1x100x100 12.4 / 8.3, 1000x1x1000 240 / 76, 1000x1000x1 90 / 72, 500x2x500 64 / 32;
+    // 20x20x20 6.7 / 8.3, 12x12x1000 12.4 / 19, 300x300x4 19.5 / 21-26. Allocation-free product: 1x1x4000 35 / 13.5, 2x2x1000 16.5 / 14.7,
+    // 1000x1x1000 235 / 141; 4x4x330 12.4 / 14.5, 300x300x4 33 / 50.
+    // (Below the finest level the other route is the assembled stencils, some 140 ps a node: 500x500x2's level 1 of 250x250x1, 12 steps, solve
+    // 23 ms marched, 28 on stencils.)
+    auto slender = [&](MarchCut c, int ny, int64_t few, int64_t other) {
+        const bool thirdBusy = 3 * h.nNodes >= c.steps * slots * dev::MARCH_NX * ny;
+        return !thirdBusy && c.steps > std::max(few, other);
+    };
     const std::vector<uint8_t> rows = rowTiles(h, dev::MARCH_NX);
     p.act64 = marchActivity(h, rows, dev::marchRows<double>() - 2);
     p.cut64 = marchCut(h, p.act64, 1, slots);
@@ -1510,13 +1522,13 @@ MarchPlan planMarch(const HostLevel& h, int l, int slots) {
         p.actTall = marchActivity(h, rows, dev::MARCH_ROWS_TALL - 2);
         p.cut32 = marchCut(h, p.act32, 1, slots);
         p.cutTall = marchCut(h, p.actTall, 1, slots);
-        // A slender grid has few columns, each a long march with most of its lanes idle: a step takes some 0.95 us, one thread
-        // per node 6-8 us a pass at 8 k to 30 k nodes (smoothing step marched / per node: 1x1x4000 voxels 32 steps, 32.7 / 8.3 us; 1x100x100
-        // 10 steps, 12.4 / 8.3; 4x4x330 7 steps, 8.3 / 8.3; 20x20x20 5 steps, 6.7 / 8.3)
-        if (!forced && std::max(p.cut32.steps, p.cut64.steps) > 6 + h.nNodes / 8000) p.march = false;
+        // (the finest level's FP64 passes take the same route)
+        const bool thin = l == 0 ? slender(p.cut32, dev::marchRows<float>() - 2, 7, 3 + h.nVox / 14000) ||
+                                       slender(p.cut64, dev::marchRows<double>() - 2, 10, 3 + h.nVox / 7500)
+                                 : slender(p.cut32, dev::marchRows<float>() - 2, 7, 3 + h.nNodes / 6400);
+        if (thin && !forced) p.march = false;
     }
-    // (the allocation-free product: 1x1x4000 35.2 / 13.5 us, 2x2x1000 11 steps, 16.5 / 14.7, 4x4x330 7 steps, 12.4 / 14.5)
-    p.dense = l == 0 && (forced || p.cut64.steps <= 8 + h.nNodes / 8000);
+    p.dense = l == 0 && (forced || !slender(p.cut64, dev::marchRows<double>() - 2, 8, 8 + h.nVox / 7500));
     return p;
 }
 
