@@ -475,9 +475,9 @@ __global__ void k_prolong(LevelView F, int CPX, int CNY, const int* __restrict__
         if ((mask & 7) == 7) continue;
         int i, j, k;
         nodeCoords(F, fn, i, j, k);
-        const float z0 = ldv<float>(zf + 3 * fn), z1 = ldv<float>(zf + 3 * fn + 1), z2 = ldv<float>(zf + 3 * fn + 2);
         float s[3];
         prolongAt<1>(CNX, CNXY, zc, i, j, k, s);
+        const float z0 = ldv<float>(zf + 3 * fn), z1 = ldv<float>(zf + 3 * fn + 1), z2 = ldv<float>(zf + 3 * fn + 2);
         constexpr bool SCALED = !std::is_same<VC, float>::value;
         if (SCALED) {
             s[0] *= sp;
@@ -930,14 +930,21 @@ __global__ void k_mx_p(long long nNodes, const uint8_t* __restrict__ nmask, cons
     for (long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x; n < nNodes; n += (long long)gridDim.x * blockDim.x) {
         const uint8_t mask = nmask[n];
         if (!first && (mask & 7) == 7) continue;
+        float zv[3], pv[3];  // (all loads before the first store: they may not pass it)
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+            if (!fixedDof(mask, c)) {
+                zv[c] = z[3 * n + c];
+                pv[c] = first ? 0.f : p[3 * n + c];
+            }
 #pragma unroll
         for (int c = 0; c < 3; c++) {
             const long long i = 3 * n + c;
             if (fixedDof(mask, c)) {
                 if (first) p[i] = 0.f;
-                continue;
+            } else {
+                p[i] = first ? zv[c] : zv[c] + beta * pv[c];
             }
-            p[i] = first ? z[i] : z[i] + beta * p[i];
         }
     }
 }
