@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <functional>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 #include <thread>
@@ -44,5 +45,23 @@ inline void parallelFor(int64_t n, const std::function<void(int64_t, int64_t)>& 
     }
     for (auto& t : th) t.join();
 }
+
+// Runs something once for each device of the process (kernel attributes belong to the device that was current when
+// they were set). An exception leaves the device undone, for the next caller; others wait for the one that runs it.
+class OncePerDevice {
+public:
+    template <class F>
+    void run(int device, F&& fn) {
+        std::lock_guard<std::mutex> g(mu_);
+        if (size_t(device) >= done_.size()) done_.resize(size_t(device) + 1, 0);
+        if (done_[size_t(device)]) return;
+        fn();
+        done_[size_t(device)] = 1;
+    }
+
+private:
+    std::mutex mu_;
+    std::vector<char> done_;
+};
 
 }  // namespace psfea

@@ -1726,8 +1726,8 @@ void SharedModel::adopt(Hierarchy&& h) {
     if (const char* e = std::getenv("PSFEA_EBE_SPLIT")) ebeSplit = std::atoi(e) == 1 ? 1 : 3;
     check(cudaStreamCreateWithFlags(&ms, cudaStreamNonBlocking), "stream");
     check(cudaEventCreateWithFlags(&readyEv, cudaEventDisableTiming), "event");
-    static std::once_flag attrOnce;
-    std::call_once(attrOnce, [] {
+    static OncePerDevice attrOnce;
+    attrOnce.run(devId, [] {
         // kernels that use more than the default 48 KB of shared memory
         auto set = [](auto kernel, size_t bytes) {
             check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)), "attr");
@@ -3117,8 +3117,8 @@ struct BlockImpl final : BlockBase {
     BlockImpl(std::shared_ptr<SharedModel> model) : M(std::move(model)), H(M->H), L(M->L), smCount(M->smCount) {
         M->ensureActiveLists();
         M->ensureBlockStencils();
-        static std::once_flag attrOnce;
-        std::call_once(attrOnce, [] {
+        static OncePerDevice attrOnce;
+        attrOnce.run(M->devId, [] {
             // the stencil rows a CTA's warps stage (31 KB for an 8-wide block)
             auto set = [](auto kernel, size_t b) {
                 check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(b)), "attr");
