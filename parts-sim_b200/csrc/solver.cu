@@ -1988,7 +1988,13 @@ void SharedModel::ensureStencils(bool half) {
         const int grid = gridFor(int64_t(cnt) * 27, 256, smCount * 32);
         if (cnt < stencilMinNodes) {
             if (D.stn8.p) continue;
-            D.stn8.alloc(size_t(cnt) * dev::STN8_ROW * sizeof(float), bytes, ms);
+            try {
+                D.stn8.alloc(size_t(cnt) * dev::STN8_ROW * sizeof(float), bytes, ms);
+            } catch (const Error& e) {  // no memory for them: the level keeps the gather
+                if (e.status != PS_EOOM) throw;
+                cudaGetLastError();
+                continue;
+            }
             dev::k_stn_build<float, float, dev::STN_LANES><<<grid, 256, 0, ms>>>(D.view, D.c32, D.stnNodes, cnt, D.stn8.as<float>(), 1.f);
             check(cudaGetLastError(), "stencil build");
             built = true;
